@@ -189,6 +189,7 @@ extern "C" int su2b_ctx_destroy(su2b_ctx *ctx) {
   if (ctx->h_traj) cudaFreeHost(ctx->h_traj);
   if (ctx->h_counts) cudaFreeHost(ctx->h_counts);
   if (ctx->h_st) cudaFreeHost(ctx->h_st);
+  if (ctx->h_cg) cudaFreeHost(ctx->h_cg);
   if (ctx->h_tparams) cudaFreeHost(ctx->h_tparams);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;

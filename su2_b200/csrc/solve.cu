@@ -110,6 +110,32 @@ int cg64(su2b_ctx *ctx, double m, double tol, int max_iter, su2b_solve_stats *st
   double2 *b = ctx->sv[SV_B], *x = ctx->sv[SV_X], *r = ctx->sv[SV_R], *p = ctx->sv[SV_P],
           *t = ctx->sv[SV_T], *Ap = ctx->sv[SV_AP];
   double *dp = ctx->part_slot(3), *np = ctx->part_slot(4);
+  // d = 2 up to about 150,000 sites: the whole solve, restarts included, in one launch on tiles
+  if (ctx->cg_plan.K) {
+    CgTileResult &h = *ctx->h_cg;
+    h.done = 0;
+    h.failed = 0;
+    const cudaError_t e = cg_tile(g, ctx->cg_plan, ctx->ph, m, b, x, tol, max_iter, ctx->cg_work,
+                                  ctx->cg_epoch, ctx->h_cg, s);
+    if (e != cudaErrorNotSupported) {
+      SU2B_CK(e);
+      ctx->launches++;
+      const cudaError_t es = cudaStreamSynchronize(s);
+      if (es != cudaSuccess || h.failed) {
+        ctx->cg_epoch += 1ull << 40;  // past every epoch the failed solve can have used
+        SU2B_CK(es);
+        return su2b_fail(ctx, SU2B_ERR_TIMEOUT, "tiled CG: a wait for another block gave up");
+      }
+      ctx->cg_epoch = h.epoch;
+      if (stats) {
+        stats->iterations = h.iters;
+        stats->restarts = h.restarts;
+        stats->residual = h.rn;
+        stats->true_residual = h.true_residual;
+      }
+      return finish_status(ctx, h.done);
+    }
+  }
   SU2B_CKS(true_residual(ctx, m, true, b, x, r, 20));
   SU2B_CKS(su2b_fetch_red(ctx, 21));
   double rr0 = ctx->h_red[20];
@@ -407,6 +433,21 @@ int su2b_fermion_setup(su2b_ctx *ctx, bool need32) {
     for (int k = 0; k < SV_N; k++)
       SU2B_CKS(dalloc2(ctx, (void **)&ctx->sv[k], ctx->V * sizeof(double2)));
     ctx->phases_valid = false;
+    // the tiled CG's packets; without room for them the other forms run
+    const CgTilePlan plan = cg_tile_plan(ctx->g);
+    if (plan.K) {
+      void *work = nullptr;
+      if (cudaMalloc(&work, cg_tile_bytes(ctx->g)) == cudaSuccess &&
+          cudaMallocHost((void **)&ctx->h_cg, sizeof(CgTileResult)) == cudaSuccess) {
+        ctx->allocs.push_back(work);
+        SU2B_CK(cudaMemsetAsync(work, 0, cg_tile_bytes(ctx->g), ctx->stream));
+        ctx->cg_work = work;
+        ctx->cg_plan = plan;
+      } else {
+        cudaFree(work);
+        cudaGetLastError();
+      }
+    }
   }
   if (need32 && !ctx->ph32) {
     SU2B_CKS(dalloc2(ctx, (void **)&ctx->ph32, ctx->NL * sizeof(float2)));

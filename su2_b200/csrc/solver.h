@@ -67,6 +67,31 @@ cudaError_t bicgstab_persistent(const Geom &g, const double2 *ph, double m, doub
                                 double2 *Ap, double2 *Ap2, double2 *sv, double2 *t,
                                 double *part, SolverState *st, void *bar_mem, int part_cap,
                                 cudaStream_t s);
+// the CG on D D^+ with its true-residual restarts on tiles in registers and shared memory, one
+// cooperative launch (cg_tile.cu): b and x (start in, solution out) in device memory.
+// plan: cg_tile_plan, K = 0 where the lattice does not take it (d != 2, too large, or no
+// cooperative launch).  work: cg_tile_bytes of memory zeroed once, kept between solves; epoch:
+// the result's epoch of the last solve with this work (0 at first).  out: pinned host memory.
+// cudaErrorNotSupported: the blocks do not fit beside each other now.
+struct CgTilePlan {
+  int K;       // sites per thread
+  int ht, hx;  // tile rows (t) and columns (x)
+  int gt, gx;  // tiles
+  int rp;      // rows per pass: ht = K rp, threads = rp hx
+  int cluster; // blocks of the cluster that holds the lattice; 0: blocks over the whole GPU
+};
+struct CgTileResult {
+  double rn, true_residual;
+  long iters, restarts;
+  unsigned long long epoch;
+  int done;    // as SolverState
+  int failed;  // a wait gave up
+};
+CgTilePlan cg_tile_plan(const Geom &g);
+size_t cg_tile_bytes(const Geom &g);
+cudaError_t cg_tile(const Geom &g, const CgTilePlan &tp, const double2 *ph, double m,
+                    const double2 *b, double2 *x, double tol, long max_iter, void *work,
+                    unsigned long long epoch, CgTileResult *out, cudaStream_t s);
 int cg_barrier_failed(const void *bar_mem, cudaStream_t s, int *failed);
 size_t cg_barrier_bytes();
 

@@ -52,6 +52,11 @@ struct su2b_ctx {
   float2 *sv32[SV32_N] = {};
   double *fderiv = nullptr;
   su2b::SolverState *st = nullptr;
+  // the tiled CG (cg_tile.cu): its plan (K = 0: not for this lattice), packets and their epoch
+  su2b::CgTilePlan cg_plan{};
+  void *cg_work = nullptr;
+  unsigned long long cg_epoch = 0;
+  su2b::CgTileResult *h_cg = nullptr;
   long x0_seed = -1;  // seed of the reference CG start held in sv[SV_X0]
 
   // set at the end of a fused trajectory: red[] then holds the plaquette sums of both the

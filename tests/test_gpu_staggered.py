@@ -195,3 +195,31 @@ def test_operator_and_solve_at_1024_squared(gpu):
         for k in range(3):
             assert np.array_equal(shift(out["plain"][k], 2), out["shifted"][k])
         assert rel(out["shifted"][3], shift(out["plain"][3], 2)) < 1e-8
+
+
+# one block; clusters of 2..16 with partial and one-row tiles; the largest of one and two sites
+# per thread; whole-GPU tilings of one and two sites per thread; past them the grid-barrier form
+@pytest.mark.parametrize("Lx,Lt", [(2, 2), (6, 4), (22, 24), (2, 600), (300, 2), (26, 38), (64, 64),
+                                   (90, 90), (128, 128), (130, 134), (256, 250), (300, 340),
+                                   (440, 400)])
+def test_cg_tilings(gpu, Lx, Lt):
+    """The CG of two-dimensional lattices at the edges of its tilings: the residual of its solution
+    by the stand-alone operator is the one it reports and below the tolerance.  Rounding of
+    b - D D^+ x: |A| |x| times a few eps, with |x| <= |b| / m^2 and |A| <= (m + 2)^2."""
+    rng = np.random.default_rng(Lx * 1000 + Lt)
+    V, m, tol = Lx * Lt, 0.2, 1e-10
+    b = rng.normal(size=2 * V)
+    nb = np.linalg.norm(b)
+    slack = 20 * 2.2e-16 * (m + 2) ** 2 / m ** 2 * nb
+    with u1(gpu, (Lx, 1, 1, Lt), 2) as c:
+        c.upload(rng.normal(size=2 * V))
+        for _ in range(2):  # the second solve meets the first one's packets
+            r = c.solve(b, m, tol=tol, tol_mode="rel")
+            res = np.linalg.norm(b - c.DDdag(m, r.x))
+            assert r.converged
+            assert r.true_residual <= tol * nb + slack
+            assert res == pytest.approx(r.true_residual, abs=slack)
+        again = c.solve(b, m, tol=2 * tol, tol_mode="rel", x0=r.x)
+        assert again.converged and again.iterations == 0 and np.array_equal(again.x, r.x)
+        few = c.solve(b, m, tol=1e-14, tol_mode="rel", max_iter=2)
+        assert few.iterations <= 2
