@@ -35,141 +35,269 @@ namespace {
 
 template <class T> using LinkT = typename LinkOf<T>::type;
 
-template <class T> __device__ __forceinline__ Su2<T> alg(T ma, T mb, T mc) {
-  return Su2<T>{T(0), mc, mb, ma};
+// an algebra element i (x s_x + y s_y + z s_z): {Im b, Re b, Im a} of the (a, b) storage
+template <class T> struct V3 {
+  T x, y, z;
+};
+template <class T> __device__ __forceinline__ V3<T> operator+(const V3<T> &a, const V3<T> &b) {
+  return V3<T>{a.x + b.x, a.y + b.y, a.z + b.z};
+}
+template <class T> __device__ __forceinline__ V3<T> operator-(const V3<T> &a, const V3<T> &b) {
+  return V3<T>{a.x - b.x, a.y - b.y, a.z - b.z};
+}
+template <class T> __device__ __forceinline__ V3<T> cross(const V3<T> &a, const V3<T> &b) {
+  return V3<T>{fm(a.y, b.z, -a.z * b.y), fm(a.z, b.x, -a.x * b.z), fm(a.x, b.y, -a.y * b.x)};
+}
+// The rotation v -> d^+ v d / |d|^2 of an almost unit d = (d0, e): v + d0 w + e x w with
+// w = f x v, f = 2 e / |d|^2; 2 / n = 4 - 2 n up to (1 - n)^2, below rounding for links that are
+// unitary to their storage precision.
+template <class T> struct Rot {
+  T d0;
+  V3<T> e, f;
+};
+template <class T> __device__ __forceinline__ Rot<T> rot_of(const Su2<T> &d) {
+  const T n = fm(d.ar, d.ar, fm(d.ai, d.ai, fm(d.br, d.br, d.bi * d.bi)));
+  const T w = fm(T(-2), n, T(4));
+  return Rot<T>{d.ar, V3<T>{d.bi, d.br, d.ai}, V3<T>{w * d.bi, w * d.br, w * d.ai}};
+}
+// d^+ v d (inverse: d v d^+) over |d|^2
+template <class T>
+__device__ __forceinline__ V3<T> rotate(const Rot<T> &r, const V3<T> &v, bool inverse) {
+  const T s = inverse ? T(-1) : T(1);
+  const V3<T> w = cross(r.f, v), u = cross(r.e, w);
+  return V3<T>{fm(s * r.d0, w.x, v.x + u.x), fm(s * r.d0, w.y, v.y + u.y),
+               fm(s * r.d0, w.z, v.z + u.z)};
 }
 
-// VJP of the force field, accumulated: lam(x,nu) += coef * VJP(x,nu).  One thread per link.
+// What pass 1 leaves for pass 2, component by component (each a field of V reals): the
+// 3 ND (ND - 1) reals a site sends to its forward neighbours, then the 3 ND of its own links.  Two
+// spare link buffers hold 4 ND components each, the staging buffer (4 ND doubles) the others.
+template <class T, int ND> struct Sent {
+  T *a, *b, *c;
+  __device__ __forceinline__ T *at(int k, size_t V) const {
+    return k < 4 * ND ? a + k * V : k < 8 * ND ? b + (k - 4 * ND) * V : c + (k - 8 * ND) * V;
+  }
+};
+
+// VJP of the force field, lam(x,nu) (+)= coef * VJP(x,nu), in two passes.  For the plaquette
+// P = A B C^+ D^+ with A = U_mu(x), B = U_nu(x+mu), C = U_mu(x+nu), D = U_nu(x), cotangents
+// m_A .. m_D, n_B = A m_B A^+, n_C = D m_C D^+, N = m_A + n_B - n_C - m_D and P = (p0, p), the
+// decorated sums of its four links reduce to
+//   A: v - w + 2 p x n_B        D: -(v + w + 2 p x n_C)
+//   B: A^+ (v - w) A            C: -D^+ (v + w) D            v = p0 N, w = p x N,
+// (vec(P N) = v - w, vec(N P) = v + w).  Pass 1, one thread per site: every plaquette once, its
+// four results into `sent`; pass 2 adds a link's own sum and what the backward neighbours sent.
+// 930 FMAs and 16 links per site in d = 4 and 384 B (FP32) of intermediate values, where one
+// thread per link forming all staples with a cotangent in each of their four places took 5,000
+// FMAs and 76 links.  Memory bounds both passes: at 24^4 FP32, cold, 27 us and 35 us with the
+// reverse of a link update in the second, against 109 us and 27 us for that update by itself.
 template <class T, int ND, int NT>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
   k_force_vjp(Geom g, const LinkT<T> *__restrict__ U, const T *__restrict__ mu,
-              T *__restrict__ lam, T coef, int accumulate) {
-  const int nu = blockIdx.y >> 1, p = blockIdx.y & 1, q = 1 - p;
-  const int cb = blockIdx.x * NT + threadIdx.x;
+              Sent<T, ND> sent) {
+  const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
+  const int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
   if (cb >= g.Vh) return;
   const Site s = site_from_eo(g, p, cb);
-  const size_t V = (size_t)g.V, NL = V * ND;
-  auto M = [&](size_t l) { return alg<T>(mu[l], mu[NL + l], mu[2 * NL + l]); };
-  const size_t ll = nu * V + (size_t)p * g.Vh + cb;
-  const Su2<T> ul = ld_link(U + ll);
-  const Su2<T> Ml = M(ll);
-  const int lpn = s.lex + fwd(g, s, nu);
-  Su2<T> D = zero_su2<T>();
+  const size_t V = (size_t)g.V, NL = V * ND, self = (size_t)p * g.Vh + cb;
+  auto M = [&](size_t l) { return V3<T>{mu[l], mu[NL + l], mu[2 * NL + l]}; };
+  Su2<T> u[ND];
+  V3<T> S[ND];
 #pragma unroll
-  for (int rho = 0; rho < ND; rho++) {
-    if (rho == nu) continue;
-    // forward: A = U_rho(x+nu), B = U_nu(x+rho)^+, C = U_rho(x)^+
-    {
-      const size_t la = rho * V + eo_of(g, lpn, q);
-      const size_t lb = nu * V + eo_of(g, s.lex + fwd(g, s, rho), q);
-      const size_t lc = rho * V + (size_t)p * g.Vh + cb;
-      const Su2<T> A = ld_link(U + la), B = dag(ld_link(U + lb)), C = dag(ld_link(U + lc));
-      const Su2<T> BC = mul(B, C), AB = mul(A, B), ABC = mul(A, BC);
-      D = add(D, mul(ABC, Ml));
-      D = add(D, mul(mul(M(la), A), BC));              // A forward: +M A
-      D = add(D, scale(T(-1), mul(A, mul(mul(B, M(lb)), C))));  // B backward: -B M
-      D = add(D, scale(T(-1), mul(AB, mul(C, M(lc)))));        // C backward: -C M
+  for (int d = 0; d < ND; d++) u[d] = ld_link(U + d * V + self), S[d] = V3<T>{0, 0, 0};
+#pragma unroll
+  for (int d = 0; d < ND - 1; d++)
+#pragma unroll
+    for (int e = d + 1; e < ND; e++) {
+      const size_t lb = e * V + eo_of(g, s.lex + fwd(g, s, d), q);
+      const size_t lc = d * V + eo_of(g, s.lex + fwd(g, s, e), q);
+      const Su2<T> P = mul(mul(u[d], ld_link(U + lb)), dag(mul(u[e], ld_link(U + lc))));
+      const V3<T> pv{P.bi, P.br, P.ai};
+      const Rot<T> ra = rot_of(u[d]), rd = rot_of(u[e]);
+      const V3<T> nb = rotate(ra, M(lb), true), nc = rotate(rd, M(lc), true);
+      const V3<T> N = (M(d * V + self) + nb) - (nc + M(e * V + self));
+      const V3<T> v{P.ar * N.x, P.ar * N.y, P.ar * N.z}, x = cross(pv, N);
+      const V3<T> lo = v - x, hi = v + x;
+      const V3<T> xb = cross(pv, nb), xc = cross(pv, nc);
+      S[d] = S[d] + (lo + (xb + xb));
+      S[e] = S[e] - (hi + (xc + xc));
+      // to U_e(x + d) and U_d(x + e): components [direction of the step][link]
+      const V3<T> to_b = rotate(ra, lo, false), to_c = rotate(rd, hi, false);
+      const int kb = 3 * ((ND - 1) * d + (e - 1)), kc = 3 * ((ND - 1) * e + d);
+      sent.at(kb, V)[self] = to_b.x;
+      sent.at(kb + 1, V)[self] = to_b.y;
+      sent.at(kb + 2, V)[self] = to_b.z;
+      sent.at(kc, V)[self] = -to_c.x;
+      sent.at(kc + 1, V)[self] = -to_c.y;
+      sent.at(kc + 2, V)[self] = -to_c.z;
     }
-    // backward: A = U_rho(x+nu-rho)^+, B = U_nu(x-rho)^+, C = U_rho(x-rho)
-    {
-      const int b = bwd(g, s, rho);
-      const size_t la = rho * V + eo_of(g, lpn + b, p);
-      const size_t lb = nu * V + eo_of(g, s.lex + b, q);
-      const size_t lc = rho * V + eo_of(g, s.lex + b, q);
-      const Su2<T> A = dag(ld_link(U + la)), B = dag(ld_link(U + lb)), C = ld_link(U + lc);
-      const Su2<T> BC = mul(B, C), AB = mul(A, B), ABC = mul(A, BC);
-      D = add(D, mul(ABC, Ml));
-      D = add(D, scale(T(-1), mul(mul(A, M(la)), BC)));  // A backward: -A M
-      D = add(D, scale(T(-1), mul(A, mul(mul(B, M(lb)), C))));  // B backward: -B M
-      D = add(D, mul(AB, mul(M(lc), C)));                // C forward: +M C
-    }
-  }
-  const Su2<T> S = mul(ul, D);
-  const T g0 = T(2) * S.bi, g1 = T(2) * S.br, g2 = T(2) * S.ai;
-  if (accumulate) {
-    lam[ll] += coef * g0;
-    lam[NL + ll] += coef * g1;
-    lam[2 * NL + ll] += coef * g2;
-  } else {
-    lam[ll] = coef * g0;
-    lam[NL + ll] = coef * g1;
-    lam[2 * NL + ll] = coef * g2;
+#pragma unroll
+  for (int d = 0; d < ND; d++) {
+    const int k = 3 * ND * (ND - 1) + 3 * d;
+    sent.at(k, V)[self] = S[d].x;
+    sent.at(k + 1, V)[self] = S[d].y;
+    sent.at(k + 2, V)[self] = S[d].z;
   }
 }
 
-// reverse of W' = exp(b Z) W, per link: lam <- R(bZ)^T lam ; mu (+)= b J(bZ)^T lam
+// Horner steps k = K .. 0 of sum_k (-1)^k t2^k / (2k + j)!, j = 1, 2, 3
+template <int k> struct SeriesJ {
+  static __device__ __forceinline__ void run(double t2, double &s1, double &c1, double &c2) {
+    constexpr double sg = (k & 1) ? -1.0 : 1.0;
+    s1 = fma(s1, t2, sg / detail::fact(2 * k + 1));
+    c1 = fma(c1, t2, sg / detail::fact(2 * k + 2));
+    c2 = fma(c2, t2, sg / detail::fact(2 * k + 3));
+    SeriesJ<k - 1>::run(t2, s1, c1, c2);
+  }
+};
+template <> struct SeriesJ<-1> {
+  static __device__ __forceinline__ void run(double, double &, double &, double &) {}
+};
+
+// reverse of W' = exp(b Z) W for link l with cotangent (l0, l1, l2):
+// lam <- R(bZ)^T lam ; mu (+)= b J(bZ)^T lam
+template <class T>
+__device__ __forceinline__ void exp_adjoint_link(size_t l, size_t NL, const T *__restrict__ Z, T b,
+                                                 double l0, double l1, double l2,
+                                                 T *__restrict__ lam, T *__restrict__ mu,
+                                                 int accumulate) {
+  const double x0 = (double)b * Z[l], x1 = (double)b * Z[NL + l], x2 = (double)b * Z[2 * NL + l];
+  const double t2 = 4.0 * (x0 * x0 + x1 * x1 + x2 * x2);  // th^2, th = 2 |x|
+  // ad v = -2 x cross v ; ad^2 v = 4 (x (x.v) - |x|^2 v)
+  auto ad = [&](double v0, double v1, double v2, double &r0, double &r1, double &r2) {
+    r0 = -2.0 * (x1 * v2 - x2 * v1);
+    r1 = -2.0 * (x2 * v0 - x0 * v2);
+    r2 = -2.0 * (x0 * v1 - x1 * v0);
+  };
+  double c1, c2, s1, s2;  // J = 1 + c1 ad + c2 ad^2 ; R = exp(ad) = 1 + s1 ad + s2 ad^2
+  if (t2 <= 0.25) {
+    // sin(th)/th, (1 - cos th)/th^2, (th - sin th)/th^3 as their series in th^2 (the first
+    // omitted terms are below 1e-16): every flow step in practice, and no cancellation.  A
+    // quarter of the FP64 work of the square root, sincospi and five divisions below
+    s1 = c1 = c2 = 0.;
+    SeriesJ<6>::run(t2, s1, c1, c2);
+    s2 = c1;
+  } else {
+    const double th = sqrt(t2);
+    double sn, cs;
+    sincospi(th * M_1_PI_D, &sn, &cs);
+    c1 = (1.0 - cs) / (th * th);
+    c2 = (th - sn) / (th * th * th);
+    s1 = sn / th;
+    s2 = (1.0 - cs) / (th * th);
+  }
+  // transposes: ad^T = -ad (skew), (ad^2)^T = ad^2
+  double a0, a1, a2v, b0, b1, b2;
+  ad(l0, l1, l2, a0, a1, a2v);
+  ad(a0, a1, a2v, b0, b1, b2);
+  const double r0 = l0 - s1 * a0 + s2 * b0, r1 = l1 - s1 * a1 + s2 * b1,
+               r2 = l2 - s1 * a2v + s2 * b2;
+  const double j0 = (double)b * (l0 - c1 * a0 + c2 * b0),
+               j1 = (double)b * (l1 - c1 * a1 + c2 * b1),
+               j2 = (double)b * (l2 - c1 * a2v + c2 * b2);
+  lam[l] = (T)r0;
+  lam[NL + l] = (T)r1;
+  lam[2 * NL + l] = (T)r2;
+  if (accumulate) {
+    mu[l] += (T)j0;
+    mu[NL + l] += (T)j1;
+    mu[2 * NL + l] += (T)j2;
+  } else {
+    mu[l] = (T)j0;
+    mu[NL + l] = (T)j1;
+    mu[2 * NL + l] = (T)j2;
+  }
+}
 template <class T>
 __global__ void k_exp_adjoint(size_t NL, const T *__restrict__ Z, T b, T *__restrict__ lam,
-                              T *__restrict__ mu, int accumulate) {
+                              T *__restrict__ mu) {
   for (size_t l = blockIdx.x * (size_t)blockDim.x + threadIdx.x; l < NL;
-       l += (size_t)gridDim.x * blockDim.x) {
-    const double x0 = (double)b * Z[l], x1 = (double)b * Z[NL + l], x2 = (double)b * Z[2 * NL + l];
-    const double l0 = lam[l], l1 = lam[NL + l], l2 = lam[2 * NL + l];
-    const double a2 = x0 * x0 + x1 * x1 + x2 * x2, al = sqrt(a2), th = 2.0 * al;
-    // ad v = -2 x cross v ; ad^2 v = 4 (x (x.v) - |x|^2 v)
-    auto ad = [&](double v0, double v1, double v2, double &r0, double &r1, double &r2) {
-      r0 = -2.0 * (x1 * v2 - x2 * v1);
-      r1 = -2.0 * (x2 * v0 - x0 * v2);
-      r2 = -2.0 * (x0 * v1 - x1 * v0);
-    };
-    double c1, c2, s1, s2;  // J = 1 + c1 ad + c2 ad^2 ; R = exp(ad) = 1 + s1 ad + s2 ad^2
-    if (th < 1e-3) {
-      const double t2 = th * th;
-      c1 = 0.5 - t2 / 24.0;
-      c2 = 1.0 / 6.0 - t2 / 120.0;
-      s1 = 1.0 - t2 / 6.0;
-      s2 = 0.5 - t2 / 24.0;
-    } else {
-      double sn, cs;
-      sincospi(th * M_1_PI_D, &sn, &cs);
-      c1 = (1.0 - cs) / (th * th);
-      c2 = (th - sn) / (th * th * th);
-      s1 = sn / th;
-      s2 = (1.0 - cs) / (th * th);
+       l += (size_t)gridDim.x * blockDim.x)
+    exp_adjoint_link(l, NL, Z, b, (double)lam[l], (double)lam[NL + l], (double)lam[2 * NL + l], lam,
+                     mu, 0);
+}
+
+// Pass 2 of the VJP, then (EXP) the reverse of the link update before the stage in the same
+// pass over the cotangent: lam is read and written once instead of twice
+template <class T, int ND, int NT, bool EXP>
+__global__ void __launch_bounds__(NT)
+  k_force_vjp_gather(Geom g, Sent<T, ND> sent, T *__restrict__ lam, T coef,
+                     int acc_lam, const T *__restrict__ Z, T b, T *__restrict__ mu, int acc_mu) {
+  const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
+  const int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  if (cb >= g.Vh) return;
+  const Site s = site_from_eo(g, p, cb);
+  const size_t V = (size_t)g.V, NL = V * ND, self = (size_t)p * g.Vh + cb;
+  T S[3 * ND];
+#pragma unroll
+  for (int k = 0; k < 3 * ND; k++) S[k] = __ldg(sent.at(3 * ND * (ND - 1) + k, V) + self);
+#pragma unroll
+  for (int d = 0; d < ND; d++) {
+    const size_t z = eo_of(g, s.lex + bwd(g, s, d), q);
+#pragma unroll
+    for (int m = 0; m < ND; m++) {
+      if (m == d) continue;
+      const int k = 3 * ((ND - 1) * d + (m < d ? m : m - 1));
+#pragma unroll
+      for (int i = 0; i < 3; i++) S[3 * m + i] += __ldg(sent.at(k + i, V) + z);
     }
-    // transposes: ad^T = -ad (skew), (ad^2)^T = ad^2
-    double a0, a1, a2v, b0, b1, b2;
-    ad(l0, l1, l2, a0, a1, a2v);
-    ad(a0, a1, a2v, b0, b1, b2);
-    const double r0 = l0 - s1 * a0 + s2 * b0, r1 = l1 - s1 * a1 + s2 * b1,
-                 r2 = l2 - s1 * a2v + s2 * b2;
-    const double j0 = (double)b * (l0 - c1 * a0 + c2 * b0),
-                 j1 = (double)b * (l1 - c1 * a1 + c2 * b1),
-                 j2 = (double)b * (l2 - c1 * a2v + c2 * b2);
-    lam[l] = (T)r0;
-    lam[NL + l] = (T)r1;
-    lam[2 * NL + l] = (T)r2;
-    if (accumulate) {
-      mu[l] += (T)j0;
-      mu[NL + l] += (T)j1;
-      mu[2 * NL + l] += (T)j2;
+  }
+  const T c2 = T(2) * coef;
+#pragma unroll
+  for (int m = 0; m < ND; m++) {
+    const size_t l = m * V + self;
+    T v[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      v[i] = acc_lam ? fm(c2, S[3 * m + i], lam[i * NL + l]) : c2 * S[3 * m + i];
+    if (EXP) {
+      exp_adjoint_link(l, NL, Z, b, (double)v[0], (double)v[1], (double)v[2], lam, mu, acc_mu);
     } else {
-      mu[l] = (T)j0;
-      mu[NL + l] = (T)j1;
-      mu[2 * NL + l] = (T)j2;
+#pragma unroll
+      for (int i = 0; i < 3; i++) lam[i * NL + l] = v[i];
     }
   }
 }
 
+// The two passes.  spare: two link buffers and the staging buffer of the context, none of which
+// holds anything between calls; they carry what pass 1 sends to pass 2.  With Z pass 2 also takes
+// the reverse of exp(b Z) (lam, and mu accumulated).
+template <class T, int ND> Sent<T, ND> sent_in(void *const (&spare)[3]) {
+  return Sent<T, ND>{(T *)spare[0], (T *)spare[1], (T *)spare[2]};
+}
 template <class T>
-cudaError_t force_vjp(const Geom &g, const void *U, const T *mu, T *lam, double coef, int acc,
-                      cudaStream_t s) {
+cudaError_t force_vjp_send(const Geom &g, const void *U, const T *mu, void *const (&spare)[3],
+                           cudaStream_t s) {
   constexpr int NT = 128;
-  const dim3 grid((g.Vh + NT - 1) / NT, 2 * g.nd);
+  const int grid = (g.Vh + NT / 2 - 1) / (NT / 2);
   const LinkT<T> *u = (const LinkT<T> *)U;
-  switch (g.nd) {
-    case 2: k_force_vjp<T, 2, NT><<<grid, NT, 0, s>>>(g, u, mu, lam, (T)coef, acc); break;
-    case 3: k_force_vjp<T, 3, NT><<<grid, NT, 0, s>>>(g, u, mu, lam, (T)coef, acc); break;
-    default: k_force_vjp<T, 4, NT><<<grid, NT, 0, s>>>(g, u, mu, lam, (T)coef, acc); break;
-  }
+#define SU2B_SEND(ND)                                                                      \
+  k_force_vjp<T, ND, NT><<<grid, NT, 0, s>>>(g, u, mu, sent_in<T, ND>(spare))
+  if (g.nd == 2) SU2B_SEND(2);
+  else if (g.nd == 3) SU2B_SEND(3);
+  else SU2B_SEND(4);
+#undef SU2B_SEND
   return cudaGetLastError();
 }
 template <class T>
-cudaError_t exp_adjoint(const Geom &g, const T *Z, double b, T *lam, T *mu, int acc,
-                        cudaStream_t s) {
+cudaError_t force_vjp_gather(const Geom &g, T *lam, double coef, int acc, void *const (&spare)[3],
+                             const T *Z, double b, T *mu, int acc_mu, cudaStream_t s) {
+  constexpr int NT = 128;
+  const int grid = (g.Vh + NT / 2 - 1) / (NT / 2);
+#define SU2B_GATHER(ND, EXP)                                                               \
+  k_force_vjp_gather<T, ND, NT, EXP><<<grid, NT, 0, s>>>(g, sent_in<T, ND>(spare), lam, (T)coef, acc, Z, \
+                                                         (T)b, mu, acc_mu)
+  if (g.nd == 2) Z ? SU2B_GATHER(2, true) : SU2B_GATHER(2, false);
+  else if (g.nd == 3) Z ? SU2B_GATHER(3, true) : SU2B_GATHER(3, false);
+  else Z ? SU2B_GATHER(4, true) : SU2B_GATHER(4, false);
+#undef SU2B_GATHER
+  return cudaGetLastError();
+}
+template <class T>
+cudaError_t exp_adjoint(const Geom &g, const T *Z, double b, T *lam, T *mu, cudaStream_t s) {
   const size_t NL = (size_t)g.V * g.nd;
   const int grid = (int)std::min<size_t>((NL + 255) / 256, 148 * 32);
-  k_exp_adjoint<T><<<grid, 256, 0, s>>>(NL, Z, (T)b, lam, mu, acc);
+  k_exp_adjoint<T><<<grid, 256, 0, s>>>(NL, Z, (T)b, lam, mu);
   return cudaGetLastError();
 }
 
@@ -246,11 +374,27 @@ int flow_adjoint_t(su2b_ctx *ctx, double eps, int n, int every, double *objectiv
   lam = (T *)sc.get(ab);
   mu = (T *)sc.get(ab);
   const FlowCoef c = flow_coef(ctx, eps);
+  void *const spare[3] = {ctx->U_old, ctx->U2, ctx->stage};
   // Z = a g(W) (+ Z with FM_HAS_IN); with Wn, also Wn = exp(b Z) W from the same kernel
   auto force = [&](const void *W, T *Z, double a, int mode, void *Wn = nullptr,
                    double b = 0.0) {
     return su2b_q_force(ctx, W, Z, nullptr, a, 1.0, Wn ? (mode | FM_UPDATE) : mode, nullptr,
                         nullptr, Wn, b);
+  };
+  // The VJP's second pass waits for the next link update's reverse, which takes it along (or
+  // for the end); nothing in between touches the cotangent or the spare buffers.
+  bool sent = false;
+  double sent_a = 0.;
+  auto vjp = [&](const void *W, double a) -> int {
+    SU2B_LAUNCH(SU2B_K_FORCE, force_vjp_send<T>(g, W, mu, spare, s));
+    sent = true;
+    sent_a = a;
+    return SU2B_OK;
+  };
+  auto gather = [&](const T *Z, double bz, int acc_mu) -> int {
+    SU2B_LAUNCH(SU2B_K_FORCE, force_vjp_gather<T>(g, lam, sent_a, 1, spare, Z, bz, mu, acc_mu, s));
+    sent = false;
+    return SU2B_OK;
   };
   // forward with checkpoints every `every` steps; the field alternates between cur and W1
   // (W1 is free until the backward pass), so every stage is fused with its link update
@@ -288,15 +432,19 @@ int flow_adjoint_t(su2b_ctx *ctx, double eps, int n, int every, double *objectiv
       SU2B_CKS(force(W1, Zs[1], c.a[1], FM_HAS_IN, W2, c.b[1]));
       SU2B_CK(cudaMemcpyAsync(Zs[2], Zs[1], ab, cudaMemcpyDeviceToDevice, s));
       SU2B_CKS(force(W2, Zs[2], c.a[2], FM_HAS_IN));
-      // reverse
-      SU2B_LAUNCH(SU2B_K_OTHER, exp_adjoint<T>(g, Zs[2], c.b[2], lam, mu, 0, s));
-      SU2B_LAUNCH(SU2B_K_FORCE, force_vjp<T>(g, W2, mu, lam, c.a[2], 1, s));
-      SU2B_LAUNCH(SU2B_K_OTHER, exp_adjoint<T>(g, Zs[1], c.b[1], lam, mu, 1, s));
-      SU2B_LAUNCH(SU2B_K_FORCE, force_vjp<T>(g, W1, mu, lam, c.a[1], 1, s));
-      SU2B_LAUNCH(SU2B_K_OTHER, exp_adjoint<T>(g, Zs[0], c.b[0], lam, mu, 1, s));
-      SU2B_LAUNCH(SU2B_K_FORCE, force_vjp<T>(g, W0, mu, lam, c.a[0], 1, s));
+      // reverse; the last stage's update starts the step's mu
+      if (sent)
+        SU2B_CKS(gather(Zs[2], c.b[2], 0));
+      else
+        SU2B_LAUNCH(SU2B_K_OTHER, exp_adjoint<T>(g, Zs[2], c.b[2], lam, mu, s));
+      SU2B_CKS(vjp(W2, c.a[2]));
+      SU2B_CKS(gather(Zs[1], c.b[1], 1));
+      SU2B_CKS(vjp(W1, c.a[1]));
+      SU2B_CKS(gather(Zs[0], c.b[0], 1));
+      SU2B_CKS(vjp(W0, c.a[0]));
     }
   }
+  if (sent) SU2B_CKS(gather(nullptr, 0., 0));
   return su2b_adj_download(ctx, lam, grad_host);
 }
 
@@ -325,12 +473,16 @@ extern "C" int su2b_force_vjp(su2b_ctx *ctx, const double *mu_host, double *out_
   if (ctx->group != SU2B_GROUP_SU2)
     return su2b_fail(ctx, SU2B_ERR_UNSUPPORTED, "the force VJP is provided for SU(2)");
   SU2B_CKS(su2b_adj_upload(ctx, mu_host, ctx->P));
-  if (ctx->link64)
-    SU2B_LAUNCH(SU2B_K_FORCE, force_vjp<double>(ctx->g, ctx->U, (const double *)ctx->P,
-                                                (double *)ctx->Z, 1.0, 0, ctx->stream));
-  else
-    SU2B_LAUNCH(SU2B_K_FORCE, force_vjp<float>(ctx->g, ctx->U, (const float *)ctx->P,
-                                               (float *)ctx->Z, 1.0, 0, ctx->stream));
+  void *const spare[3] = {ctx->U_old, ctx->U2, ctx->stage};
+  auto vjp = [&](auto zero) -> int {
+    using T = decltype(zero);
+    SU2B_LAUNCH(SU2B_K_FORCE, force_vjp_send<T>(ctx->g, ctx->U, (const T *)ctx->P, spare,
+                                                ctx->stream));
+    SU2B_LAUNCH(SU2B_K_FORCE, force_vjp_gather<T>(ctx->g, (T *)ctx->Z, 1.0, 0, spare, (const T *)nullptr,
+                                                  0.0, (T *)nullptr, 0, ctx->stream));
+    return SU2B_OK;
+  };
+  SU2B_CKS(ctx->link64 ? vjp(0.0) : vjp(0.0f));
   return su2b_adj_download(ctx, ctx->Z, out_host);
 }
 

@@ -66,6 +66,45 @@ def test_force_vjp_finite_differences(gpu, orc):
             assert fd == pytest.approx(vjp[3 * link + k], abs=2e-6 * max(1, abs(fd)))
 
 
+@pytest.mark.parametrize("dims,nd", [((6, 1, 1, 4), 2), ((2, 1, 1, 2), 2), ((4, 6, 1, 10), 3),
+                                     ((6, 6, 6, 6), 4), ((2, 4, 6, 2), 4)],
+                         ids=["6x4-d2", "2x2-d2", "4x6x10-d3", "6^4", "2x4x6x2"])
+def test_force_vjp_geometries(gpu, orc, dims, nd):
+    """The two-pass VJP in every dimension, at half volumes that are and are not whole blocks:
+    central finite differences along seeded directions (FP64; O(h^2) truncation), FP32 within
+    1e-5 (sums of about a hundred FP32 terms), and the buffers it borrows: the field stays, and
+    the next trajectory is that of a context that took no VJP."""
+    U = orc.hotstart(0, dims, nd, 9, 1.0, 654321)
+    n = U.size // 4
+    rng = np.random.default_rng(n)
+    mu = rng.normal(size=3 * n)
+    v = {}
+    for prec in ("fp64", "mixed"):
+        with gpu.gaugeconfig(*dims, nd, 2.0, precision=prec) as c, \
+                gpu.gaugeconfig(*dims, nd, 2.0, precision=prec) as d:
+            c.upload(U)
+            d.upload(U)
+            v[prec] = c.force_vjp(mu)
+            assert np.array_equal(c.download(), d.download())
+            a = c.md_update("omf2", 2, 0.5, seed=3, accept_reject=False)
+            b = d.md_update("omf2", 2, 0.5, seed=3, accept_reject=False)
+            assert a == b and np.array_equal(c.download(), d.download())
+    assert rel(v["mixed"], v["fp64"]) < 1e-5
+
+    from su2_b200.autograd import _exp_links
+
+    def phi(w):
+        g = orc.gauge_derivative(0, dims, nd, 2.0, _exp_links(U, w), 1.0, 1.0)
+        return float(mu @ g)
+
+    for _ in range(6):
+        w = rng.normal(size=(n, 3))
+        h = 1e-5
+        fd = (phi(h * w) - phi(-h * w)) / (2 * h)
+        scale = np.linalg.norm(v["fp64"]) * np.sqrt(3)
+        assert fd == pytest.approx(float(v["fp64"] @ w.ravel()), abs=1e-6 * scale)
+
+
 @pytest.mark.parametrize("every", [0, 1, 3])
 def test_flow_adjoint_finite_differences(gpu, orc, every):
     dims, nd = (4, 4, 4, 4), 4
