@@ -240,13 +240,6 @@ __global__ void __launch_bounds__(NT)
   reduce_into<NT>(part, n, ncomp, out, sh);
 }
 
-// Programmatic dependent launch between the chained force launches of a trajectory: each
-// block lets the next launch start as soon as it is itself resident, and waits for the
-// previous launch to complete (and its writes to be visible) before it touches global
-// memory.  Both are no-ops for a launch without a programmatic dependency.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // fused staple/force/momentum(/link update) kernel: one thread per site, force_site body
 template <class T, int ND, int NT, int MINB, bool ANISO>
 __global__ void __launch_bounds__(NT, MINB)
@@ -725,23 +718,6 @@ __global__ void __launch_bounds__(NT, MINB)
   }
 }
 
-// launch with the programmatic-stream-serialization attribute when pdl is set
-template <typename... KArgs, typename... Args>
-cudaError_t launch_force(void (*kern)(KArgs...), dim3 grid, int nt, cudaStream_t s, bool pdl,
-                         Args... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(nt);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 template <class T>
 cudaError_t force_update(const Geom &g, const void *U, int group, T *P, const T *extra, double f,
                          double scale, double xi, int mode, double *kin_part, int *nblocks,
@@ -762,15 +738,15 @@ cudaError_t force_update(const Geom &g, const void *U, int group, T *P, const T 
     cudaError_t e_;                                                                        \
     switch (g.nd) {                                                                        \
       case 2:                                                                              \
-        e_ = launch_force(k_force_su2<T, 2, NTV, MB, AN>, grid, NTV, s, pdl,               \
+        e_ = launch_force(k_force_su2<T, 2, NTV, MB, AN>, grid, NTV, s, pdl, 0,             \
                           SU2B_FORCE_ARGS);                                                \
         break;                                                                             \
       case 3:                                                                              \
-        e_ = launch_force(k_force_su2<T, 3, NTV, MB, AN>, grid, NTV, s, pdl,               \
+        e_ = launch_force(k_force_su2<T, 3, NTV, MB, AN>, grid, NTV, s, pdl, 0,             \
                           SU2B_FORCE_ARGS);                                                \
         break;                                                                             \
       default:                                                                             \
-        e_ = launch_force(k_force_su2<T, 4, NTV, MB, AN>, grid, NTV, s, pdl,               \
+        e_ = launch_force(k_force_su2<T, 4, NTV, MB, AN>, grid, NTV, s, pdl, 0,             \
                           SU2B_FORCE_ARGS);                                                \
         break;                                                                             \
     }                                                                                      \
@@ -785,7 +761,7 @@ cudaError_t force_update(const Geom &g, const void *U, int group, T *P, const T 
     const dim3 grid(cdiv(g.ncb, NTV / 4));                                                  \
     nb = grid.x;                                                                           \
     const cudaError_t e_ =                                                                 \
-      launch_force(k_force_su2_split<T, NTV, MB>, grid, NTV, s, pdl, SU2B_FORCE_ARGS);     \
+      launch_force(k_force_su2_split<T, NTV, MB>, grid, NTV, s, pdl, 0, SU2B_FORCE_ARGS);     \
     if (e_ != cudaSuccess) return e_;                                                      \
   } while (0)
 #define SU2B_FORCE_LINK(MB)                                                                  \
@@ -795,13 +771,13 @@ cudaError_t force_update(const Geom &g, const void *U, int group, T *P, const T 
     cudaError_t e_;                                                                        \
     switch (g.nd) {                                                                        \
       case 2:                                                                              \
-        e_ = launch_force(k_force_su2_link<T, 2, MB>, grid, 64, s, pdl, SU2B_FORCE_ARGS);  \
+        e_ = launch_force(k_force_su2_link<T, 2, MB>, grid, 64, s, pdl, 0, SU2B_FORCE_ARGS);  \
         break;                                                                             \
       case 3:                                                                              \
-        e_ = launch_force(k_force_su2_link<T, 3, MB>, grid, 96, s, pdl, SU2B_FORCE_ARGS);  \
+        e_ = launch_force(k_force_su2_link<T, 3, MB>, grid, 96, s, pdl, 0, SU2B_FORCE_ARGS);  \
         break;                                                                             \
       default:                                                                             \
-        e_ = launch_force(k_force_su2_link<T, 4, MB>, grid, 128, s, pdl, SU2B_FORCE_ARGS); \
+        e_ = launch_force(k_force_su2_link<T, 4, MB>, grid, 128, s, pdl, 0, SU2B_FORCE_ARGS); \
         break;                                                                             \
     }                                                                                      \
     if (e_ != cudaSuccess) return e_;                                                      \
@@ -815,7 +791,7 @@ cudaError_t force_update(const Geom &g, const void *U, int group, T *P, const T 
     const dim3 grid(cdiv(g.ncb, NTV / 4));                                                  \
     nb = grid.x;                                                                           \
     const cudaError_t e_ =                                                                 \
-      launch_force(k_force_su2_xsplit<T, NTV, MB>, grid, NTV, s, pdl, SU2B_FORCE_ARGS);    \
+      launch_force(k_force_su2_xsplit<T, NTV, MB>, grid, NTV, s, pdl, 0, SU2B_FORCE_ARGS);    \
     if (e_ != cudaSuccess) return e_;                                                      \
   } while (0)
     // the anisotropic action (rare) runs one launch shape; the tuned shapes are isotropic and

@@ -15,12 +15,10 @@
 // one Philox4x32-10 draw per hit, counter {reference link index, hit, sweep, TAG_METRO}:
 // 32-bit uniforms for alpha, u, theta and the accept test, the same stream in both
 // precisions.
-#include "su2b_internal.h"
+#include "site_ops.cuh"
 
 namespace su2b {
 namespace {
-
-template <class T> using LinkT = typename LinkOf<T>::type;
 
 // The FP64 accept test u < exp(-dS) (dS >= 0), decided by FP32 exp where that is safe.  The
 // FP32 value differs from the FP64 one by at most the rounding of dS to float (|dS| 2^-24
@@ -36,132 +34,182 @@ __device__ __forceinline__ bool accept_fp64(double u, double dS) {
   return u < exp(-dS);
 }
 
-// One link of a pass with FP32 storage (see the file comment); returns its accepted hits.
-template <int ND>
-__device__ __forceinline__ unsigned metro_link_fp32(const Geom &g, Link32 *__restrict__ U, int mu,
-                                                    int p, int cb, double beta_nc, double delta,
-                                                    int N_hit, uint64_t seed, uint32_t sweep,
-                                                    float wt, float ws) {
-  const Site s = site_from_eo(g, p, cb);
+// restoreSU in FP64 of a product of two unit elements: |u|^2 = 1 + e with e at the rounding of the
+// storage precision, and two Newton steps from 1 for its inverse square root leave 1e-20 for
+// e up to 2^-16, where a square root and a division cost forty FP64 instructions and the
+// longest latency of a hit.  Anything further from 1 (a field uploaded unnormalised) takes those.
+__device__ __forceinline__ Su2<double> restore_near(const Su2<double> &u) {
+  const double n = fma(u.ar, u.ar, fma(u.ai, u.ai, fma(u.br, u.br, u.bi * u.bi)));
+  if (!(fabs(n - 1.0) < 0x1p-16)) return restore_su(u);
+  const double y = fma(-0.5, n, 1.5), ir = y * fma(-0.5 * n, y * y, 1.5);
+  return Su2<double>{u.ar * ir, u.ai * ir, u.br * ir, u.bi * ir};
+}
+
+// random_element (random_element.hh:9-34) of hit n, in the storage precision, and the hit's
+// accept uniform
+__device__ __forceinline__ Su2<double> proposal(uint32_t lref, int n, uint32_t sweep, uint64_t seed,
+                                                double delta, double &accept) {
+  uint32_t r[4];
+  philox(lref, (uint32_t)n, sweep, TAG_METRO, seed, r);
+  double sa, ca, st, ct;
+  sincospi(2.0 * delta * u01_32(r[0]), &sa, &ca);
+  const double uu = 2.0 * u01_32(r[1]) - 1.0;
+  sincospi(2.0 * u01_32(r[2]), &st, &ct);
+  const double rr = sqrt(1.0 - uu * uu);
+  accept = u01_32(r[3]);
+  return Su2<double>{ca, sa * uu, sa * rr * st, sa * rr * ct};
+}
+__device__ __forceinline__ Su2<float> proposal(uint32_t lref, int n, uint32_t sweep, uint64_t seed,
+                                               float delta, double &accept) {
+  uint32_t r[4];
+  philox(lref, (uint32_t)n, sweep, TAG_METRO, seed, r);
+  float sa, ca, st, ct;
+  sincospif(2.0f * delta * (float)u01_32(r[0]), &sa, &ca);
+  const float uu = fmaf(2.0f, (float)u01_32(r[1]), -1.0f);
+  sincospif(2.0f * (float)u01_32(r[2]), &st, &ct);
+  const float rr = sqrtf(fmaxf(0.0f, fmaf(-uu, uu, 1.0f)));
+  accept = u01_32(r[3]);
+  return Su2<float>{ca, sa * uu, sa * rr * st, sa * rr * ct};
+}
+
+// the staple sum of U_mu(x) (get_staples.hh:26-80) in the storage precision.  Plain loads: with
+// programmatic launches the read-only cache may hold lines from before the previous pass.
+template <class T, int ND>
+__device__ __forceinline__ Su2<T> staple_sum(const Geom &g, const LinkT<T> *U, const Site &s, int mu,
+                                             T wt, T ws) {
+  const int p = s.p;
   const int lpm = s.lex + fwd_rt(g, s, mu);  // mu is known at run time only
-  Su2<float> K = zero_su2<float>();
+  Su2<T> K = zero_su2<T>();
 #pragma unroll
   for (int nu = 0; nu < ND; nu++) {
     if (nu == mu) continue;
     const int lpn = s.lex + fwd(g, s, nu);
-    const Su2<float> A = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, lpm, 1 - p));
-    const Su2<float> B = ld_link_rw(U + (size_t)mu * g.V + eo_of(g, lpn, 1 - p));
-    const Su2<float> D = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, s.lex, p));
+    const Su2<T> A = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, lpm, 1 - p));
+    const Su2<T> B = ld_link_rw(U + (size_t)mu * g.V + eo_of(g, lpn, 1 - p));
+    const Su2<T> D = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, s.lex, p));
     K = mul_acc(K, scale((nu == 0 || mu == 0) ? wt : ws, mul(A, dag(B))), dag(D));
   }
 #pragma unroll
   for (int nu = 0; nu < ND; nu++) {
     if (nu == mu) continue;
     const int b = bwd(g, s, nu);
-    const Su2<float> A = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, lpm + b, p));
-    const Su2<float> B = ld_link_rw(U + (size_t)mu * g.V + eo_of(g, s.lex + b, 1 - p));
-    const Su2<float> D = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, s.lex + b, 1 - p));
+    const Su2<T> A = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, lpm + b, p));
+    const Su2<T> B = ld_link_rw(U + (size_t)mu * g.V + eo_of(g, s.lex + b, 1 - p));
+    const Su2<T> D = ld_link_rw(U + (size_t)nu * g.V + eo_of(g, s.lex + b, 1 - p));
     K = mul_acc(K, scale((nu == 0 || mu == 0) ? wt : ws, mul(dag(A), dag(B))), D);
   }
-  const Su2<double> K64 = to64(K);
-  const size_t l = (size_t)mu * g.V + (size_t)p * g.Vh + cb;
-  Su2<float> u = ld_link_rw(U + l);
-  double tr_u = retr_mul(to64(u), K64);
-  const uint32_t lref = (uint32_t)(s.lex + g.lex0) * (uint32_t)g.nd + (uint32_t)mu;
-  const float d2 = (float)(2.0 * delta);
-  unsigned acc = 0;
-  for (int n = 0; n < N_hit; n++) {
-    uint32_t r[4];
-    philox(lref, (uint32_t)n, sweep, TAG_METRO, seed, r);
-    float sa, ca, st, ct;
-    sincospif(d2 * (float)u01_32(r[0]), &sa, &ca);
-    const float uu = fmaf(2.0f, (float)u01_32(r[1]), -1.0f);
-    sincospif(2.0f * (float)u01_32(r[2]), &st, &ct);
-    const float rr = sqrtf(fmaxf(0.0f, fmaf(-uu, uu, 1.0f)));
-    const Su2<float> R{ca, sa * uu, sa * rr * st, sa * rr * ct};
-    const Su2<float> uR = mul(u, R);
-    const double tr_uR = retr_mul(to64(uR), K64);
-    const double dS = beta_nc * (tr_u - tr_uR);
-    bool a = dS < 0;
-    if (!a) a = accept_fp64(u01_32(r[3]), dS);
-    if (a) {
-      u = from64<float>(restore_su(to64(uR)));
-      tr_u = retr_mul(to64(u), K64);
-      acc++;
-    }
-  }
-  st_link(U + l, u);
-  return acc;
+  return K;
+}
+// hit n: U -> U R with the accept test on dS = beta/Nc (ReTr(U K) - ReTr(U R K))
+template <class T>
+__device__ __forceinline__ unsigned metro_hit(Su2<T> &u, double &tr_u, const Su2<double> &K64,
+                                              const Su2<T> &R, double accept, double beta_nc) {
+  const Su2<T> uR = mul(u, R);
+  const double dS = beta_nc * (tr_u - retr_mul(to64(uR), K64));
+  const Su2<T> v = from64<T>(restore_near(to64(uR)));
+  const double tr_v = retr_mul(to64(v), K64);
+  if (!(dS < 0 || accept_fp64(accept, dS))) return 0;
+  u = v;
+  tr_u = tr_v;
+  return 1;
 }
 
-// eight resident blocks of 128 threads (64 registers, no spills): the FP64 pass takes 3 %
-// less time than with the compiler's free choice of 78 registers; FP32 links use 61 anyway
-template <class T, int ND, int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT)
+template <class T, int ND, int NT, int MINB>
+__global__ void __launch_bounds__(NT, MINB)
   k_metro_su2(Geom g, LinkT<T> *__restrict__ U, int mu, int p, double beta_nc, double delta,
-              int N_hit, uint64_t seed, uint32_t sweep, unsigned long long *counts, double wt,
-              double ws) {
+              int N_hit, uint64_t seed, uint32_t sweep, unsigned long long *counts, T wt, T ws) {
   __shared__ unsigned int sh_acc;
   if (threadIdx.x == 0) sh_acc = 0;
-  __syncthreads();
+  pdl_trigger();
   // the sites cb0 .. cb0 + ncb - 1 of parity p (all of them but in a time slab)
   const int cb = g.cb0 + blockIdx.x * NT + threadIdx.x;
+  const bool on = cb < g.cb0 + g.ncb;
+  const Site s = site_from_eo(g, p, on ? cb : g.cb0);
+  const uint32_t lref = (uint32_t)(s.lex + g.lex0) * (uint32_t)g.nd + (uint32_t)mu;
+  double ua;
+  Su2<T> R = proposal(lref, 0, sweep, seed, (T)delta, ua);
+  pdl_wait();  // the previous pass's links
+  __syncthreads();
   unsigned int acc = 0;
-  if constexpr (sizeof(T) == 4) {
-    if (cb < g.cb0 + g.ncb)
-      acc = metro_link_fp32<ND>(g, (Link32 *)U, mu, p, cb, beta_nc, delta, N_hit, seed, sweep,
-                                (float)wt, (float)ws);
-  } else if (cb < g.cb0 + g.ncb) {
-    const Site s = site_from_eo(g, p, cb);
-    // staple sum in FP64
-    const int lpm = s.lex + fwd_rt(g, s, mu);  // mu is known at run time only
-    Su2<double> K = zero_su2<double>();
-#pragma unroll
-    for (int nu = 0; nu < ND; nu++) {
-      if (nu == mu) continue;
-      const int lpn = s.lex + fwd(g, s, nu);
-      const Su2<double> A = to64(ld_link_rw(U + (size_t)nu * g.V + eo_of(g, lpm, 1 - p)));
-      const Su2<double> B = to64(ld_link_rw(U + (size_t)mu * g.V + eo_of(g, lpn, 1 - p)));
-      const Su2<double> D = to64(ld_link_rw(U + (size_t)nu * g.V + eo_of(g, s.lex, p)));
-      K = add(K, scale((nu == 0 || mu == 0) ? wt : ws, mul(mul(A, dag(B)), dag(D))));
-    }
-#pragma unroll
-    for (int nu = 0; nu < ND; nu++) {
-      if (nu == mu) continue;
-      const int b = bwd(g, s, nu);
-      const Su2<double> A = to64(ld_link_rw(U + (size_t)nu * g.V + eo_of(g, lpm + b, p)));
-      const Su2<double> B = to64(ld_link_rw(U + (size_t)mu * g.V + eo_of(g, s.lex + b, 1 - p)));
-      const Su2<double> D = to64(ld_link_rw(U + (size_t)nu * g.V + eo_of(g, s.lex + b, 1 - p)));
-      K = add(K, scale((nu == 0 || mu == 0) ? wt : ws, mul(mul(dag(A), dag(B)), D)));
-    }
+  if (on) {
+    const Su2<T> K = staple_sum<T, ND>(g, U, s, mu, wt, ws);
+    const Su2<double> K64 = to64(K);
     const size_t l = (size_t)mu * g.V + (size_t)p * g.Vh + cb;
-    Su2<double> u = to64(ld_link_rw(U + l));
-    const uint32_t lref = (uint32_t)(s.lex + g.lex0) * (uint32_t)g.nd + (uint32_t)mu;
+    Su2<T> u = ld_link_rw(U + l);
+    double tr_u = retr_mul(to64(u), K64);
     for (int n = 0; n < N_hit; n++) {
-      uint32_t r[4];
-      philox(lref, (uint32_t)n, sweep, TAG_METRO, seed, r);
-      double sa, ca, st, ct;
-      sincospi(2.0 * delta * u01_32(r[0]), &sa, &ca);
-      const double uu = 2.0 * u01_32(r[1]) - 1.0;
-      sincospi(2.0 * u01_32(r[2]), &st, &ct);
-      const double rr = sqrt(1.0 - uu * uu);
-      const Su2<double> R{ca, sa * uu, sa * rr * st, sa * rr * ct};
-      const Su2<double> uR = mul(u, R);
-      const double dS = beta_nc * (retr_mul(u, K) - retr_mul(uR, K));
-      bool a = dS < 0;
-      if (!a) a = accept_fp64(u01_32(r[3]), dS);
-      if (a) {
-        u = restore_su(uR);
-        acc++;
-      }
+      const Su2<T> Rn = R;
+      const double un = ua;
+      if (n + 1 < N_hit) R = proposal(lref, n + 1, sweep, seed, (T)delta, ua);
+      acc += metro_hit(u, tr_u, K64, Rn, un, beta_nc);
     }
-    st_link(U + l, from64<T>(u));
+    st_link(U + l, u);
   }
   if (acc) atomicAdd(&sh_acc, acc);
   __syncthreads();
   if (threadIdx.x == 0 && sh_acc) {
     atomicAdd(counts, (unsigned long long)sh_acc);
     if (mu == 0) atomicAdd(counts + 1, (unsigned long long)sh_acc);
+  }
+}
+
+// The same for passes of few links, which the chain of a link's hits bounds: a block of eight
+// warps takes 32 links; all warps draw proposals (they depend on nothing but the hit) into
+// shared memory, sixteen hits at a time and the first ones while the previous pass still runs,
+// and warp 0 applies them.  At 100^2, ten hits: 47 us per sweep, 57 us with
+// one thread per link (65 us before the chain of a hit lost its square root and division and the
+// passes their launch gaps).
+constexpr int WIDE_HITS = 16;
+template <class T, int ND>
+__global__ void __launch_bounds__(256, 2)
+  k_metro_su2_wide(Geom g, LinkT<T> *__restrict__ U, int mu, int p, double beta_nc, double delta,
+                   int N_hit, uint64_t seed, uint32_t sweep, unsigned long long *counts, T wt,
+                   T ws) {
+  __shared__ LinkT<T> prop[2][WIDE_HITS][32];
+  __shared__ double acc_u[2][WIDE_HITS][32];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int cb = g.cb0 + blockIdx.x * 32 + lane;
+  const bool on = cb < g.cb0 + g.ncb;
+  const Site s = site_from_eo(g, p, on ? cb : g.cb0);
+  const uint32_t lref = (uint32_t)(s.lex + g.lex0) * (uint32_t)g.nd + (uint32_t)mu;
+  auto draw = [&](int chunk, int first, int step) {
+    for (int i = first; i < WIDE_HITS && chunk * WIDE_HITS + i < N_hit; i += step)
+      prop[chunk & 1][i][lane] = as_link(proposal(lref, chunk * WIDE_HITS + i, sweep, seed, (T)delta,
+                                                  acc_u[chunk & 1][i][lane]));
+  };
+  draw(0, w, 8);
+  pdl_wait();  // the previous pass's links
+  const size_t l = (size_t)mu * g.V + s.p * (size_t)g.Vh + (s.lex >> 1);
+  Su2<T> u;
+  Su2<double> K64;
+  double tr_u = 0.;
+  if (w == 0) {
+    u = ld_link_rw(U + l);
+    K64 = to64(staple_sum<T, ND>(g, U, s, mu, wt, ws));
+    tr_u = retr_mul(to64(u), K64);
+  }
+  unsigned acc = 0;
+  for (int c = 0; c * WIDE_HITS < N_hit; c++) {
+    __syncthreads();
+    if (w == 0) {
+      const int n = min(WIDE_HITS, N_hit - c * WIDE_HITS);
+      for (int i = 0; i < n; i++)
+        acc += metro_hit(u, tr_u, K64, from_link(prop[c & 1][i][lane]), acc_u[c & 1][i][lane],
+                         beta_nc);
+    } else {
+      draw(c + 1, w - 1, 7);
+    }
+  }
+  if (w) return;
+  if (on)
+    st_link(U + l, u);
+  else
+    acc = 0;
+  acc = __reduce_add_sync(0xffffffffu, acc);
+  if (lane == 0 && acc) {
+    atomicAdd(counts, (unsigned long long)acc);
+    if (mu == 0) atomicAdd(counts + 1, (unsigned long long)acc);
   }
 }
 
@@ -239,7 +287,7 @@ template <class T>
 cudaError_t metropolis_pass(const Geom &g, void *U, int group, int mu, int parity, double beta,
                             double xi, double delta, int N_hit, uint64_t seed, uint32_t sweep,
                             unsigned long long *counts, cudaStream_t s) {
-  constexpr int NT = 128;
+  constexpr int NT = 128, MINB = 8;
   // anisotropic weights of get_staples (get_staples.hh:58-79): 1/xi for planes with
   // direction 0, xi otherwise; both 1 (exactly) for the isotropic action
   const double wt = xi == 1.0 ? 1.0 : 1.0 / xi, ws = xi;
@@ -247,36 +295,36 @@ cudaError_t metropolis_pass(const Geom &g, void *U, int group, int mu, int parit
   if (group == 0) {
     LinkT<T> *u = (LinkT<T> *)U;
     const double bn = beta / 2.0;
+    // up to two blocks of 32 links per SM the chain of a link's hits bounds a pass (10^4, eight
+    // hits: 73 us per sweep against 95 us); at 12^4, 10,368 links, the eight warps of a block
+    // cost more than they hide (109 us against 103 us)
+    const bool wide = g.ncb <= 2 * 148 * 32;
+#define SU2B_METRO(ND)                                                                     \
+  (wide ? launch_force(k_metro_su2_wide<T, ND>, dim3((g.ncb + 31) / 32), 256, s, true, 0, g, u, mu, \
+                       parity, bn, delta, N_hit, seed, sweep, counts, (T)wt, (T)ws)        \
+        : launch_force(k_metro_su2<T, ND, NT, MINB>, dim3(grid), NT, s, true, 0, g, u, mu, parity, bn, \
+                       delta, N_hit, seed, sweep, counts, (T)wt, (T)ws))
     switch (g.nd) {
-      case 2:
-        k_metro_su2<T, 2, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, bn, delta, N_hit, seed,
-                                                  sweep, counts, wt, ws);
-        break;
-      case 3:
-        k_metro_su2<T, 3, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, bn, delta, N_hit, seed,
-                                                  sweep, counts, wt, ws);
-        break;
-      default:
-        k_metro_su2<T, 4, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, bn, delta, N_hit, seed,
-                                                  sweep, counts, wt, ws);
-        break;
+      case 2: return SU2B_METRO(2);
+      case 3: return SU2B_METRO(3);
+      default: return SU2B_METRO(4);
     }
-  } else {
-    double *u = (double *)U;
-    switch (g.nd) {
-      case 2:
-        k_metro_u1<2, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, beta, delta, N_hit, seed, sweep,
-                                              counts, wt, ws);
-        break;
-      case 3:
-        k_metro_u1<3, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, beta, delta, N_hit, seed, sweep,
-                                              counts, wt, ws);
-        break;
-      default:
-        k_metro_u1<4, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, beta, delta, N_hit, seed, sweep,
-                                              counts, wt, ws);
-        break;
-    }
+#undef SU2B_METRO
+  }
+  double *u = (double *)U;
+  switch (g.nd) {
+    case 2:
+      k_metro_u1<2, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, beta, delta, N_hit, seed, sweep,
+                                            counts, wt, ws);
+      break;
+    case 3:
+      k_metro_u1<3, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, beta, delta, N_hit, seed, sweep,
+                                            counts, wt, ws);
+      break;
+    default:
+      k_metro_u1<4, NT><<<grid, NT, 0, s>>>(g, u, mu, parity, beta, delta, N_hit, seed, sweep,
+                                            counts, wt, ws);
+      break;
   }
   return cudaGetLastError();
 }

@@ -8,6 +8,30 @@ namespace su2b {
 
 template <class T> using LinkT = typename LinkOf<T>::type;
 
+// Programmatic dependent launch between the chained force launches of a trajectory: each
+// block lets the next launch start as soon as it is itself resident, and waits for the
+// previous launch to complete (and its writes to be visible) before it touches global
+// memory.  Both are no-ops for a launch without a programmatic dependency.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// launch with the programmatic-stream-serialization attribute when pdl is set
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_force(void (*kern)(KArgs...), dim3 grid, int nt, cudaStream_t s,
+                                bool pdl, size_t smem, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(nt);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // Prefetch into L1 of the momentum components of link l (SoA, NL apart): the force step
 // reads them only at its end, where every thread then waits on them; requested at the start
 // the lines arrive while the staples are summed (about 4 % of the launch at 32^4)

@@ -255,6 +255,24 @@ def test_metropolis_checkerboard(gpu, orc, group, dims, nd):
         np.testing.assert_array_equal(rates, r_want)
 
 
+# few links per pass (32 to a block, sixteen hits drawn at a time) and many (one thread each); the
+# last two sizes lie on the two sides of the rule, 9,472 links
+@pytest.mark.parametrize("dims,nd,hits", [((4, 4, 4, 4), 4, 0), ((4, 4, 4, 4), 4, 1),
+                                          ((6, 1, 1, 10), 2, 16), ((6, 1, 1, 10), 2, 17),
+                                          ((4, 6, 1, 10), 3, 35), ((12, 12, 12, 10), 4, 3),
+                                          ((12, 12, 12, 12), 4, 3)])
+def test_metropolis_pass_forms(gpu, orc, dims, nd, hits):
+    U = hot(orc, 0, dims, nd)
+    with make(gpu, 0, dims, nd, beta=2.3) as c:
+        c.upload(U)
+        for k in range(2):
+            U, want = orc.metropolis_checkerboard(0, dims, nd, 2.3, 0.3, hits, 99, k, U)
+            rates = c.sweep(0.3, hits, 99, k)
+            assert rel(c.download(), U) < 1e-11
+            if hits:
+                np.testing.assert_array_equal(rates, want)
+
+
 @pytest.mark.parametrize("group,dims,nd", [g for g in GEOMS if g[0] == 0],
                          ids=[i for g, i in zip(GEOMS, GEOM_IDS) if g[0] == 0])
 def test_metropolis_checkerboard_mixed_precision(gpu, orc, group, dims, nd):
