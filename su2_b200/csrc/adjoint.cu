@@ -408,8 +408,8 @@ int flow_adjoint_t(su2b_ctx *ctx, double eps, int n, int every, double *objectiv
   }
   cur = fa;
   // objective t^2 E_p(t), E_p = d(d-1)/2 - P/(V Nc) (flat-gradient_flow.hh:151)
-  SU2B_CKS(su2b_q_plaq(ctx, cur, 40));
-  SU2B_CKS(su2b_fetch_red(ctx, 43));
+  SU2B_CKS(su2b_q_plaq(ctx, cur, ctx->h_red + 40));
+  SU2B_CK(cudaStreamSynchronize(s));
   const double d = g.nd, t = n * eps, VNc = (double)ctx->V * ctx->Nc();
   if (objective) *objective = t * t * (d * (d - 1) / 2.0 - ctx->h_red[40] / VNc);
   if (!grad_host) return SU2B_OK;
@@ -455,8 +455,8 @@ extern "C" int su2b_action_backward(su2b_ctx *ctx, double grad_out, double *S, d
   ctx->begin_call();
   SU2B_CK(cudaSetDevice(ctx->device));
   if (S) {
-    SU2B_CKS(su2b_q_plaq(ctx, ctx->U, 40));
-    SU2B_CKS(su2b_fetch_red(ctx, 43));
+    SU2B_CKS(su2b_q_plaq(ctx, ctx->U, ctx->h_red + 40));
+    SU2B_CK(cudaStreamSynchronize(ctx->stream));
     *S = -ctx->beta * ctx->h_red[42] / ctx->Nc();
   }
   if (!dS_host) return SU2B_OK;

@@ -160,7 +160,8 @@ extern "C" int su2b_ctx_create(int group, int Lx, int Ly, int Lz, int Lt, int nd
       (st = dalloc(ctx, &ctx->part, sizeof(double) * 3 * ctx->part_cap * NSLOT)) ||
       (st = dalloc(ctx, &ctx->red, sizeof(double) * 64)) ||
       (st = dalloc(ctx, &ctx->traj, sizeof(TrajDev))) ||
-      (st = dalloc(ctx, &ctx->counts, sizeof(unsigned long long) * 4)))
+      (st = dalloc(ctx, &ctx->counts, sizeof(unsigned long long) * 4)) ||
+      (st = dalloc(ctx, &ctx->ticket, sizeof(unsigned))))
     return fin(st);
   if (cudaMallocHost((void **)&ctx->h_red, sizeof(double) * 64) != cudaSuccess ||
       cudaMallocHost((void **)&ctx->h_traj, sizeof(TrajDev)) != cudaSuccess ||
@@ -168,7 +169,9 @@ extern "C" int su2b_ctx_create(int group, int Lx, int Ly, int Lz, int Lt, int nd
       cudaMallocHost((void **)&ctx->h_st, sizeof(SolverState)) != cudaSuccess ||
       cudaMallocHost((void **)&ctx->h_tparams, sizeof(TrajParams)) != cudaSuccess)
     return fin(SU2B_ERR_NOMEM);
-  if (cudaMemsetAsync(ctx->U, 0, lb * NL, ctx->stream) != cudaSuccess) return fin(SU2B_ERR_CUDA);
+  if (cudaMemsetAsync(ctx->U, 0, lb * NL, ctx->stream) != cudaSuccess ||
+      cudaMemsetAsync(ctx->ticket, 0, sizeof(unsigned), ctx->stream) != cudaSuccess)
+    return fin(SU2B_ERR_CUDA);
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fin(SU2B_ERR_CUDA);
   return fin(SU2B_OK);
 }
@@ -335,24 +338,24 @@ int su2b_adj_download(su2b_ctx *ctx, const void *dev, double *host) {
 
 // ------------------------------------------------------------------------------------
 // reductions (queued; results land in ctx->red[slot..])
-int su2b_q_plaq(su2b_ctx *ctx, const void *U, int red_slot) {
+int su2b_q_plaq(su2b_ctx *ctx, const void *U, double *out) {
   int nb = 0;
   double *part = ctx->part_slot(0);
+  const Finish fin{out, ctx->ticket};
   if (ctx->link64)
-    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_partials<double>(ctx->g, U, ctx->group, ctx->xi, part, &nb, ctx->stream));
+    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_partials<double>(ctx->g, U, ctx->group, ctx->xi, part, &nb, ctx->stream, fin));
   else
-    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_partials<float>(ctx->g, U, ctx->group, ctx->xi, part, &nb, ctx->stream));
-  SU2B_LAUNCH(SU2B_K_OTHER, reduce_final(part, nb, 3, ctx->red + red_slot, ctx->stream));
+    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_partials<float>(ctx->g, U, ctx->group, ctx->xi, part, &nb, ctx->stream, fin));
   return SU2B_OK;
 }
-int su2b_q_clover(su2b_ctx *ctx, const void *U, int cloverdef, int red_slot) {
+int su2b_q_clover(su2b_ctx *ctx, const void *U, int cloverdef, double *out) {
   int nb = 0;
   double *part = ctx->part_slot(2);
+  const Finish fin{out, ctx->ticket};
   if (ctx->link64)
-    SU2B_LAUNCH(SU2B_K_CLOVER, clover_partials<double>(ctx->g, U, ctx->group, cloverdef, part, &nb, ctx->stream));
+    SU2B_LAUNCH(SU2B_K_CLOVER, clover_partials<double>(ctx->g, U, ctx->group, cloverdef, part, &nb, ctx->stream, fin));
   else
-    SU2B_LAUNCH(SU2B_K_CLOVER, clover_partials<float>(ctx->g, U, ctx->group, cloverdef, part, &nb, ctx->stream));
-  SU2B_LAUNCH(SU2B_K_OTHER, reduce_final(part, nb, 3, ctx->red + red_slot, ctx->stream));
+    SU2B_LAUNCH(SU2B_K_CLOVER, clover_partials<float>(ctx->g, U, ctx->group, cloverdef, part, &nb, ctx->stream, fin));
   return SU2B_OK;
 }
 int su2b_fetch_red(su2b_ctx *ctx, int n) {
@@ -365,8 +368,8 @@ int su2b_fetch_red(su2b_ctx *ctx, int n) {
 extern "C" int su2b_gauge_energy(su2b_ctx *ctx, int spatial_only, double *out) {
   CKS(enter(ctx));
   NEED(out, "out is NULL");
-  CKS(su2b_q_plaq(ctx, ctx->U, 0));
-  CKS(su2b_fetch_red(ctx, 3));
+  CKS(su2b_q_plaq(ctx, ctx->U, ctx->h_red));
+  CK(cudaStreamSynchronize(ctx->stream));
   *out = ctx->h_red[spatial_only ? 1 : 0];
   return SU2B_OK;
 }
@@ -375,16 +378,16 @@ extern "C" int su2b_retr_sum_plaquettes(su2b_ctx *ctx, int spatial_only, double 
   NEED(out, "out is NULL");
   if (ctx->xi == 1.0) return su2b_gauge_energy(ctx, spatial_only, out);
   NEED(!spatial_only, "anisotropic spatial-only plaquette sums are not provided");
-  CKS(su2b_q_plaq(ctx, ctx->U, 0));
-  CKS(su2b_fetch_red(ctx, 3));
+  CKS(su2b_q_plaq(ctx, ctx->U, ctx->h_red));
+  CK(cudaStreamSynchronize(ctx->stream));
   *out = ctx->h_red[2];
   return SU2B_OK;
 }
 extern "C" int su2b_gauge_action(su2b_ctx *ctx, double *out) {
   CKS(enter(ctx));
   NEED(out, "out is NULL");
-  CKS(su2b_q_plaq(ctx, ctx->U, 0));
-  CKS(su2b_fetch_red(ctx, 3));
+  CKS(su2b_q_plaq(ctx, ctx->U, ctx->h_red));
+  CK(cudaStreamSynchronize(ctx->stream));
   *out = -ctx->beta * ctx->h_red[2] / ctx->Nc();
   return SU2B_OK;
 }
@@ -405,8 +408,8 @@ extern "C" int su2b_energy_density(su2b_ctx *ctx, int cloverdef, int ss, double 
                                    double *Q) {
   CKS(enter(ctx));
   NEED(E && Q, "E or Q is NULL");
-  CKS(su2b_q_clover(ctx, ctx->U, cloverdef, 0));
-  CKS(su2b_fetch_red(ctx, 3));
+  CKS(su2b_q_clover(ctx, ctx->U, cloverdef, ctx->h_red));
+  CK(cudaStreamSynchronize(ctx->stream));
   su2b_finish_clover(ctx->h_red, (double)ctx->V, cloverdef, ss, E, Q);
   return SU2B_OK;
 }
@@ -581,31 +584,28 @@ extern "C" int su2b_gradient_flow(su2b_ctx *ctx, double tmax, double eps, double
   const double den = (double)ctx->V * ctx->Nc();
   double t[3] = {tstart, tstart, tstart};
   int nr = 0;
-  while (t[1] < tmax - eps) {
-    t[0] = t[2];
-    t[1] = t[0] + eps;
-    // two steps per record, Vt -> U2 -> Vt, every stage fused with its link update
-    CKS(su2b_q_flow_step_to(ctx, Vt, ctx->U2, eps));
-    // the reference prints the observables of the middle step only
-    CKS(su2b_q_plaq(ctx, ctx->U2, 0));
-    CKS(su2b_q_clover(ctx, ctx->U2, 1, 3));
-    t[2] = t[1] + eps;
-    CKS(su2b_q_flow_step_to(ctx, ctx->U2, Vt, eps));
-    CKS(su2b_fetch_red(ctx, 6));
-    const double *r = ctx->h_red;
-    const double P1 = r[0] / den, Pss1 = r[1] / den;
-    double E1, Q1, Ess1, Qss1;
-    su2b_finish_clover(r + 3, (double)ctx->V, 1, 0, &E1, &Q1);
-    su2b_finish_clover(r + 3, (double)ctx->V, 1, 1, &Ess1, &Qss1);
-    const double Ep = ndims_fact - P1;
-    const double Ep_ss = ndims_fact_ss - Pss1;
-    const double Ep_ts = Ep - Ep_ss;
-    const double Ep_ts_bar = Ep_ts / (double)(d - 1);
-    const double Ep_ss_bar = Ep_ss / ndims_fact_ss;
-    const double xi_R = sqrt(Ep_ts_bar / Ep_ss_bar);
-    if (nr < max_rows) {
+  // the sums of up to ten records land in h_red while the next steps are already queued: the
+  // device waits for the host once in ten records
+  constexpr int QUEUED = 10;
+  double t1[QUEUED];
+  int queued = 0;
+  auto flush = [&]() -> int {
+    CK(cudaStreamSynchronize(ctx->stream));
+    for (int k = 0; k < queued; k++, nr++) {
+      if (nr >= max_rows) continue;
+      const double *r = ctx->h_red + 6 * k;
+      const double P1 = r[0] / den, Pss1 = r[1] / den;
+      double E1, Q1, Ess1, Qss1;
+      su2b_finish_clover(r + 3, (double)ctx->V, 1, 0, &E1, &Q1);
+      su2b_finish_clover(r + 3, (double)ctx->V, 1, 1, &Ess1, &Qss1);
+      const double Ep = ndims_fact - P1;
+      const double Ep_ss = ndims_fact_ss - Pss1;
+      const double Ep_ts = Ep - Ep_ss;
+      const double Ep_ts_bar = Ep_ts / (double)(d - 1);
+      const double Ep_ss_bar = Ep_ss / ndims_fact_ss;
+      const double xi_R = sqrt(Ep_ts_bar / Ep_ss_bar);
       double *o = rows + 9 * (size_t)nr;
-      o[0] = t[1];
+      o[0] = t1[k];
       o[1] = xi_R;
       o[2] = P1;
       o[3] = Pss1;
@@ -615,9 +615,23 @@ extern "C" int su2b_gradient_flow(su2b_ctx *ctx, double tmax, double eps, double
       o[7] = Ess1;
       o[8] = Q1;
     }
-    nr++;
+    queued = 0;
+    return SU2B_OK;
+  };
+  while (t[1] < tmax - eps) {
+    t[0] = t[2];
+    t[1] = t[0] + eps;
+    // two steps per record, Vt -> U2 -> Vt, every stage fused with its link update
+    CKS(su2b_q_flow_step_to(ctx, Vt, ctx->U2, eps));
+    // the reference prints the observables of the middle step only
+    CKS(su2b_q_plaq(ctx, ctx->U2, ctx->h_red + 6 * queued));
+    CKS(su2b_q_clover(ctx, ctx->U2, 1, ctx->h_red + 6 * queued + 3));
+    t1[queued++] = t[1];
+    t[2] = t[1] + eps;
+    CKS(su2b_q_flow_step_to(ctx, ctx->U2, Vt, eps));
+    if (queued == QUEUED) CKS(flush());
   }
-  CK(cudaStreamSynchronize(ctx->stream));
+  CKS(flush());
   *n_rows = nr;
   return SU2B_OK;
 }

@@ -111,27 +111,25 @@ __global__ void k_spinor_to_host(Geom g, const double2 *__restrict__ psi, double
 // plaquettes: per site, sum over planes mu<nu of ReTr U_mu(x) U_nu(x+mu) U_mu(x+nu)^+ U_nu(x)^+
 // (flat-gauge_energy.hpp:31-94), FP64 products.  Partials {full, spatial, xi-weighted}.
 // Resident blocks of 256 threads: four with FP32 links (64 registers), three with FP64 links
-// (80 registers, no spills; the plaquette call 67 against 71 us at 32^4 with two)
+// (80 registers, no spills; the plaquette call 67 against 71 us at 32^4 with two).  The
+// plaquette kernel's blocks stay and take band after band of 32 sites of one parity, so there
+// is one wave of them to finish: 55 us at 32^4, 27 us at 24^4 (35 with a block per band and the
+// sum in a second launch).
 template <class T, int NT> constexpr int plaq_min_blocks() {
   return sizeof(T) == 8 ? 768 / NT : 1024 / NT;
 }
 
 template <class T, int ND, int NT>
 __global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
-  k_plaq_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part) {
-  __shared__ double shk[4 * (NT / 32)];
-  const int w = threadIdx.x >> 5, p = w & 1;
-  const int cb = g.cb0 + blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
-  double full = 0., spat = 0., wsum = 0.;
-  if (cb < g.cb0 + g.ncb) plaq_site<T, ND>(g, U, p, cb, xi, full, spat, wsum);
-  const int b = blockIdx.x;
-  double v[3] = {full, spat, wsum};
-  block_sums<NT, 3>(v, shk);
-  if (threadIdx.x == 0) {
-    part[3 * b] = v[0];
-    part[3 * b + 1] = v[1];
-    part[3 * b + 2] = v[2];
+  k_plaq_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part, Finish fin) {
+  __shared__ double shk[3 * (NT / 32)];
+  double v[3] = {0., 0., 0.};
+  for (int c = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); 32 * (c >> 1) < g.ncb;
+       c += gridDim.x * (NT / 32)) {  // band c/2 of 32 sites, parity c%2
+    const int b = 32 * (c >> 1) + (threadIdx.x & 31);
+    if (b < g.ncb) plaq_site<T, ND>(g, U, c & 1, g.cb0 + b, xi, v[0], v[1], v[2]);
   }
+  finish_sums<NT, 3>(v, part, fin, shk);
 }
 
 // The start of a trajectory in one pass over the sites: the Philox momenta of the site's
@@ -178,8 +176,8 @@ __global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
 
 template <int ND, int NT>
 __global__ void __launch_bounds__(NT)
-  k_plaq_u1(Geom g, const double *__restrict__ U, double xi, double *part) {
-  __shared__ double shk[4 * (NT / 32)];
+  k_plaq_u1(Geom g, const double *__restrict__ U, double xi, double *part, Finish fin) {
+  __shared__ double shk[3 * (NT / 32)];
   const int w = threadIdx.x >> 5, p = w & 1;
   const int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
   double full = 0., spat = 0., wsum = 0.;
@@ -203,14 +201,8 @@ __global__ void __launch_bounds__(NT)
       }
     }
   }
-  const int b = blockIdx.x;
   double v[3] = {full, spat, wsum};
-  block_sums<NT, 3>(v, shk);
-  if (threadIdx.x == 0) {
-    part[3 * b] = v[0];
-    part[3 * b + 1] = v[1];
-    part[3 * b + 2] = v[2];
-  }
+  finish_sums<NT, 3>(v, part, fin, shk);
 }
 
 // out[k] = sum over b of part[b*ncomp + k], one block, in an order fixed by n: thread t sums
@@ -635,23 +627,24 @@ cudaError_t spinor_to_host(const Geom &g, const double2 *psi, double *aos, cudaS
 
 template <class T>
 cudaError_t plaq_partials(const Geom &g, const void *U, int group, double xi, double *part,
-                          int *nblocks, cudaStream_t s) {
+                          int *nblocks, cudaStream_t s, Finish fin) {
   constexpr int NT = 256;
-  const dim3 grid(cdiv(group == 0 ? g.ncb : g.Vh, NT / 2));
+  const dim3 grid(group == 0 ? min(cdiv(g.ncb, NT / 2), 148 * plaq_min_blocks<T, NT>())
+                             : cdiv(g.Vh, NT / 2));
   *nblocks = grid.x;
   if (group == 0) {
     const LinkT<T> *u = (const LinkT<T> *)U;
     switch (g.nd) {
-      case 2: k_plaq_su2<T, 2, NT><<<grid, NT, 0, s>>>(g, u, xi, part); break;
-      case 3: k_plaq_su2<T, 3, NT><<<grid, NT, 0, s>>>(g, u, xi, part); break;
-      default: k_plaq_su2<T, 4, NT><<<grid, NT, 0, s>>>(g, u, xi, part); break;
+      case 2: k_plaq_su2<T, 2, NT><<<grid, NT, 0, s>>>(g, u, xi, part, fin); break;
+      case 3: k_plaq_su2<T, 3, NT><<<grid, NT, 0, s>>>(g, u, xi, part, fin); break;
+      default: k_plaq_su2<T, 4, NT><<<grid, NT, 0, s>>>(g, u, xi, part, fin); break;
     }
   } else {
     const double *u = (const double *)U;
     switch (g.nd) {
-      case 2: k_plaq_u1<2, NT><<<grid, NT, 0, s>>>(g, u, xi, part); break;
-      case 3: k_plaq_u1<3, NT><<<grid, NT, 0, s>>>(g, u, xi, part); break;
-      default: k_plaq_u1<4, NT><<<grid, NT, 0, s>>>(g, u, xi, part); break;
+      case 2: k_plaq_u1<2, NT><<<grid, NT, 0, s>>>(g, u, xi, part, fin); break;
+      case 3: k_plaq_u1<3, NT><<<grid, NT, 0, s>>>(g, u, xi, part, fin); break;
+      default: k_plaq_u1<4, NT><<<grid, NT, 0, s>>>(g, u, xi, part, fin); break;
     }
   }
   return cudaGetLastError();
@@ -961,7 +954,7 @@ cudaError_t cond_restore(const Geom &g, void *U, const void *U_old, int group,
   template cudaError_t adj_from_host<T>(const Geom &, const double *, T *, int, cudaStream_t); \
   template cudaError_t adj_to_host<T>(const Geom &, const T *, double *, int, cudaStream_t);   \
   template cudaError_t plaq_partials<T>(const Geom &, const void *, int, double, double *,   \
-                                        int *, cudaStream_t);                                 \
+                                        int *, cudaStream_t, Finish);                                 \
   template cudaError_t force_update<T>(const Geom &, const void *, int, T *, const T *,      \
                                        double, double, double, int, double *, int *, void *,  \
                                        double, cudaStream_t, int, bool);                      \

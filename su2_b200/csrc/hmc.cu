@@ -212,7 +212,7 @@ int enqueue_fused(su2b_ctx *ctx, const std::vector<FOp> &fops, bool host_momenta
                                                       ctx->xi, ctx->part_slot(1), &nb_start, s,
                                                       !cached));
   } else {
-    SU2B_CKS(su2b_q_plaq(ctx, S, 1));
+    SU2B_CKS(su2b_q_plaq(ctx, S, ctx->red + 1));
   }
   const double f = ctx->beta / ctx->Nc();
   void *cur = S;
@@ -417,11 +417,11 @@ extern "C" int su2b_hmc_trajectory(su2b_ctx *ctx, const su2b_hmc_params *prm,
     SU2B_CKS(su2b_fermion_heatbath_q(ctx, prm->fermion_mass, prm->pf_source_host, prm->seed,
                                      prm->traj, prm->pf_complex, 8));
   // S_G old -> red[1..3]
-  SU2B_CKS(su2b_q_plaq(ctx, ctx->U, 1));
+  SU2B_CKS(su2b_q_plaq(ctx, ctx->U, ctx->red + 1));
   SU2B_CK(cudaMemcpyAsync(ctx->U_old, ctx->U, ctx->link_bytes() * ctx->NL,
                           cudaMemcpyDeviceToDevice, s));
   SU2B_CKS(integrate(ctx, ops, prm, 4, &cg_iters));
-  SU2B_CKS(su2b_q_plaq(ctx, ctx->U, 5));
+  SU2B_CKS(su2b_q_plaq(ctx, ctx->U, ctx->red + 5));
   if (ferm) {
     long it = 0;
     SU2B_CKS(su2b_fermion_action_q(ctx, prm->fermion_mass, prm->cg_tol, prm->cg_max_iter,
@@ -442,7 +442,7 @@ extern "C" int su2b_hmc_trajectory(su2b_ctx *ctx, const su2b_hmc_params *prm,
     else
       SU2B_LAUNCH(SU2B_K_OTHER, negate_adj<float>(ctx->g, (float *)ctx->P, ctx->group, s));
     SU2B_CKS(integrate(ctx, ops, prm, 10, &cg_iters));
-    SU2B_CKS(su2b_q_plaq(ctx, ctx->U, 11));
+    SU2B_CKS(su2b_q_plaq(ctx, ctx->U, ctx->red + 11));
     SU2B_CK(cudaMemsetAsync(ctx->red + 14, 0, sizeof(double), s));
     if (ferm) {
       long it = 0;

@@ -4,6 +4,7 @@
 // All three read the device links in the even/odd layout; products are accumulated in FP64
 // whatever the link storage (FP32 links of a mixed-precision context are promoted), and sums
 // go through per-block partials reduced in a fixed order.
+#include <algorithm>
 #include <utility>
 #include "site_ops.cuh"
 #include "su2b.h"
@@ -59,95 +60,124 @@ struct Point {
   __device__ __forceinline__ int par() const { return (c0 + c1 + c2 + c3) & 1; }
 };
 
-// polyakov_loop (polyakov_loop.hh:26-38): one thread per spatial point, the product of the
-// temporal links along t, ReTr (SU(2): 2 Re a; U(1): Re of the phase product)
-template <class T, int NT>
-__global__ void __launch_bounds__(NT)
-  k_polyakov(Geom g, const void *__restrict__ Uv, int group, double *part) {
-  __shared__ double sh[NT / 32];
+// polyakov_loop (polyakov_loop.hh:26-38): the product of the temporal links along t over each
+// spatial point, ReTr (SU(2): 2 Re a; U(1): Re of the phase product).  A point's line is one
+// chain of products, and there are few points (4096 at 16^4), so eight warps take eight
+// segments of the lines of 32 points and their products are joined pairwise, in the order of
+// t, in shared memory: a call at 16^4 takes 17 us, 23 us with one thread per point and a second
+// launch for the sum, and 25 us against 30 us at 32^4.
+template <class T>
+__global__ void __launch_bounds__(256)
+  k_polyakov(Geom g, const void *__restrict__ Uv, int group, double *part, Finish fin) {
+  __shared__ double sh[8];
+  __shared__ Su2<double> line[8][32];
   const int V3 = g.L[1] * g.L[2] * g.L[3];
-  const int s3 = blockIdx.x * NT + threadIdx.x;
-  double v = 0.;
+  const int lane = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const int s3 = blockIdx.x * 32 + lane;
+  const int per = (g.L[0] + 7) / 8, t0 = min(seg * per, g.L[0]), t1 = min(t0 + per, g.L[0]);
+  Su2<double> P{1.0, 0.0, 0.0, 0.0};  // U(1): the phase product in (ar, ai)
   if (s3 < V3) {
     const int z = s3 % g.L[3], y = (s3 / g.L[3]) % g.L[2], x = s3 / (g.L[3] * g.L[2]);
     if (group == 0) {
       const LinkT<T> *U = (const LinkT<T> *)Uv;
-      Su2<double> P{1.0, 0.0, 0.0, 0.0};
-      for (int t = 0; t < g.L[0]; t++) P = mul(P, link_at<T>(g, U, 0, t * V3 + s3, (t + x + y + z) & 1));
-      v = retr(P);
+#pragma unroll 4
+      for (int t = t0; t < t1; t++)
+        P = mul(P, link_at<T>(g, U, 0, t * V3 + s3, (t + x + y + z) & 1));
     } else {
       const double *U = (const double *)Uv;
-      double2 P = make_double2(1.0, 0.0);
-      for (int t = 0; t < g.L[0]; t++)
-        P = cmul2(P, phase(angle_at(g, U, 0, t * V3 + s3, (t + x + y + z) & 1)));
-      v = P.x;
+      double2 e = make_double2(1.0, 0.0);
+      for (int t = t0; t < t1; t++)
+        e = cmul2(e, phase(angle_at(g, U, 0, t * V3 + s3, (t + x + y + z) & 1)));
+      P.ar = e.x;
+      P.ai = e.y;
     }
   }
-  const double r = block_sum<NT>(v, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = r;
+  line[seg][lane] = P;
+#pragma unroll
+  for (int h = 1; h < 8; h *= 2) {
+    __syncthreads();
+    if (seg % (2 * h) == 0) {
+      P = mul(P, line[seg + h][lane]);
+      line[seg][lane] = P;
+    }
+  }
+  double v[1] = {seg == 0 && s3 < V3 ? (group == 0 ? retr(P) : P.ar) : 0.};
+  finish_sums<256, 1>(v, part, fin, sh);
 }
 
 // planar_wilsonloop_dir (wilsonloop.hh:51-91) summed over the planes (mu, 0), mu >= 1, by
-// wilsonloop (wilsonloop.hh:147-157): one thread per site, loop x -> +t e_0 -> +r e_mu ->
-// -t e_0 -> -r e_mu
+// wilsonloop (wilsonloop.hh:147-157): the loop x -> +t e_0 -> +r e_mu -> -t e_0 -> -r e_mu as
+//   ReTr [T(x) S(x+t)] [S(x) T(x+r)]^+
+// of straight lines walked forwards.  One thread per site takes all planes: T(x) is the same
+// in each, and the two S lines are walked side by side; 40 links are read for a 4 x 4 loop in
+// d = 4 where the walk around it reads 48, and the chain of products is half as long.  Bound
+// by those reads, which L2 serves: a call takes 118 us at 32^4 and 25 us at 16^4, 131 us and
+// 32 us with the walk around the loop.  Eight blocks per SM (64 registers); twelve spill and
+// take 195 us.
+constexpr int WILSON_BLOCKS = 8;
 template <class T, int NT>
-__global__ void __launch_bounds__(NT)
-  k_wilson(Geom g, const void *__restrict__ Uv, int group, int R, int Tt, double *part) {
+__global__ void __launch_bounds__(NT, WILSON_BLOCKS)
+  k_wilson(Geom g, const void *__restrict__ Uv, int group, int R, int Tt, double *part,
+           Finish fin) {
   __shared__ double sh[NT / 32];
-  const int lex0 = blockIdx.x * NT + threadIdx.x;
-  double v = 0.;
-  if (lex0 < g.V) {
-    const Site s0 = site_from_lex(g, lex0);
-    for (int mu = 1; mu < g.nd; mu++) {
-      Point c(s0);
-      auto step = [&](int d, int dir) { c.step(g, d, dir); };
-      auto here = [&]() { return c.lex(g); };
-      auto par = [&]() { return c.par(); };
-      if (group == 0) {
-        const LinkT<T> *U = (const LinkT<T> *)Uv;
-        Su2<double> L{1.0, 0.0, 0.0, 0.0};
-        for (int k = 0; k < Tt; k++) {
-          L = mul(L, link_at<T>(g, U, 0, here(), par()));
-          step(0, 1);
+  double v[1] = {0.};
+  for (int x = blockIdx.x * NT + threadIdx.x; x < g.V; x += gridDim.x * NT) {
+    const Site s = site_from_lex(g, x);
+    const int Lt = g.L[0], st = g.st[0];
+    // a point on a line: the coordinate c along it, its index and parity
+    struct Walk {
+      int c, lex, par;
+      __device__ __forceinline__ void step(int L, int st) {
+        const bool wrap = ++c == L;
+        lex += wrap ? -(L - 1) * st : st;
+        if (wrap) c = 0;
+        par ^= 1;  // active extents are even: a wrap changes the parity as a step does
+      }
+    };
+    Walk w{s.c[0], x, s.p};
+    if (group == 0) {
+      const LinkT<T> *U = (const LinkT<T> *)Uv;
+      Su2<double> T0{1.0, 0.0, 0.0, 0.0};
+#pragma unroll 4
+      for (int i = 0; i < Tt; i++, w.step(Lt, st)) T0 = mul(T0, link_at<T>(g, U, 0, w.lex, w.par));
+      for (int mu = 1; mu < g.nd; mu++) {
+        const int Lm = pick4(mu, g.L[0], g.L[1], g.L[2], g.L[3]);
+        const int sm = pick4(mu, g.st[0], g.st[1], g.st[2], g.st[3]);
+        Walk a{coord_rt(s, mu), w.lex, w.par}, b{a.c, x, s.p};
+        Su2<double> A = T0, B{1.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+        for (int i = 0; i < R; i++, a.step(Lm, sm), b.step(Lm, sm)) {
+          A = mul(A, link_at<T>(g, U, mu, a.lex, a.par));
+          B = mul(B, link_at<T>(g, U, mu, b.lex, b.par));
         }
-        for (int k = 0; k < R; k++) {
-          L = mul(L, link_at<T>(g, U, mu, here(), par()));
-          step(mu, 1);
+        b.c = s.c[0];
+#pragma unroll 4
+        for (int i = 0; i < Tt; i++, b.step(Lt, st))
+          B = mul(B, link_at<T>(g, U, 0, b.lex, b.par));
+        v[0] += retr_mul(A, dag(B));
+      }
+    } else {
+      const double *U = (const double *)Uv;
+      double2 T0 = make_double2(1.0, 0.0);
+      for (int i = 0; i < Tt; i++, w.step(Lt, st))
+        T0 = cmul2(T0, phase(angle_at(g, U, 0, w.lex, w.par)));
+      for (int mu = 1; mu < g.nd; mu++) {
+        const int Lm = pick4(mu, g.L[0], g.L[1], g.L[2], g.L[3]);
+        const int sm = pick4(mu, g.st[0], g.st[1], g.st[2], g.st[3]);
+        Walk a{coord_rt(s, mu), w.lex, w.par}, b{a.c, x, s.p};
+        double2 A = T0, B = make_double2(1.0, 0.0);
+        for (int i = 0; i < R; i++, a.step(Lm, sm), b.step(Lm, sm)) {
+          A = cmul2(A, phase(angle_at(g, U, mu, a.lex, a.par)));
+          B = cmul2(B, phase(angle_at(g, U, mu, b.lex, b.par)));
         }
-        for (int k = 0; k < Tt; k++) {
-          step(0, -1);
-          L = mul(L, dag(link_at<T>(g, U, 0, here(), par())));
-        }
-        for (int k = 0; k < R; k++) {
-          step(mu, -1);
-          L = mul(L, dag(link_at<T>(g, U, mu, here(), par())));
-        }
-        v += retr(L);
-      } else {
-        const double *U = (const double *)Uv;
-        double2 L = make_double2(1.0, 0.0);
-        for (int k = 0; k < Tt; k++) {
-          L = cmul2(L, phase(angle_at(g, U, 0, here(), par())));
-          step(0, 1);
-        }
-        for (int k = 0; k < R; k++) {
-          L = cmul2(L, phase(angle_at(g, U, mu, here(), par())));
-          step(mu, 1);
-        }
-        for (int k = 0; k < Tt; k++) {
-          step(0, -1);
-          L = cmul2(L, phase(-angle_at(g, U, 0, here(), par())));
-        }
-        for (int k = 0; k < R; k++) {
-          step(mu, -1);
-          L = cmul2(L, phase(-angle_at(g, U, mu, here(), par())));
-        }
-        v += L.x;
+        b.c = s.c[0];
+        for (int i = 0; i < Tt; i++, b.step(Lt, st))
+          B = cmul2(B, phase(angle_at(g, U, 0, b.lex, b.par)));
+        v[0] += A.x * B.x + A.y * B.y;
       }
     }
   }
-  const double r = block_sum<NT>(v, sh);
-  if (threadIdx.x == 0) part[blockIdx.x] = r;
+  finish_sums<NT, 1>(v, part, fin, sh);
 }
 
 // APEsmearing (smearape.hh:97-131) with get_staples_APE (get_staples.hh:89-110), one thread
@@ -244,17 +274,17 @@ extern "C" int su2b_polyakov_loop(su2b_ctx *ctx, double *out) {
   SU2B_CKS(enter_ctx(ctx));
   SU2B_NEED(out, "out is NULL");
   const int V3 = ctx->g.L[1] * ctx->g.L[2] * ctx->g.L[3];
-  const int nb = (V3 + NT_O - 1) / NT_O;
+  const int nb = (V3 + 31) / 32;
   double *part = ctx->part_slot(0);
+  const Finish fin{ctx->h_red, ctx->ticket};
   if (ctx->link64)
-    k_polyakov<double, NT_O><<<nb, NT_O, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, part);
+    k_polyakov<double><<<nb, 256, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, part, fin);
   else
-    k_polyakov<float, NT_O><<<nb, NT_O, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, part);
+    k_polyakov<float><<<nb, 256, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, part, fin);
   SU2B_CK(cudaGetLastError());
   ctx->launches++;
-  SU2B_LAUNCH(SU2B_K_OTHER, reduce_final(part, nb, 1, ctx->red + 48, ctx->stream));
-  SU2B_CKS(su2b_fetch_red(ctx, 49));
-  *out = ctx->h_red[48] / (double)ctx->V;
+  SU2B_CK(cudaStreamSynchronize(ctx->stream));
+  *out = ctx->h_red[0] / (double)ctx->V;
   return SU2B_OK;
 }
 
@@ -264,17 +294,18 @@ extern "C" int su2b_wilson_loop(su2b_ctx *ctx, int r, int t, double *out) {
   SU2B_CKS(enter_ctx(ctx));
   SU2B_NEED(out, "out is NULL");
   SU2B_NEED(r >= 0 && t >= 0, "loop extents must be non-negative");
-  const int nb = (ctx->g.V + NT_O - 1) / NT_O;
+  constexpr int NT = 128;
+  const int nb = std::min((ctx->g.V + NT - 1) / NT, 148 * WILSON_BLOCKS);
   double *part = ctx->part_slot(0);
+  const Finish fin{ctx->h_red, ctx->ticket};
   if (ctx->link64)
-    k_wilson<double, NT_O><<<nb, NT_O, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, r, t, part);
+    k_wilson<double, NT><<<nb, NT, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, r, t, part, fin);
   else
-    k_wilson<float, NT_O><<<nb, NT_O, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, r, t, part);
+    k_wilson<float, NT><<<nb, NT, 0, ctx->stream>>>(ctx->g, ctx->U, ctx->group, r, t, part, fin);
   SU2B_CK(cudaGetLastError());
   ctx->launches++;
-  SU2B_LAUNCH(SU2B_K_OTHER, reduce_final(part, nb, 1, ctx->red + 48, ctx->stream));
-  SU2B_CKS(su2b_fetch_red(ctx, 49));
-  *out = ctx->h_red[48] / (double)ctx->V / (double)ctx->Nc() / (double)ctx->g.nd;
+  SU2B_CK(cudaStreamSynchronize(ctx->stream));
+  *out = ctx->h_red[0] / (double)ctx->V / (double)ctx->Nc() / (double)ctx->g.nd;
   return SU2B_OK;
 }
 

@@ -849,8 +849,8 @@ int flow_step(su2b_slabs *h, int a, int b, double eps) {
 int measure(su2b_slabs *h, int k, int cloverdef, int slot) {
   for (int r = 0; r < h->count; r++) {
     su2b_ctx *c = h->sl[r];
-    int rc = su2b_q_plaq(c, h->buf[r][k], slot);
-    if (rc == SU2B_OK) rc = su2b_q_clover(c, h->buf[r][k], cloverdef, slot + 3);
+    int rc = su2b_q_plaq(c, h->buf[r][k], c->red + slot);
+    if (rc == SU2B_OK) rc = su2b_q_clover(c, h->buf[r][k], cloverdef, c->red + slot + 3);
     if (rc != SU2B_OK) return from_ctx(h, rc);
   }
   return SU2B_OK;

@@ -37,6 +37,7 @@ struct su2b_ctx {
   su2b::TrajDev *traj = nullptr;
   su2b::TrajParams *tparams = nullptr, *h_tparams = nullptr;
   unsigned long long *counts = nullptr;
+  unsigned *ticket = nullptr;  // of finish_sums, zero between launches
 
   // pinned host mirrors
   double *h_red = nullptr;
@@ -117,8 +118,9 @@ std::vector<HmcFusedOp> su2b_fuse(const std::vector<HmcOp> &ops);
 int su2b_fail(su2b_ctx *ctx, int code, const char *fmt, ...);
 int su2b_adj_upload(su2b_ctx *ctx, const double *host, void *dev);
 int su2b_adj_download(su2b_ctx *ctx, const void *dev, double *host);
-int su2b_q_plaq(su2b_ctx *ctx, const void *U, int red_slot);
-int su2b_q_clover(su2b_ctx *ctx, const void *U, int cloverdef, int red_slot);
+// three plaquette / clover sums of U into out, device memory or the pinned h_red
+int su2b_q_plaq(su2b_ctx *ctx, const void *U, double *out);
+int su2b_q_clover(su2b_ctx *ctx, const void *U, int cloverdef, double *out);
 int su2b_fetch_red(su2b_ctx *ctx, int n);
 // E and Q of energy_density (flat-energy_density.hh:57-164) from the clover sums r[0..2] of V sites
 void su2b_finish_clover(const double *r, double V, int cloverdef, int ss, double *E, double *Q);

@@ -21,10 +21,11 @@ cudaError_t spinor_from_host(const Geom &g, const double *aos, double2 *psi, cud
 cudaError_t spinor_to_host(const Geom &g, const double2 *psi, double *aos, cudaStream_t s);
 
 // ---- reductions ----
-// plaquette partial sums, 3 per block {full, spatial-only, xi-weighted}; returns #blocks
+// plaquette partial sums, 3 per block {full, spatial-only, xi-weighted}; returns #blocks.
+// fin.out: their sums over the blocks as well
 template <class T>
 cudaError_t plaq_partials(const Geom &g, const void *U, int group, double xi, double *part,
-                          int *nblocks, cudaStream_t s);
+                          int *nblocks, cudaStream_t s, Finish fin = {});
 // out[k] = sum_b part[b*ncomp + k] in a fixed order, k < ncomp
 cudaError_t reduce_final(const double *part, int nblocks, int ncomp, double *out,
                          cudaStream_t s);
@@ -123,10 +124,10 @@ cudaError_t metropolis_pass(const Geom &g, void *U, int group, int mu, int parit
                             unsigned long long *counts, cudaStream_t s);
 
 // ---- clover energy density / charge ----
-// per-block partials {E, E_ss, Q, Q_ss}
+// per-block partials {E, E_ss, Q}; fin.out: their sums over the blocks as well
 template <class T>
 cudaError_t clover_partials(const Geom &g, const void *U, int group, int cloverdef,
-                            double *part, int *nblocks, cudaStream_t s);
+                            double *part, int *nblocks, cudaStream_t s, Finish fin = {});
 
 // ---- staggered fermions ----
 cudaError_t u1_phases(const Geom &g, const double *theta, double2 *ph, cudaStream_t s);

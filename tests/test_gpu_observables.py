@@ -87,3 +87,45 @@ def test_observable_errors(gpu):
             c.APEsmearing(0.5, spatial=True)  # no spatial plane in d = 2
         with pytest.raises(su2_b200.Su2bError):
             c.wilsonloop(-1, 2)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("dims,nd", [((20, 18, 20, 22), 4), ((56, 52, 1, 58), 3),
+                                     ((398, 1, 1, 402), 2), ((2, 2, 2, 2), 4)])
+def test_sums_over_more_bands_than_blocks(gpu, orc, dims, nd, precision):
+    """Lattices with more bands of sites than the GPU holds blocks (and the smallest), where
+    the blocks of the measurement kernels take several bands each, the last of them uneven.
+    Per site the products carry a few ulp (2^-53) and the FP32 links are exact in both; the
+    sums run over V sites of terms of order one: 1e-12 of the sum of absolute values."""
+    if precision == "mixed" and nd == 3:
+        pytest.skip("one dimension of the FP32 path is enough at this size")
+    U = orc.hotstart(0, dims, nd, 31, 0.7, 2024)
+    V = int(np.prod(dims))
+    with make(gpu, 0, dims, nd, precision) as c:
+        c.upload(U)
+        U = c.download()
+        plaquettes = {}
+        for _ in range(2):  # the second call finds the ticket back at zero
+            for spatial in (False, True):
+                plaquettes[spatial] = c.gauge_energy(spatial)
+                if precision == "fp64":
+                    assert plaquettes[spatial] == pytest.approx(
+                        orc.gauge_energy(0, dims, nd, U, spatial), abs=1e-12 * V)
+        for clover in (True, False):
+            E, Q = c.energy_density(clover)
+            Eo, Qo = orc.energy_density(0, dims, nd, U, clover, False)
+            assert E == pytest.approx(Eo, rel=1e-12)
+            assert Q == pytest.approx(Qo, abs=1e-12 * V)
+        assert c.polyakov_loop_spatial_average() == pytest.approx(
+            orc.polyakov_loop(0, dims, nd, U), abs=1e-13)
+        for r, t in ((2, 1), (3, 5)):
+            assert c.wilsonloop(r, t) == pytest.approx(orc.wilson_loop(0, dims, nd, U, r, t),
+                                                       abs=1e-13)
+        if precision == "mixed":
+            # the plaquette products of FP32 links are FP32: a translated field has the same
+            # terms in other bands
+            Lx, Ly, Lz, Lt = dims
+            c.upload(np.roll(U.reshape(Lt, Lx, Ly, Lz, -1), (1, 1), (0, 1)).ravel())
+            for spatial in (False, True):
+                assert c.gauge_energy(spatial) == pytest.approx(plaquettes[spatial],
+                                                                abs=1e-12 * V)
