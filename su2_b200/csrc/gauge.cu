@@ -120,15 +120,20 @@ template <class T, int NT> constexpr int plaq_min_blocks() {
 }
 
 template <class T, int ND, int NT>
-__global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
-  k_plaq_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part, Finish fin) {
-  __shared__ double shk[3 * (NT / 32)];
-  double v[3] = {0., 0., 0.};
+__device__ __forceinline__ void plaq_bands(const Geom &g, const LinkT<T> *__restrict__ U,
+                                           double xi, double (&v)[3]) {
   for (int c = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); 32 * (c >> 1) < g.ncb;
        c += gridDim.x * (NT / 32)) {  // band c/2 of 32 sites, parity c%2
     const int b = 32 * (c >> 1) + (threadIdx.x & 31);
     if (b < g.ncb) plaq_site<T, ND>(g, U, c & 1, g.cb0 + b, xi, v[0], v[1], v[2]);
   }
+}
+template <class T, int ND, int NT>
+__global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
+  k_plaq_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part, Finish fin) {
+  __shared__ double shk[3 * (NT / 32)];
+  double v[3] = {0., 0., 0.};
+  plaq_bands<T, ND, NT>(g, U, xi, v);
   finish_sums<NT, 3>(v, part, fin, shk);
 }
 
@@ -144,6 +149,7 @@ __global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
   __shared__ double shk[4 * (NT / 32)];
   const int w = threadIdx.x >> 5, p = w & 1;
   const int cb = g.cb0 + blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  pdl_trigger();
   double k2 = 0., full = 0., spat = 0., wsum = 0.;
   if (cb < g.cb0 + g.ncb) {
     const uint64_t seed = tp->seed;
@@ -497,68 +503,63 @@ __global__ void k_accept(const double *__restrict__ red, const TrajParams *__res
                          TrajDev *out) {
   accept_body(red, tp, out);
 }
-// the closing reductions of a fused trajectory and its accept/reject in one launch: the
-// start partials (momenta pass, 4 components, skipped when ns = 0) into red[0..3], the final
-// kinetic partials into red[4] (skipped when nk = 0), the end plaquette partials into
-// red[5..7], then the accept step on thread 0.  Every thread strides over all three partial
-// arrays at once with eight accumulators (the loads of one stride are independent), then a
-// fixed shuffle tree per warp and the warp sums in order.
+// The end of a fused trajectory in one launch: the plaquettes of the final field (as
+// k_plaq_su2), and in the block that finishes last the closing sums and the accept step.  It
+// adds up the start partials (momenta pass, 4 components, skipped when ns = 0) into red[0..3],
+// the final kinetic partials into red[4] (skipped when nk = 0) and the end plaquettes into
+// red[5..7], each in an order fixed by the grids, and writes red[0..9] and the result to the
+// pinned host copies as well.  A separate reduction launch, two copies and a memset that it
+// replaces took 13 us of the 70 us of a trajectory of ten steps at 8^4.
 // cached_start: the momenta pass summed no plaquettes (its components 1..3 are zero); the
 // start field is the previous trajectory's result, whose plaquette sums are still in red[]:
 // red[5..7] if that trajectory was accepted (out->accepted), else red[1..3].  They are taken
 // before the end plaquettes overwrite red[5..7].
-__global__ void __launch_bounds__(1024)
-  k_reduce_accept(const double *__restrict__ ps, int ns, const double *__restrict__ pk, int nk,
-                  const double *__restrict__ pp, int np, double *red,
-                  const TrajParams *__restrict__ tp, TrajDev *out, int cached_start) {
-  constexpr int NT = 1024, NC = 8;
-  __shared__ double sh[NC][NT / 32];
-  __shared__ double sum[NC];
-  double acc[NC];
+template <class T, int ND, int NT>
+__global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
+  k_plaq_accept_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part,
+                    TrajTail e) {
+  constexpr int NC = 8;
+  __shared__ double shk[NC * (NT / 32)];
+  pdl_wait();
+  double v[3] = {0., 0., 0.};
+  plaq_bands<T, ND, NT>(g, U, xi, v);
+  if (!leave_sums<NT, 3>(v, part, e.ticket, shk)) return;
+  double a[NC];
 #pragma unroll
-  for (int c = 0; c < NC; c++) acc[c] = 0.;
-  const int nmax = max(ns, max(nk, np));
+  for (int k = 0; k < NC; k++) a[k] = 0.;
+  const int nmax = max(e.ns, max(e.nk, (int)gridDim.x));
+#pragma unroll 2
   for (int b = threadIdx.x; b < nmax; b += NT) {
-    if (b < ns) {
+    if (b < e.ns) {
 #pragma unroll
-      for (int k = 0; k < 4; k++) acc[k] += ps[(size_t)b * 4 + k];
+      for (int k = 0; k < 4; k++) a[k] += e.ps[(size_t)b * 4 + k];
     }
-    if (b < nk) acc[4] += pk[b];
-    if (b < np) {
+    if (b < e.nk) a[4] += e.pk[b];
+    if (b < (int)gridDim.x) {
 #pragma unroll
-      for (int k = 0; k < 3; k++) acc[5 + k] += pp[(size_t)b * 3 + k];
+      for (int k = 0; k < 3; k++) a[5 + k] += __ldcg(part + (size_t)b * 3 + k);
     }
   }
-#pragma unroll
-  for (int c = 0; c < NC; c++) {
-    double v = acc[c];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sh[c][threadIdx.x >> 5] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 32 * NC) {  // warp c sums component c over the 32 warp partials
-    const int c = threadIdx.x >> 5, l = threadIdx.x & 31;
-    double v = sh[c][l];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (l == 0) sum[c] = v;
-  }
-  __syncthreads();
+  block_sums<NT, NC>(a, shk);
   if (threadIdx.x == 0) {
-    if (cached_start) {
-      const bool prev_accepted = out->accepted != 0;
+    double *red = e.red;
+    if (e.cached_start) {
+      const bool prev_accepted = e.out->accepted != 0;
 #pragma unroll
       for (int k = 1; k < 4; k++) red[k] = prev_accepted ? red[4 + k] : red[k];
-      red[0] = sum[0];
-    } else if (ns > 0) {
+      red[0] = a[0];
+    } else if (e.ns > 0) {
 #pragma unroll
-      for (int k = 0; k < 4; k++) red[k] = sum[k];
+      for (int k = 0; k < 4; k++) red[k] = a[k];
     }
-    if (nk > 0) red[4] = sum[4];
+    if (e.nk > 0) red[4] = a[4];
 #pragma unroll
-    for (int k = 5; k < 8; k++) red[k] = sum[k];
-    accept_body(red, tp, out);
+    for (int k = 5; k < 8; k++) red[k] = a[k];
+    red[8] = red[9] = 0.;  // no fermion action
+    accept_body(red, e.tp, e.out);
+    *e.h_out = *e.out;
+#pragma unroll
+    for (int k = 0; k < 10; k++) e.h_red[k] = red[k];
   }
 }
 
@@ -923,11 +924,17 @@ cudaError_t accept_step(const double *red, const TrajParams *tp, TrajDev *out, c
   k_accept<<<1, 1, 0, s>>>(red, tp, out);
   return cudaGetLastError();
 }
-cudaError_t reduce_accept(const double *ps, int ns, const double *pk, int nk, const double *pp,
-                          int np, double *red, const TrajParams *tp, TrajDev *out,
-                          bool cached_start, cudaStream_t s) {
-  k_reduce_accept<<<1, 1024, 0, s>>>(ps, ns, pk, nk, pp, np, red, tp, out, (int)cached_start);
-  return cudaGetLastError();
+template <class T>
+cudaError_t plaq_accept(const Geom &g, const void *U, double xi, double *part,
+                        const TrajTail &e, bool pdl, cudaStream_t s) {
+  constexpr int NT = 256;
+  const dim3 grid(min(cdiv(g.ncb, NT / 2), 148 * plaq_min_blocks<T, NT>()));
+  const LinkT<T> *u = (const LinkT<T> *)U;
+  switch (g.nd) {
+    case 2: return launch_force(k_plaq_accept_su2<T, 2, NT>, grid, NT, s, pdl, 0, g, u, xi, part, e);
+    case 3: return launch_force(k_plaq_accept_su2<T, 3, NT>, grid, NT, s, pdl, 0, g, u, xi, part, e);
+    default: return launch_force(k_plaq_accept_su2<T, 4, NT>, grid, NT, s, pdl, 0, g, u, xi, part, e);
+  }
 }
 
 template <class T>
@@ -963,6 +970,8 @@ cudaError_t cond_restore(const Geom &g, void *U, const void *U_old, int group,
   template cudaError_t adj_round_axpy<T>(const Geom &, T *, const T *, int, double, double,  \
                                          cudaStream_t);                                       \
   template cudaError_t restore_links<T>(const Geom &, void *, int, cudaStream_t);            \
+  template cudaError_t plaq_accept<T>(const Geom &, const void *, double, double *,          \
+                                      const TrajTail &, bool, cudaStream_t);                 \
   template cudaError_t momenta_philox<T>(const Geom &, T *, int, const TrajParams *,         \
                                          double *, int *, cudaStream_t);                      \
   template cudaError_t momenta_plaq<T>(const Geom &, const void *, T *, const TrajParams *,  \

@@ -198,9 +198,8 @@ int enqueue_fused(su2b_ctx *ctx, const std::vector<FOp> &fops, bool host_momenta
   cudaStream_t s = ctx->stream;
   int nb = 0;
   // partial sums: the start pass in slot 1, the final kinetic energy in slot 2, the end
-  // plaquettes in slot 0; all three are reduced by the accept launch
-  int nb_start = 0, nb_kin = 0, nb_plaq = 0;
-  SU2B_CK(cudaMemsetAsync(ctx->red + 8, 0, 2 * sizeof(double), s));
+  // plaquettes in slot 0; all three are reduced by the last launch
+  int nb_start = 0, nb_kin = 0;
   if (!host_momenta) {
     // momenta, kinetic energy and the plaquettes of the start field in one pass
     if (ctx->link64)
@@ -277,17 +276,15 @@ int enqueue_fused(su2b_ctx *ctx, const std::vector<FOp> &fops, bool host_momenta
     SU2B_CKS(su2b_q_restore(ctx, cur));
     F = cur;
   }
+  const TrajTail end{ctx->part_slot(1), ctx->part_slot(2), nb_start, nb_kin,
+                     cached && !host_momenta, ctx->ticket, ctx->tparams, ctx->red, ctx->h_red,
+                     ctx->traj, ctx->h_traj};
   if (ctx->link64)
-    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_partials<double>(ctx->g, F, ctx->group, ctx->xi,
-                                                        ctx->part_slot(0), &nb_plaq, s));
+    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_accept<double>(ctx->g, F, ctx->xi, ctx->part_slot(0), end,
+                                                      !ctx->prof, s));
   else
-    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_partials<float>(ctx->g, F, ctx->group, ctx->xi,
-                                                       ctx->part_slot(0), &nb_plaq, s));
-  SU2B_LAUNCH(SU2B_K_OTHER, reduce_accept(ctx->part_slot(1), nb_start, ctx->part_slot(2), nb_kin,
-                                          ctx->part_slot(0), nb_plaq, ctx->red, ctx->tparams,
-                                          ctx->traj, cached && !host_momenta, s));
-  SU2B_CK(cudaMemcpyAsync(ctx->h_traj, ctx->traj, sizeof(TrajDev), cudaMemcpyDeviceToHost, s));
-  SU2B_CK(cudaMemcpyAsync(ctx->h_red, ctx->red, 20 * sizeof(double), cudaMemcpyDeviceToHost, s));
+    SU2B_LAUNCH(SU2B_K_PLAQUETTE, plaq_accept<float>(ctx->g, F, ctx->xi, ctx->part_slot(0), end,
+                                                     !ctx->prof, s));
   *fin = F;
   return SU2B_OK;
 }

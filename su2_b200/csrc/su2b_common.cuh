@@ -411,22 +411,29 @@ struct Finish {
   double *out;
   unsigned *ticket;
 };
+// leaves the block's sums in part[]; true in the block that comes last (ticket = nullptr: none)
 template <int NT, int K>
-__device__ __forceinline__ void finish_sums(double (&v)[K], double *part, const Finish &fin,
-                                            double *sh) {
+__device__ __forceinline__ bool leave_sums(double (&v)[K], double *part, unsigned *ticket,
+                                           double *sh) {
   block_sums<NT, K>(v, sh);
   if (threadIdx.x == 0)
 #pragma unroll
     for (int k = 0; k < K; k++) part[(size_t)K * blockIdx.x + k] = v[k];
-  if (!fin.out) return;
+  if (!ticket) return false;
   __shared__ bool last;
   if (threadIdx.x == 0) {
     __threadfence();
-    last = atomicInc(fin.ticket, gridDim.x - 1) == gridDim.x - 1;
+    last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!last) return;
+  if (!last) return false;
   __threadfence();
+  return true;
+}
+template <int NT, int K>
+__device__ __forceinline__ void finish_sums(double (&v)[K], double *part, const Finish &fin,
+                                            double *sh) {
+  if (!leave_sums<NT, K>(v, part, fin.out ? fin.ticket : nullptr, sh)) return;
 #pragma unroll
   for (int k = 0; k < K; k++) v[k] = 0.;
 #pragma unroll 4

@@ -110,9 +110,21 @@ struct TrajDev {
   int pad;
 };
 cudaError_t accept_step(const double *red, const TrajParams *tp, TrajDev *out, cudaStream_t s);
-cudaError_t reduce_accept(const double *ps, int ns, const double *pk, int nk, const double *pp,
-                          int np, double *red, const TrajParams *tp, TrajDev *out,
-                          bool cached_start, cudaStream_t s);
+// the end of a fused SU(2) trajectory: the plaquettes of the final field, the closing sums and
+// the accept step in one launch
+struct TrajTail {
+  const double *ps;  // the start pass's partials, 4 per block (ns = 0: red[0..3] holds them)
+  const double *pk;  // the final kinetic partials
+  int ns, nk;
+  int cached_start;  // the start plaquettes are the previous trajectory's
+  unsigned *ticket;
+  const TrajParams *tp;
+  double *red, *h_red;  // red[0..9] and its pinned copy
+  TrajDev *out, *h_out;
+};
+template <class T>
+cudaError_t plaq_accept(const Geom &g, const void *U, double xi, double *part,
+                        const TrajTail &e, bool pdl, cudaStream_t s);
 template <class T>
 cudaError_t cond_restore(const Geom &g, void *U, const void *U_old, int group,
                          const TrajDev *flag, cudaStream_t s);
