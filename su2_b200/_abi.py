@@ -146,7 +146,8 @@ BATCH_VARIANTS = 4
 BATCH_SHAPES = [(64, 8), (128, 4), (128, 6), (256, 3)]
 # (threads per block, min resident blocks per SM) of the force kernel's launch shapes; the
 # "split" shapes run two threads per site (d = 4; other d use (128, 8)), "xsplit" with the
-# cross-plane products formed once per site and swapped in shared memory; the anisotropic
+# cross-plane products formed once per site and swapped in shared memory; (256, 3) runs three
+# threads per link on d = 4 lattices of at most 1024 sites per time slice; the anisotropic
 # action always runs (128, 6)
 FORCE_SHAPES = [(256, 4), (128, 8), (128, 4), (128, 6), (256, 2), (256, 3), ("split", 128, 8),
                 (64, 16), ("xsplit", 128, 8), ("link", 128, 6), ("split", 128, 5), ("pair", 128, 8)]

@@ -245,8 +245,7 @@ __global__ void __launch_bounds__(NT, MINB)
               const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
               double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   __shared__ double sh[NT / 32];
-  pdl_trigger();
-  pdl_wait();
+  pdl_start<MINB>();
   // warps alternate between the parities of one band of NT/2 sites per parity, so the
   // +-z / +-y neighbours of a site are mostly the own links of another warp of the block
   const int w = threadIdx.x >> 5;
@@ -273,8 +272,7 @@ __global__ void __launch_bounds__(32 * ND, MINB)
                    double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   constexpr int NT = 32 * ND;
   __shared__ double sh[NT / 32];
-  pdl_trigger();
-  pdl_wait();
+  pdl_start<MINB>();
   const int mu = threadIdx.x >> 5, p = blockIdx.x & 1;
   const int cb = g.cb0 + (blockIdx.x >> 1) * 32 + (threadIdx.x & 31);
   double k2 = 0.;
@@ -293,6 +291,57 @@ __global__ void __launch_bounds__(32 * ND, MINB)
 #undef SU2B_LINK_BODY
   if (mode & FM_KINETIC) {
     const double r = block_sum<NT>(k2, sh);
+    if (threadIdx.x == 0) kin_part[blockIdx.x] = r;
+  }
+}
+
+// The fused force step of a d = 4 lattice that leaves most of the GPU idle: three threads per
+// link, one for each plane it lies in.  Warp mu + 4 j of a block takes the j-th plane of the
+// links mu of 32 sites; the staple sums meet in shared memory and warps 0..3 finish the links.
+// What a launch of so few threads takes is one thread's chain of loads and products: two
+// staples long here, six with one thread per link.  8^4, ten steps: FP64 49.5 us a trajectory
+// (one thread per link 55.3), FP32 44.4 us (48.4); 12^4, where the SMs are full: 99 us (75).
+template <class T>
+__global__ void __launch_bounds__(384, 1)
+  k_force_su2_planes(Geom g, const LinkT<T> *__restrict__ U, T *__restrict__ P,
+                     const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
+                     double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
+  __shared__ double sh[12];
+  __shared__ LinkT<T> xs[2][4][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, mu = w & 3, j = w >> 2;
+  const int p = blockIdx.x & 1, cb = g.cb0 + (blockIdx.x >> 1) * 32 + lane;
+  const bool on = cb < g.cb0 + g.ncb;  // lanes past the end compute the last site, write nothing
+  const int c = on ? cb : g.cb0 + g.ncb - 1;
+  const Site s = site_from_eo(g, p, c);
+  const size_t V = (size_t)g.V, l = mu * V + (size_t)p * g.Vh + c;
+  pdl_start<1>();
+  if (j == 0 && (mode & FM_HAS_IN)) prefetch_momenta(P, l, 4 * V);
+  Su2<T> K;
+  switch (w) {  // direction and plane are compile-time constants in each warp's body
+    case 0: K = staple_pair<T, 0, 1>(g, U, s, p); break;
+    case 1: K = staple_pair<T, 1, 0>(g, U, s, p); break;
+    case 2: K = staple_pair<T, 2, 0>(g, U, s, p); break;
+    case 3: K = staple_pair<T, 3, 0>(g, U, s, p); break;
+    case 4: K = staple_pair<T, 0, 2>(g, U, s, p); break;
+    case 5: K = staple_pair<T, 1, 2>(g, U, s, p); break;
+    case 6: K = staple_pair<T, 2, 1>(g, U, s, p); break;
+    case 7: K = staple_pair<T, 3, 1>(g, U, s, p); break;
+    case 8: K = staple_pair<T, 0, 3>(g, U, s, p); break;
+    case 9: K = staple_pair<T, 1, 3>(g, U, s, p); break;
+    case 10: K = staple_pair<T, 2, 3>(g, U, s, p); break;
+    default: K = staple_pair<T, 3, 2>(g, U, s, p); break;
+  }
+  if (j > 0) xs[j - 1][mu][lane] = as_link(K);
+  Su2<T> u;
+  if (j == 0) u = ld_link(U + l);
+  __syncthreads();
+  double k2 = 0.;
+  if (j == 0 && on) {
+    K = add(add(K, from_link(xs[0][mu][lane])), from_link(xs[1][mu][lane]));
+    k2 = finish_link<T>(u, K, l, 4 * V, P, extra, f, scale_, mode, Uout, dt_upd);
+  }
+  if (mode & FM_KINETIC) {
+    const double r = block_sum<384>(k2, sh);
     if (threadIdx.x == 0) kin_part[blockIdx.x] = r;
   }
 }
@@ -665,8 +714,7 @@ __global__ void __launch_bounds__(NT, MINB)
                     const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
                     double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   __shared__ double sh[NT / 32];
-  pdl_trigger();
-  pdl_wait();
+  pdl_start<MINB>();
   const int w = threadIdx.x >> 5;
   const int half = w & 1, p = (w >> 1) & 1;
   const int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
@@ -693,8 +741,7 @@ __global__ void __launch_bounds__(NT, MINB)
   static_assert(NT == 128, "two warp pairs per block, hardware barriers 1 and 2");
   __shared__ double sh[NT / 32];
   __shared__ LinkT<T> xs[2][NT];
-  pdl_trigger();
-  pdl_wait();
+  pdl_start<MINB>();
   const int w = threadIdx.x >> 5;
   const int half = w & 1, p = (w >> 1) & 1;
   const int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
@@ -710,6 +757,16 @@ __global__ void __launch_bounds__(NT, MINB)
     const double r = block_sum<NT>(k2, sh);
     if (threadIdx.x == 0) kin_part[blockIdx.x] = r;
   }
+}
+
+// Three threads per link or (256, 3) for shape 5.  Up to about 160 blocks of 32 sites the three
+// threads are the fastest of all shapes (10 x 8 x 8 x 12 FP64 59.6 us a trajectory of ten steps,
+// one thread per link 60.4; 10^4, 314 blocks: 79 against 64), and (256, 3) is not, which on
+// larger lattices ties with (128, 6).  The line is drawn in the sites of a time slice, not in
+// all sites, so that a slab takes the shape that the whole lattice takes, bit for bit; long
+// lattices that it admits are left to the tuner, which times the other shapes as well.
+static bool force_planes_apply(const Geom &g) {
+  return g.nd == 4 && (long)g.L[1] * g.L[2] * g.L[3] <= 1024;
 }
 
 template <class T>
@@ -799,7 +856,17 @@ cudaError_t force_update(const Geom &g, const void *U, int group, T *P, const T 
         case 2: SU2B_FORCE_LAUNCH(128, 4, false); break;
         case 3: SU2B_FORCE_LAUNCH(128, 6, false); break;
         case 4: SU2B_FORCE_LAUNCH(256, 2, false); break;
-        case 5: SU2B_FORCE_LAUNCH(256, 3, false); break;
+        case 5:
+          if (force_planes_apply(g)) {
+            const dim3 grid(2 * cdiv(g.ncb, 32));
+            nb = grid.x;
+            const cudaError_t e_ =
+              launch_force(k_force_su2_planes<T>, grid, 384, s, pdl, 0, SU2B_FORCE_ARGS);
+            if (e_ != cudaSuccess) return e_;
+          } else {
+            SU2B_FORCE_LAUNCH(256, 3, false);
+          }
+          break;
         case 6: SU2B_FORCE_SPLIT(128, 8); break;
         case 8: SU2B_FORCE_XSPLIT(128, 8); break;
         case 9: SU2B_FORCE_LINK(6); break;

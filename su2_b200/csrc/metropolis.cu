@@ -120,7 +120,9 @@ __global__ void __launch_bounds__(NT, MINB)
               int N_hit, uint64_t seed, uint32_t sweep, unsigned long long *counts, T wt, T ws) {
   __shared__ unsigned int sh_acc;
   if (threadIdx.x == 0) sh_acc = 0;
-  pdl_trigger();
+  // as pdl_start: the next pass's blocks enter early behind the last wave of several, not
+  // beside a single one (a sweep at 16^4 FP64 106 us against 115 us)
+  if (gridDim.x > 148u * MINB) pdl_trigger();
   // the sites cb0 .. cb0 + ncb - 1 of parity p (all of them but in a time slab)
   const int cb = g.cb0 + blockIdx.x * NT + threadIdx.x;
   const bool on = cb < g.cb0 + g.ncb;

@@ -518,6 +518,32 @@ def test_every_force_launch_shape_below_four_dims(gpu, orc, precision, dims, nd)
             c.upload(U)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (10, 2, 6, 4), (10, 10, 10, 2), (32, 8, 4, 2),
+                                  (8, 8, 18, 2)])
+def test_three_threads_per_link(gpu, orc, precision, dims):
+    """Shape 5 on both sides of its rule (1024 sites per time slice), with whole and partial
+    bands of 32 sites: the oracle's force, with another derivative added and without, and the
+    links, momenta and kinetic energy of one-thread-per-site trajectories to the rounding of
+    the staple sums (5 force steps of terms of order one)."""
+    U = hot(orc, 0, dims, 4)
+    F = orc.gauge_derivative(0, dims, 4, 2.3, U)
+    tol = 1e-12 if precision == "fp64" else 1e-5
+    out = {}
+    for v in (5, 2):
+        with make(gpu, 0, dims, 4, beta=2.3, precision=precision) as c:
+            c.upload(U)
+            c.force_variant = v
+            assert rel(c.derivative(), F) < tol
+            r = [c.md_update("leapfrog", 4, 0.2, seed=3, traj=k, accept_reject=False)
+                 for k in range(2)]
+            out[v] = r, c.download()
+    assert rel(out[5][1], out[2][1]) < tol
+    for a, b in zip(out[5][0], out[2][0]):
+        np.testing.assert_allclose([*a.H_old, *a.H_new], [*b.H_old, *b.H_new], rtol=10 * tol,
+                                   atol=10 * tol * int(np.prod(dims)))
+
+
 def test_autotune_cache(gpu, orc, tmp_path):
     group, dims, nd = 0, (16, 16, 16, 16), 4
     U = hot(orc, group, dims, nd)
