@@ -102,6 +102,27 @@ int finish_status(su2b_ctx *ctx, int done) {
   return SU2B_OK;
 }
 
+// The tiled CG's plan and packets, made for the first CG of a context (BiCGStab and CG_mixed
+// do without them); without room for them the other forms run.
+int cg_tile_setup(su2b_ctx *ctx) {
+  if (ctx->cg_planned) return SU2B_OK;
+  ctx->cg_planned = true;
+  const CgTilePlan plan = cg_tile_plan(ctx->g);
+  if (!plan.K) return SU2B_OK;
+  void *work = nullptr;
+  if (cudaMalloc(&work, cg_tile_bytes(ctx->g)) == cudaSuccess &&
+      cudaMallocHost((void **)&ctx->h_cg, sizeof(CgTileResult)) == cudaSuccess) {
+    ctx->allocs.push_back(work);
+    SU2B_CK(cudaMemsetAsync(work, 0, cg_tile_bytes(ctx->g), ctx->stream));
+    ctx->cg_work = work;
+    ctx->cg_plan = plan;
+  } else {
+    cudaFree(work);
+    cudaGetLastError();
+  }
+  return SU2B_OK;
+}
+
 // CG on D Ddag (CG.hpp:36-94), b in SV_B, x in SV_X (start in, solution out)
 int cg64(su2b_ctx *ctx, double m, double tol, int max_iter, su2b_solve_stats *stats) {
   const int n = (int)ctx->V;
@@ -111,6 +132,7 @@ int cg64(su2b_ctx *ctx, double m, double tol, int max_iter, su2b_solve_stats *st
           *t = ctx->sv[SV_T], *Ap = ctx->sv[SV_AP];
   double *dp = ctx->part_slot(3), *np = ctx->part_slot(4);
   // d = 2 up to about 150,000 sites: the whole solve, restarts included, in one launch on tiles
+  SU2B_CKS(cg_tile_setup(ctx));
   if (ctx->cg_plan.K) {
     CgTileResult &h = *ctx->h_cg;
     h.done = 0;
@@ -433,21 +455,6 @@ int su2b_fermion_setup(su2b_ctx *ctx, bool need32) {
     for (int k = 0; k < SV_N; k++)
       SU2B_CKS(dalloc2(ctx, (void **)&ctx->sv[k], ctx->V * sizeof(double2)));
     ctx->phases_valid = false;
-    // the tiled CG's packets; without room for them the other forms run
-    const CgTilePlan plan = cg_tile_plan(ctx->g);
-    if (plan.K) {
-      void *work = nullptr;
-      if (cudaMalloc(&work, cg_tile_bytes(ctx->g)) == cudaSuccess &&
-          cudaMallocHost((void **)&ctx->h_cg, sizeof(CgTileResult)) == cudaSuccess) {
-        ctx->allocs.push_back(work);
-        SU2B_CK(cudaMemsetAsync(work, 0, cg_tile_bytes(ctx->g), ctx->stream));
-        ctx->cg_work = work;
-        ctx->cg_plan = plan;
-      } else {
-        cudaFree(work);
-        cudaGetLastError();
-      }
-    }
   }
   if (need32 && !ctx->ph32) {
     SU2B_CKS(dalloc2(ctx, (void **)&ctx->ph32, ctx->NL * sizeof(float2)));

@@ -55,6 +55,7 @@ struct su2b_ctx {
   su2b::SolverState *st = nullptr;
   // the tiled CG (cg_tile.cu): its plan (K = 0: not for this lattice), packets and their epoch
   su2b::CgTilePlan cg_plan{};
+  bool cg_planned = false;
   void *cg_work = nullptr;
   unsigned long long cg_epoch = 0;
   su2b::CgTileResult *h_cg = nullptr;
