@@ -80,6 +80,30 @@ def test_mixed_cg(gpu, orc, dims, nd):
     assert rel(r.x, r64.x) < 1e-7
 
 
+@pytest.mark.parametrize("L,T,tiled", [(4, 6, True), (48, 64, True), (150, 140, True),
+                                       (420, 400, False)])
+def test_mixed_cg_on_tiles(gpu, L, T, tiled):
+    """Two-dimensional lattices that the tiled CG holds: the mixed solver is that FP64 solve,
+    bit for bit, its closing residual counted as an update; a larger lattice takes the FP32
+    iterations and agrees to the tolerance (1e-10 of |b| over the smallest eigenvalue of
+    D D^+, 0.2^2).  At the iteration limit the residual it returns is the iterated one."""
+    rng = np.random.default_rng(L)
+    U, b = rng.normal(size=2 * L * T) * 0.5, rng.normal(size=2 * L * T)
+    with u1(gpu, (L, 1, 1, T), 2, precision="mixed") as c:
+        c.upload(U)
+        r = c.solve(b, 0.2, tol=1e-10, tol_mode="rel", solver="CG_mixed")
+        r64 = c.solve(b, 0.2, tol=1e-10, tol_mode="rel", solver="CG")
+        assert r.converged and r.restarts >= 1
+        assert r.true_residual <= 1e-10 * np.linalg.norm(b)
+        if tiled:
+            np.testing.assert_array_equal(r.x, r64.x)
+            assert r.restarts == r64.restarts + 1 and r.iterations == r64.iterations
+        else:
+            assert np.linalg.norm(r.x - r64.x) <= 2 * 1e-10 * np.linalg.norm(b) / 0.04
+        r = c.solve(b, 0.2, tol=1e-10, tol_mode="rel", solver="CG_mixed", max_iter=3)
+        assert not r.converged and r.iterations == 3 and r.true_residual == r.residual > 0
+
+
 def test_solver_iteration_limit(gpu, orc):
     dims, nd = (8, 1, 1, 6), 2
     U, b, _ = setup(orc, dims, nd)
