@@ -1,5 +1,5 @@
-// cg_tile.cu -- the CG on D D^+ for two-dimensional lattices, the whole solve in one launch with
-// the lattice held in registers and shared memory.
+// cg_tile.cu -- the CG on D D^+ and the BiCGStab on D for two-dimensional lattices, the whole
+// solve in one launch with the lattice held in registers and shared memory.
 //
 // A block owns a tile of the lattice, a thread K of its sites: p, x, r, t = D^+ p and b live in
 // registers for the whole solve.  A phase needs two things from the other blocks, the vector's
@@ -19,6 +19,9 @@
 // (solve.cu, CG.hpp:36-94), with <p, A p> = |D^+ p|^2 and D^+ p carried by linearity:
 //   A: publish t;  alpha = rr / |t|^2;  x += alpha p;  r -= alpha D t
 //   B: publish r;  beta = |r|^2 / rr;  p = r + beta p;  t = D^+ r + beta t
+// The BiCGStab on D runs on the same tiles in three phases an iteration (bi_run), mass 0.05 to
+// 1e-12: 2.8 ms for 717 iterations at 64^2 where k_bicgstab_persistent takes 9.4 ms for 723,
+// 7.3 ms at 256^2 against 11.9 ms.
 // Every block adds the partials in the same order, so all take the same decisions.  Every wait
 // is bounded: one that gives up tells the host and all blocks return.
 #include <algorithm>
@@ -33,6 +36,7 @@ namespace {
 
 constexpr int MAX_THREADS = 512;
 constexpr int MAX_BLOCKS = 160;  // partials a warp polls: 5 per lane
+constexpr int BI_SUMS = 5;  // sums of one phase at most: the BiCGStab's (the CG: 1)
 constexpr long SPIN_LIMIT = 1L << 21;  // polls of an L2 round trip each: gives up after a second
 
 __device__ __forceinline__ void put_packet(ulonglong2 *p, double v, unsigned long long epoch) {
@@ -58,7 +62,7 @@ struct CgTileArgs {
   const double2 *b;
   double2 *x;
   ulonglong2 *halo;  // [2][V][2] packets: a boundary site's value by epoch parity
-  ulonglong2 *sums;  // [2][MAX_BLOCKS], alternating from sum to sum
+  ulonglong2 *sums;  // [2][BI_SUMS][MAX_BLOCKS], alternating from phase to phase with sums
   unsigned long long epoch;  // last epoch used by earlier solves
   CgTileResult *out;
   int *err;
@@ -83,8 +87,11 @@ __device__ __forceinline__ double2 hop2(double m, double sgn, double2 v, const d
   return make_double2(m * v.x + sgn * ar, m * v.y + sgn * ai);
 }
 
-// The solve on any tiling.  phase(v, sgn, out, sum, part, total): out = m v + sgn hop(v), and the
-// lattice's sum of `part` into total where sum is set; false: give up.
+// The solve on any tiling.  phase<N sums, hop>(v, sgn, out, part, total): out = m v + sgn hop(v)
+// where hop is set, and the lattice's sums of part[0..N-1] into total; false: give up.
+template <int N> using Sums = std::integral_constant<int, N>;
+using Hop = std::true_type;
+using NoHop = std::false_type;
 struct CgEnd {
   double rn, ex;
   long iters, restarts;
@@ -92,7 +99,12 @@ struct CgEnd {
 };
 template <int K, class Phase>
 __device__ __forceinline__ bool cg_run(const bool (&on)[K], double2 (&x)[K], const double2 (&b)[K],
-                                       double tol, long max_iter, Phase &&phase, CgEnd &end) {
+                                       double tol, long max_iter, Phase &&phase_n, CgEnd &end) {
+  auto phase = [&](const double2 (&v)[K], double sgn, double2 (&out)[K], bool sum, double part,
+                   double &total) {
+    return sum ? phase_n(Sums<1>(), Hop(), v, sgn, out, &part, &total)
+               : phase_n(Sums<0>(), Hop(), v, sgn, out, &part, &total);
+  };
   double2 r[K], p[K], t[K], w[K], aw[K];
   auto norm = [&](const double2 (&v)[K]) {
     double s = 0.;
@@ -163,6 +175,102 @@ __device__ __forceinline__ bool cg_run(const bool (&on)[K], double2 (&x)[K], con
   return true;
 }
 
+// BiCGStab on D (BiCGStab.hpp:36-106, the iteration of bicgstab64 in solve.cu), three phases each:
+//   A: publish p;  v = D p;  <r0, v> = <D^+ r0, p>, which needs no v;  |r|^2 of the last iteration
+//   B: publish s = r - alpha v;  t = D s;  <r0, s>
+//   C: sums alone: <t, s>, |t|^2, <r0, t>;  omega;  x += alpha p + omega s;  r = s - omega t;
+//      <r0, r> = <r0, s> - omega <r0, t>;  beta;  p = r + beta p - beta omega v
+// D p and D s are applied directly, not carried by recurrences.  A step's |r|^2 arrives with the
+// next step's phase A, which is where it is looked at.
+template <int K, class Phase>
+__device__ __forceinline__ bool bi_run(const bool (&on)[K], double2 (&x)[K], const double2 (&b)[K],
+                                       double tol, long max_iter, Phase &&phase, CgEnd &end) {
+  double2 r[K], p[K], v[K], t[K], r0[K], w0[K];
+  // <a, c> over the thread's sites
+  auto dot = [&](const double2 (&a)[K], const double2 (&c)[K], double *re, double *im) {
+    double sr = 0., si = 0.;
+#pragma unroll
+    for (int k = 0; k < K; k++)
+      if (on[k]) {
+        sr += a[k].x * c[k].x + a[k].y * c[k].y;
+        if (im) si += a[k].x * c[k].y - a[k].y * c[k].x;
+      }
+    *re = sr;
+    if (im) *im = si;
+  };
+  double part[BI_SUMS], sum[BI_SUMS];
+  double rn = 0., ex = 0.;
+  long iters = 0, restarts = 0;
+  int done = 0;
+#pragma unroll
+  for (int k = 0; k < K; k++) r[k] = p[k] = v[k] = t[k] = r0[k] = w0[k] = make_double2(0., 0.);
+  for (bool start = true;; start = false) {
+    // the true residual b - D x, its norm and D^+ of it
+    if (!phase(Sums<0>(), Hop(), x, 1., v, part, sum)) return false;
+#pragma unroll
+    for (int k = 0; k < K; k++) r0[k] = make_double2(b[k].x - v[k].x, b[k].y - v[k].y);
+    dot(r0, r0, part, nullptr);
+    if (!phase(Sums<1>(), Hop(), r0, -1., w0, part, sum)) return false;
+    ex = sqrt(sum[0]);
+    if (!start) {
+      if (!(rn < ex && iters < max_iter)) break;
+      restarts++;
+    }
+    rn = ex;
+    if (!(rn > tol)) {
+      done = 1;
+      break;
+    }
+    done = 0;
+    double2 rho = make_double2(sum[0], 0.);
+#pragma unroll
+    for (int k = 0; k < K; k++) r[k] = p[k] = r0[k];
+    for (bool first = true;; first = false) {
+      dot(w0, p, part, part + 1);
+      dot(r, r, part + 2, nullptr);
+      if (!phase(Sums<3>(), Hop(), p, 1., v, part, sum)) return false;
+      if (!first) {
+        rn = sqrt(sum[2]);
+        if (rn != rn) done = 3;
+        else if (!(rn > tol)) done = 1;
+        else if (iters >= max_iter) done = 2;
+        if (done) break;
+      }
+      const double2 alpha = cdivs(rho, make_double2(sum[0], sum[1]));
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const double2 av = cm(alpha, v[k]);
+        r[k] = make_double2(r[k].x - av.x, r[k].y - av.y);
+      }
+      dot(r0, r, part, part + 1);
+      if (!phase(Sums<2>(), Hop(), r, 1., t, part, sum)) return false;
+      const double2 r0s = make_double2(sum[0], sum[1]);
+      dot(t, r, part, part + 1);
+      dot(t, t, part + 2, nullptr);
+      dot(r0, t, part + 3, part + 4);
+      if (!phase(Sums<5>(), NoHop(), r, 1., t, part, sum)) return false;
+      const double2 omega = make_double2(sum[0] / sum[2], sum[1] / sum[2]);
+      const double2 ot = cm(omega, make_double2(sum[3], sum[4]));
+      const double2 next = make_double2(r0s.x - ot.x, r0s.y - ot.y);
+      const double2 beta = cm(cdivs(next, rho), cdivs(alpha, omega));
+      const double2 bo = cm(beta, omega);
+      rho = next;
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const double2 ap = cm(alpha, p[k]), os = cm(omega, r[k]), wt = cm(omega, t[k]);
+        x[k] = make_double2(x[k].x + os.x + ap.x, x[k].y + os.y + ap.y);
+        r[k] = make_double2(r[k].x - wt.x, r[k].y - wt.y);
+        const double2 bp = cm(beta, p[k]), bv = cm(bo, v[k]);
+        p[k] = make_double2(r[k].x + bp.x - bv.x, r[k].y + bp.y - bv.y);
+      }
+      iters++;
+    }
+    if (done != 1) break;
+  }
+  end = CgEnd{rn, ex, iters, restarts, done};
+  return true;
+}
+
 __device__ __forceinline__ void write_result(CgTileResult *out, const CgEnd &e,
                                              unsigned long long epoch) {
   out->rn = e.rn;
@@ -173,11 +281,12 @@ __device__ __forceinline__ void write_result(CgTileResult *out, const CgEnd &e,
   out->epoch = epoch;
 }
 
-template <int K>
+template <int K, bool BI>
 __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_tile(CgTileArgs a) {
+  constexpr int NSM = BI ? BI_SUMS : 1;
   __shared__ double2 tile[K * MAX_THREADS];
-  __shared__ double shw[MAX_THREADS / 32];
-  __shared__ double sh_sum;
+  __shared__ double shw[NSM][MAX_THREADS / 32];
+  __shared__ double sh_sum[NSM];
   __shared__ int sh_bad;
   const CgTilePlan tp = a.tp;
   const int Lt = a.g.L[0], Lx = a.g.L[1], V = a.g.V, Vh = a.g.Vh;
@@ -227,16 +336,18 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_tile(CgTileArgs a) {
       }
     }
   };
-  // One phase: v to the neighbours, out = m v + sgn hop(v); the sum of `part` over the lattice
-  // where sum is set (out's stencil runs meanwhile).  false: a wait gave up.
-  auto phase = [&](const double2 (&v)[K], double sgn, double2 (&out)[K], bool sum, double part,
-                   double &total) -> bool {
+  // One phase: v to the neighbours, out = m v + sgn hop(v); the sums of part[] over the lattice
+  // (out's stencil runs meanwhile), each by a warp of its own.  false: a wait gave up.
+  auto phase = [&](auto ns, auto hop, const double2 (&v)[K], double sgn, double2 (&out)[K],
+                   const double *part, double *total) -> bool {
+    constexpr int NS = decltype(ns)::value;
+    constexpr bool HOP = decltype(hop)::value;
     ep++;
     ulonglong2 *const hb = a.halo + (size_t)(ep & 1) * 2 * V;
 #pragma unroll
     for (int k = 0; k < K; k++) {
       const int row = r0 + k * tp.rp;
-      if (!on[k]) continue;
+      if (!HOP || !on[k]) continue;
       tile[row * tp.hx + c] = v[k];
       if ((tp.gt > 1 && (row == 0 || row == rows - 1)) || (tp.gx > 1 && (c == 0 || c == cols - 1))) {
         ulonglong2 *q = hb + 2 * ((t0 + row) * Lx + xc);
@@ -244,23 +355,25 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_tile(CgTileArgs a) {
         put_packet(q + 1, v[k].y, ep);
       }
     }
-    if (sum) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-      if (lane == 0) shw[warp] = part;
+    for (int j = 0; j < NS; j++) {
+      double s = part[j];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) shw[j][warp] = s;
     }
     __syncthreads();
-    if (sum) nsum++;
-    ulonglong2 *const sb = a.sums + (size_t)(nsum & 1) * MAX_BLOCKS;
-    if (sum && warp == 0) {
-      double s = lane < nw ? shw[lane] : 0.;
+    if (NS) nsum++;
+    ulonglong2 *const sb = a.sums + (size_t)(nsum & 1) * BI_SUMS * MAX_BLOCKS;
+    for (int j = warp; j < NS; j += nw) {
+      double s = lane < nw ? shw[j][lane] : 0.;
 #pragma unroll
       for (int o = MAX_THREADS / 64; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) put_packet(sb + blockIdx.x, s, ep);
+      if (lane == 0) put_packet(sb + j * MAX_BLOCKS + blockIdx.x, s, ep);
     }
 #pragma unroll
     for (int k = 0; k < K; k++) {
-      if (!on[k]) continue;
+      if (!HOP || !on[k]) continue;
       const int row = r0 + k * tp.rp, tt = t0 + row;
       // forward and backward in t, then in x: inside the tile (or around the lattice in it)
       // from shared memory, else from its packets
@@ -287,7 +400,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_tile(CgTileArgs a) {
                     vxf = make_double2(w[4], w[5]), vxb = make_double2(w[6], w[7]);
       out[k] = hop2(a.m, sgn, v[k], uf[k], ub[k], vtf, vtb, vxf, vxb, tt);
     }
-    if (sum && warp == 0) {
+    for (int i = warp; i < NS; i += nw) {
       constexpr int N = MAX_BLOCKS / 32;
       const ulonglong2 *src[N];
       double q[N], s = 0.;
@@ -295,7 +408,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_tile(CgTileArgs a) {
 #pragma unroll
       for (int j = 0; j < N; j++) {
         q[j] = 0.;
-        src[j] = sb + lane + 32 * j;
+        src[j] = sb + i * MAX_BLOCKS + lane + 32 * j;
         if (lane + 32 * j < (int)gridDim.x) want |= 1u << j;
       }
       wait(std::integral_constant<int, N>(), src, want, q);
@@ -303,14 +416,17 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_tile(CgTileArgs a) {
       for (int j = 0; j < N; j++) s += q[j];
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) sh_sum = s;
+      if (lane == 0) sh_sum[i] = s;
     }
-    __syncthreads();  // the sum is in; the tile may be rewritten
-    total = sh_sum;
+    __syncthreads();  // the sums are in; the tile may be rewritten
+#pragma unroll
+    for (int j = 0; j < NS; j++) total[j] = sh_sum[j];
     return sh_bad == 0;
   };
   CgEnd end;
-  if (!cg_run<K>(on, x, b, a.tol, a.max_iter, phase, end)) return;
+  const bool good = BI ? bi_run<K>(on, x, b, a.tol, a.max_iter, phase, end)
+                       : cg_run<K>(on, x, b, a.tol, a.max_iter, phase, end);
+  if (!good) return;
 #pragma unroll
   for (int k = 0; k < K; k++)
     if (on[k]) a.x[eo(t0 + r0 + k * tp.rp, xc)] = x[k];
@@ -339,18 +455,20 @@ __device__ __forceinline__ double2 lds(uint32_t a) {
   asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a) : "memory");
   return v;
 }
-template <int K> struct ClusterBuf {
+template <int K, bool BI> struct ClusterBuf {
+  static constexpr int NSM = BI ? BI_SUMS : 1;
   double2 tile[K * MAX_THREADS];
   double2 rim[MAX_RIM];        // t forward, t backward, x forward, x backward
-  double thr[MAX_THREADS];     // the threads' partials
-  double part[MAX_CLUSTER];    // the blocks' partials
+  double thr[NSM][MAX_THREADS];   // the threads' partials
+  double part[NSM][MAX_CLUSTER];  // the blocks' partials
   unsigned long long bar;
 };
-template <int K>
+template <int K, bool BI>
 __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  ClusterBuf<K> *const B = (ClusterBuf<K> *)smem;
-  constexpr uint32_t STEP = sizeof(ClusterBuf<K>);
+  using Buf = ClusterBuf<K, BI>;
+  Buf *const B = (Buf *)smem;
+  constexpr uint32_t STEP = sizeof(Buf);
   __shared__ unsigned sh_bad;  // the first phase in which a wait gave up
   const CgTilePlan tp = a.tp;
   const int Lt = a.g.L[0], Lx = a.g.L[1], V = a.g.V, Vh = a.g.Vh;
@@ -368,14 +486,16 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(saddr(&B[k].bar)) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (tid < 2 * MAX_CLUSTER) B[tid / MAX_CLUSTER].part[tid % MAX_CLUSTER] = 0.;
+  for (int i = tid; i < 2 * Buf::NSM * MAX_CLUSTER; i += blockDim.x)
+    B[i / (Buf::NSM * MAX_CLUSTER)].part[0][i % (Buf::NSM * MAX_CLUSTER)] = 0.;
   const uint32_t my_bar = saddr(&B[0].bar);
   // this block's slot in the partials of block `lane`, and that block's barrier
   const int peer = lane < nb ? lane : 0;
-  const uint32_t mine = cluster_addr(saddr(&B[0].part[blockIdx.x]), peer);
+  const uint32_t mine = cluster_addr(saddr(&B[0].part[0][blockIdx.x]), peer);
   const uint32_t peer_bar = cluster_addr(my_bar, peer);
-  const int incoming =
-    nb * 8 + (rows > 0 ? 16 * ((tp.gt > 1 ? 2 * cols : 0) + (tp.gx > 1 ? 2 * rows : 0)) : 0);
+  // bytes of a phase besides the sums
+  const int rims =
+    rows > 0 ? 16 * ((tp.gt > 1 ? 2 * cols : 0) + (tp.gx > 1 ? 2 * rows : 0)) : 0;
 
   bool on[K];
   double2 uf[K][2], ub[K][2], x[K], b[K];
@@ -429,18 +549,21 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
   }
   cluster_sync();  // every block runs and its barriers are set before anything is sent to it
   unsigned n = 0;
-  auto phase = [&](const double2 (&v)[K], double sgn, double2 (&out)[K], bool, double pt,
-                   double &total) -> bool {
+  auto phase = [&](auto ns, auto hop, const double2 (&v)[K], double sgn, double2 (&out)[K],
+                   const double *pt, double *total) -> bool {
+    constexpr int NS = decltype(ns)::value > 1 ? decltype(ns)::value : 1;
+    constexpr bool HOP = decltype(hop)::value;
     const uint32_t off = (n & 1) * STEP, parity = (n >> 1) & 1;
-    ClusterBuf<K> &C = B[n & 1];
+    Buf &C = B[n & 1];
     n++;
     if (tid == 0)
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(my_bar + off),
-                   "r"(incoming)
+                   "r"(NS * nb * 8 + (HOP ? rims : 0))
                    : "memory");
-    C.thr[tid] = pt;
 #pragma unroll
-    for (int k = 0; k < K; k++) {
+    for (int j = 0; j < NS; j++) C.thr[j][tid] = decltype(ns)::value ? pt[j] : 0.;
+#pragma unroll
+    for (int k = 0; k < (HOP ? K : 0); k++) {
       auto push = [&](uint32_t d, uint32_t db) {
         if (d)
           asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.f64 [%0], {%1, %2}, [%3];" ::"r"(d + off),
@@ -456,10 +579,10 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
     }
     __syncthreads();
     if (*(volatile unsigned *)&sh_bad < n) return false;  // in an earlier phase: the same for all
-    if (warp == 0) {
+    for (int i = warp; i < NS; i += nw) {  // a warp for each sum
       double q[MAX_THREADS / 32];
 #pragma unroll
-      for (int j = 0; j < MAX_THREADS / 32; j++) q[j] = j < nw ? C.thr[lane + 32 * j] : 0.;
+      for (int j = 0; j < MAX_THREADS / 32; j++) q[j] = j < nw ? C.thr[i][lane + 32 * j] : 0.;
 #pragma unroll
       for (int o = MAX_THREADS / 64; o > 0; o >>= 1)
 #pragma unroll
@@ -467,7 +590,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) q[0] += __shfl_xor_sync(0xffffffffu, q[0], o);
       if (lane < nb)
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(mine + off),
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.f64 [%0], %1, [%2];" ::"r"(mine + off + (uint32_t)(i * 8 * MAX_CLUSTER)),
                      "d"(q[0]), "r"(peer_bar + off)
                      : "memory");
     }
@@ -489,27 +612,31 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
     }
     double2 w[K][4];
 #pragma unroll
-    for (int k = 0; k < K; k++)
+    for (int k = 0; k < (HOP ? K : 0); k++)
 #pragma unroll
       for (int j = 0; j < 4; j++) w[k][j] = lds(src[k][j] + off);
     // every thread adds the blocks' partials in the same order
-    double2 q[MAX_CLUSTER / 2];
-    const uint32_t pa = saddr(&B[0].part[0]) + off;
+    const uint32_t pa = saddr(&B[0].part[0][0]) + off;
 #pragma unroll
-    for (int j = 0; j < MAX_CLUSTER / 2; j++) q[j] = lds(pa + 16 * j);
+    for (int i = 0; i < NS; i++) {
+      double2 q[MAX_CLUSTER / 2];
 #pragma unroll
-    for (int o = MAX_CLUSTER / 4; o > 0; o >>= 1)
+      for (int j = 0; j < MAX_CLUSTER / 2; j++) q[j] = lds(pa + 8 * MAX_CLUSTER * i + 16 * j);
 #pragma unroll
-      for (int j = 0; j < o; j++) q[j].x += q[j + o].x, q[j].y += q[j + o].y;
-    total = q[0].x + q[0].y;
+      for (int o = MAX_CLUSTER / 4; o > 0; o >>= 1)
 #pragma unroll
-    for (int k = 0; k < K; k++)
+        for (int j = 0; j < o; j++) q[j].x += q[j + o].x, q[j].y += q[j + o].y;
+      total[i] = q[0].x + q[0].y;
+    }
+#pragma unroll
+    for (int k = 0; k < (HOP ? K : 0); k++)
       out[k] = hop2(a.m, sgn, v[k], uf[k], ub[k], w[k][0], w[k][1], w[k][2], w[k][3],
                     t0 + r0 + k * tp.rp);
     return true;
   };
   CgEnd end;
-  const bool good = cg_run<K>(on, x, b, a.tol, a.max_iter, phase, end);
+  const bool good = BI ? bi_run<K>(on, x, b, a.tol, a.max_iter, phase, end)
+                       : cg_run<K>(on, x, b, a.tol, a.max_iter, phase, end);
   if (good) {
 #pragma unroll
     for (int k = 0; k < K; k++)
@@ -526,7 +653,7 @@ template <int K> int tile_blocks(int *slots) {
     int coop = 0, sms = 0, per_sm = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_tile<K>, MAX_THREADS, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_tile<K, false>, MAX_THREADS, 0);
     slots[dev] = 1 + (coop && per_sm >= 1 ? sms : 0);
   }
   return slots[dev] - 1;
@@ -562,28 +689,34 @@ inline cudaLaunchConfig_t cluster_config(int size, int nt, size_t smem, cudaStre
   cfg.numAttrs = 1;
   return cfg;
 }
+template <int K, bool BI> bool set_cluster_attributes() {
+  if (cudaFuncSetAttribute(k_cg_cluster<K, BI>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+        cudaSuccess &&
+      cudaFuncSetAttribute(k_cg_cluster<K, BI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)(2 * sizeof(ClusterBuf<K, BI>))) == cudaSuccess)
+    return true;
+  cudaGetLastError();
+  return false;
+}
+template <int K, bool BI> bool cluster_fits(int size, const CgTilePlan &q) {
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config(size, (q.rp * q.hx + 31) / 32 * 32,
+                                                 2 * sizeof(ClusterBuf<K, BI>), nullptr, &attr);
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, k_cg_cluster<K, BI>, &cfg) == cudaSuccess && n >= 1)
+    return true;
+  cudaGetLastError();
+  return false;
+}
 template <int K> bool plan_cluster(const Geom &g, CgTilePlan *p) {
-  if (cudaFuncSetAttribute(k_cg_cluster<K>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-        cudaSuccess ||
-      cudaFuncSetAttribute(k_cg_cluster<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)(2 * sizeof(ClusterBuf<K>))) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
+  if (!set_cluster_attributes<K, false>()) return false;
   double best = 1e30;
   for (int size = 1; size <= MAX_CLUSTER; size *= 2) {
     CgTilePlan q{};
     // a second block costs the cluster's barrier, as much as 200 sites
     const double c = plan(g, K, size, MAX_RIM, &q) + (size > 1 ? 200. : 0.);
     if (!q.K || c >= best) continue;
-    cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = cluster_config(size, (q.rp * q.hx + 31) / 32 * 32, 2 * sizeof(ClusterBuf<K>),
-                                                   nullptr, &attr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_cg_cluster<K>, &cfg) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      continue;
-    }
+    if (!cluster_fits<K, false>(size, q)) continue;
     best = c;
     *p = q;
     p->cluster = size;
@@ -602,32 +735,48 @@ CgTilePlan cg_tile_plan(const Geom &g) {
   if (!p.K) plan(g, 2, std::min(tile_blocks<2>(slots[1]), MAX_BLOCKS), 1 << 30, &p);
   return p;
 }
+// whether the BiCGStab runs on a plan made for the CG
+bool cg_tile_bicgstab(const CgTilePlan &p) {
+  if (!p.K) return false;
+  if (p.cluster)
+    return p.K == 1 ? set_cluster_attributes<1, true>() && cluster_fits<1, true>(p.cluster, p)
+                    : set_cluster_attributes<2, true>() && cluster_fits<2, true>(p.cluster, p);
+  int per_sm = 0;
+  const cudaError_t e =
+    p.K == 1 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_tile<1, true>, MAX_THREADS, 0)
+             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cg_tile<2, true>, MAX_THREADS, 0);
+  cudaGetLastError();
+  return e == cudaSuccess && per_sm >= 1;
+}
 size_t cg_tile_bytes(const Geom &g) {
-  return sizeof(ulonglong2) * ((size_t)4 * g.V + 2 * MAX_BLOCKS + 1);
+  return sizeof(ulonglong2) * ((size_t)4 * g.V + 2 * BI_SUMS * MAX_BLOCKS + 1);
 }
 
-cudaError_t cg_tile(const Geom &g, const CgTilePlan &tp, const double2 *ph, double m,
-                    const double2 *b, double2 *x, double tol, long max_iter, void *work,
+cudaError_t cg_tile(const Geom &g, const CgTilePlan &tp, bool bicgstab, const double2 *ph,
+                    double m, const double2 *b, double2 *x, double tol, long max_iter, void *work,
                     unsigned long long epoch, CgTileResult *out, cudaStream_t s) {
   CgTileArgs a{};
   a.g = g, a.tp = tp, a.ph = ph, a.m = m, a.b = b, a.x = x, a.tol = tol, a.max_iter = max_iter;
   a.halo = (ulonglong2 *)work;
   a.sums = a.halo + (size_t)4 * g.V;
-  a.err = (int *)(a.sums + 2 * MAX_BLOCKS);
+  a.err = (int *)(a.sums + 2 * BI_SUMS * MAX_BLOCKS);
   a.epoch = epoch, a.out = out;
   const int nt = (tp.rp * tp.hx + 31) / 32 * 32;
   if (tp.cluster) {
+    const auto kern = bicgstab ? (tp.K == 1 ? k_cg_cluster<1, true> : k_cg_cluster<2, true>)
+                               : (tp.K == 1 ? k_cg_cluster<1, false> : k_cg_cluster<2, false>);
+    const size_t buf = bicgstab ? (tp.K == 1 ? sizeof(ClusterBuf<1, true>) : sizeof(ClusterBuf<2, true>))
+                                : (tp.K == 1 ? sizeof(ClusterBuf<1, false>) : sizeof(ClusterBuf<2, false>));
     cudaLaunchAttribute attr;
-    const cudaLaunchConfig_t cfg = cluster_config(
-      tp.cluster, nt, 2 * (tp.K == 1 ? sizeof(ClusterBuf<1>) : sizeof(ClusterBuf<2>)), s, &attr);
-    return tp.K == 1 ? cudaLaunchKernelEx(&cfg, k_cg_cluster<1>, a)
-                     : cudaLaunchKernelEx(&cfg, k_cg_cluster<2>, a);
+    const cudaLaunchConfig_t cfg = cluster_config(tp.cluster, nt, 2 * buf, s, &attr);
+    return cudaLaunchKernelEx(&cfg, kern, a);
   }
   cudaError_t e = cudaMemsetAsync(a.err, 0, sizeof(int), s);
   if (e != cudaSuccess) return e;
   void *args[] = {&a};
-  e = cudaLaunchCooperativeKernel(tp.K == 1 ? (const void *)k_cg_tile<1> : (const void *)k_cg_tile<2>,
-                                  dim3(tp.gt * tp.gx), dim3(nt), args, 0, s);
+  const auto kern = bicgstab ? (tp.K == 1 ? k_cg_tile<1, true> : k_cg_tile<2, true>)
+                             : (tp.K == 1 ? k_cg_tile<1, false> : k_cg_tile<2, false>);
+  e = cudaLaunchCooperativeKernel((const void *)kern, dim3(tp.gt * tp.gx), dim3(nt), args, 0, s);
   if (e == cudaErrorCooperativeLaunchTooLarge) {  // fewer SMs free: the other forms
     cudaGetLastError();
     return cudaErrorNotSupported;

@@ -102,8 +102,8 @@ int finish_status(su2b_ctx *ctx, int done) {
   return SU2B_OK;
 }
 
-// The tiled CG's plan and packets, made for the first CG of a context (BiCGStab and CG_mixed
-// do without them); without room for them the other forms run.
+// The tiled solves' plan and packets, made for the first solve of a context; without room for
+// them the other forms run.
 int cg_tile_setup(su2b_ctx *ctx) {
   if (ctx->cg_planned) return SU2B_OK;
   ctx->cg_planned = true;
@@ -125,17 +125,22 @@ int cg_tile_setup(su2b_ctx *ctx) {
 
 // d = 2 up to about 150,000 sites: the whole solve, restarts included, in one launch on tiles.
 // ran: false where another form has to run.
-int cg_tiled(su2b_ctx *ctx, double m, double tol, int max_iter, su2b_solve_stats *stats,
-             bool *ran) {
+int cg_tiled(su2b_ctx *ctx, bool bicgstab, double m, double tol, int max_iter,
+             su2b_solve_stats *stats, bool *ran) {
   *ran = false;
   SU2B_CKS(cg_tile_setup(ctx));
   if (!ctx->cg_plan.K) return SU2B_OK;
+  if (bicgstab) {
+    if (ctx->bi_tiled < 0) ctx->bi_tiled = cg_tile_bicgstab(ctx->cg_plan);
+    if (!ctx->bi_tiled) return SU2B_OK;
+  }
   cudaStream_t s = ctx->stream;
   CgTileResult &h = *ctx->h_cg;
   h.done = 0;
   h.failed = 0;
-  const cudaError_t e = cg_tile(ctx->g, ctx->cg_plan, ctx->ph, m, ctx->sv[SV_B], ctx->sv[SV_X],
-                                tol, max_iter, ctx->cg_work, ctx->cg_epoch, ctx->h_cg, s);
+  const cudaError_t e = cg_tile(ctx->g, ctx->cg_plan, bicgstab, ctx->ph, m, ctx->sv[SV_B],
+                                ctx->sv[SV_X], tol, max_iter, ctx->cg_work, ctx->cg_epoch,
+                                ctx->h_cg, s);
   if (e == cudaErrorNotSupported) return SU2B_OK;
   SU2B_CK(e);
   ctx->launches++;
@@ -143,7 +148,7 @@ int cg_tiled(su2b_ctx *ctx, double m, double tol, int max_iter, su2b_solve_stats
   if (es != cudaSuccess || h.failed) {
     ctx->cg_epoch += 1ull << 40;  // past every epoch the failed solve can have used
     SU2B_CK(es);
-    return su2b_fail(ctx, SU2B_ERR_TIMEOUT, "tiled CG: a wait for another block gave up");
+    return su2b_fail(ctx, SU2B_ERR_TIMEOUT, "tiled solve: a wait for another block gave up");
   }
   ctx->cg_epoch = h.epoch;
   *ran = true;
@@ -165,7 +170,7 @@ int cg64(su2b_ctx *ctx, double m, double tol, int max_iter, su2b_solve_stats *st
           *t = ctx->sv[SV_T], *Ap = ctx->sv[SV_AP];
   double *dp = ctx->part_slot(3), *np = ctx->part_slot(4);
   bool ran = false;
-  const int rc = cg_tiled(ctx, m, tol, max_iter, stats, &ran);
+  const int rc = cg_tiled(ctx, false, m, tol, max_iter, stats, &ran);
   if (rc != SU2B_OK || ran) return rc;
   SU2B_CKS(true_residual(ctx, m, true, b, x, r, 20));
   SU2B_CKS(su2b_fetch_red(ctx, 21));
@@ -245,6 +250,9 @@ int bicgstab64(su2b_ctx *ctx, double m, double tol, int max_iter, su2b_solve_sta
           *t = ctx->sv[SV_T], *Ap = ctx->sv[SV_AP], *sv = ctx->sv[SV_S], *r0 = ctx->sv[SV_R0];
   double *dp = ctx->part_slot(3), *np = ctx->part_slot(3) + 2 * ctx->part_cap;
   double *dp2 = ctx->part_slot(5), *np2 = ctx->part_slot(5) + 2 * ctx->part_cap;
+  bool ran = false;
+  const int rc = cg_tiled(ctx, true, m, tol, max_iter, stats, &ran);
+  if (rc != SU2B_OK || ran) return rc;
   SU2B_CKS(true_residual(ctx, m, false, b, x, r0, 20));
   SU2B_CKS(su2b_fetch_red(ctx, 21));
   SolverState h{};
@@ -326,7 +334,7 @@ int cg_mixed(su2b_ctx *ctx, double m, double tol, int max_iter, double delta,
   // (at mass 0.05, to 1e-12: 32^2 0.43 against 2.11 ms, 64^2 0.77 / 3.23, 256^2 2.18 / 3.93,
   // 380 x 390 3.59 / 5.22).  Its closing true residual counts as the FP64 update it is.
   bool ran = false;
-  const int rc = cg_tiled(ctx, m, tol, max_iter, stats, &ran);
+  const int rc = cg_tiled(ctx, false, m, tol, max_iter, stats, &ran);
   if (ran && stats) {
     stats->restarts++;
     if (rc != SU2B_OK) stats->true_residual = stats->residual;

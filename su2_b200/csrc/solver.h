@@ -6,6 +6,23 @@
 
 namespace su2b {
 
+__device__ __forceinline__ double2 cm(double2 a, double2 b) {
+  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double2 cmc(double2 a, double2 b) {  // conj(a) * b
+  return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
+}
+// libgcc's complex division for ordinary magnitudes (Smith, CACM 5 (1962) 435)
+__device__ __forceinline__ double2 cdivs(double2 x, double2 y) {
+  const double a = x.x, b = x.y, c = y.x, d = y.y;
+  if (fabs(c) < fabs(d)) {
+    const double ratio = c / d, denom = (c * ratio) + d;
+    return make_double2(((a * ratio) + b) / denom, ((b * ratio) - a) / denom);
+  }
+  const double ratio = d / c, denom = (d * ratio) + c;
+  return make_double2(((b * ratio) + a) / denom, (b - (a * ratio)) / denom);
+}
+
 // Scalars of one solve, kept in device memory so iterations run without host round trips.
 // done: 0 running, 1 converged, 2 iteration limit, 3 NaN residual.
 struct SolverState {
@@ -89,8 +106,9 @@ struct CgTileResult {
 };
 CgTilePlan cg_tile_plan(const Geom &g);
 size_t cg_tile_bytes(const Geom &g);
-cudaError_t cg_tile(const Geom &g, const CgTilePlan &tp, const double2 *ph, double m,
-                    const double2 *b, double2 *x, double tol, long max_iter, void *work,
+bool cg_tile_bicgstab(const CgTilePlan &p);
+cudaError_t cg_tile(const Geom &g, const CgTilePlan &tp, bool bicgstab, const double2 *ph,
+                    double m, const double2 *b, double2 *x, double tol, long max_iter, void *work,
                     unsigned long long epoch, CgTileResult *out, cudaStream_t s);
 int cg_barrier_failed(const void *bar_mem, cudaStream_t s, int *failed);
 size_t cg_barrier_bytes();

@@ -23,23 +23,6 @@ template <class R> struct C2;
 template <> struct C2<double> { typedef double2 type; };
 template <> struct C2<float> { typedef float2 type; };
 
-__device__ __forceinline__ double2 cm(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cmc(double2 a, double2 b) {  // conj(a) * b
-  return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
-}
-// libgcc's complex division for ordinary magnitudes (Smith, CACM 5 (1962) 435)
-__device__ __forceinline__ double2 cdivs(double2 x, double2 y) {
-  const double a = x.x, b = x.y, c = y.x, d = y.y;
-  if (fabs(c) < fabs(d)) {
-    const double ratio = c / d, denom = (c * ratio) + d;
-    return make_double2(((a * ratio) + b) / denom, ((b * ratio) - a) / denom);
-  }
-  const double ratio = d / c, denom = (d * ratio) + c;
-  return make_double2(((b * ratio) + a) / denom, (b - (a * ratio)) / denom);
-}
-
 __device__ __forceinline__ bool finished(const SolverState *st) {
   return st != nullptr && st->done != 0;
 }

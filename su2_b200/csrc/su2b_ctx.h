@@ -56,6 +56,7 @@ struct su2b_ctx {
   // the tiled CG (cg_tile.cu): its plan (K = 0: not for this lattice), packets and their epoch
   su2b::CgTilePlan cg_plan{};
   bool cg_planned = false;
+  int bi_tiled = -1;  // whether the BiCGStab runs on the plan (-1: not asked yet)
   void *cg_work = nullptr;
   unsigned long long cg_epoch = 0;
   su2b::CgTileResult *h_cg = nullptr;

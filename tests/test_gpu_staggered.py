@@ -221,6 +221,34 @@ def test_operator_and_solve_at_1024_squared(gpu):
         assert rel(out["shifted"][3], shift(out["plain"][3], 2)) < 1e-8
 
 
+@pytest.mark.parametrize("Lx,Lt", [(2, 2), (6, 4), (2, 600), (300, 2), (26, 38), (64, 64), (90, 90),
+                                   (130, 134), (256, 250), (300, 340), (440, 400)])
+def test_bicgstab_tilings(gpu, Lx, Lt):
+    """The BiCGStab on the same tilings (and past them), sharing the CG's packets: the residual
+    of its solution by the stand-alone D is the one it reports and below the tolerance.
+    Rounding of b - D x: |D| |x| times a few eps, with |x| <= |b| / m and |D| <= m + 2."""
+    rng = np.random.default_rng(Lx * 1000 + Lt)
+    V, m, tol = Lx * Lt, 0.3, 1e-10
+    b = rng.normal(size=2 * V)
+    nb = np.linalg.norm(b)
+    slack = 20 * 2.2e-16 * (m + 2) / m * nb
+    with u1(gpu, (Lx, 1, 1, Lt), 2) as c:
+        c.upload(rng.normal(size=2 * V))
+        for _ in range(2):
+            r = c.solve(b, m, tol=tol, tol_mode="rel", solver="BiCGStab")
+            res = np.linalg.norm(b - c.apply_D(m, r.x))
+            assert r.converged
+            assert r.true_residual <= tol * nb + slack
+            assert res == pytest.approx(r.true_residual, abs=slack)
+            assert c.solve(b, m, tol=tol, tol_mode="rel").converged
+        again = c.solve(b, m, tol=2 * tol, tol_mode="rel", x0=r.x, solver="BiCGStab")
+        assert again.converged and again.iterations == 0 and np.array_equal(again.x, r.x)
+        few = c.solve(b, m, tol=1e-14, tol_mode="rel", max_iter=2, solver="BiCGStab")
+        assert few.iterations <= 2
+        zero = c.solve(np.zeros(2 * V), m, tol=1e-10, solver="BiCGStab")
+        assert zero.converged and zero.iterations == 0 and not zero.x.any()
+
+
 # one block; clusters of 2..16 with partial and one-row tiles; the largest of one and two sites
 # per thread; whole-GPU tilings of one and two sites per thread; past them the grid-barrier form
 @pytest.mark.parametrize("Lx,Lt", [(2, 2), (6, 4), (22, 24), (2, 600), (300, 2), (26, 38), (64, 64),
