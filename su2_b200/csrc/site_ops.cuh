@@ -127,6 +127,10 @@ __device__ __forceinline__ double force_site_impl(const Geom &g, const LinkT<T> 
 #pragma unroll
     for (int mu = 0; mu < ND; mu++) prefetch_momenta(P, mu * V + self, NL);
   }
+  if (mode & FM_EXTRA) {
+#pragma unroll
+    for (int mu = 0; mu < ND; mu++) prefetch_momenta(extra, mu * V + self, NL);
+  }
 #pragma unroll
   for (int mu = 0; mu < ND; mu++) {
     ux[mu] = ld_link(U + mu * V + self);
