@@ -170,6 +170,8 @@ extern "C" int su2b_ctx_create(int group, int Lx, int Ly, int Lz, int Lt, int nd
       cudaMallocHost((void **)&ctx->h_tparams, sizeof(TrajParams)) != cudaSuccess)
     return fin(SU2B_ERR_NOMEM);
   if (cudaMemsetAsync(ctx->U, 0, lb * NL, ctx->stream) != cudaSuccess ||
+      cudaMemsetAsync(ctx->counts, 0, 4 * sizeof(unsigned long long), ctx->stream) !=
+        cudaSuccess ||
       cudaMemsetAsync(ctx->ticket, 0, sizeof(unsigned), ctx->stream) != cudaSuccess)
     return fin(SU2B_ERR_CUDA);
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fin(SU2B_ERR_CUDA);
@@ -479,18 +481,17 @@ extern "C" int su2b_metropolis_sweep(su2b_ctx *ctx, double delta, int N_hit, uin
   CKS(enter(ctx));
   NEED(rates, "rates is NULL");
   NEED(N_hit >= 0, "N_hit < 0");
-  CK(cudaMemsetAsync(ctx->counts, 0, 2 * sizeof(unsigned long long), ctx->stream));
   for (int mu = 0; mu < ctx->g.nd; mu++)
     for (int p = 0; p < 2; p++) {
+      const bool last = mu == ctx->g.nd - 1 && p == 1;
+      const MetroCounts counts{ctx->counts, last ? ctx->h_counts : nullptr, ctx->ticket};
       if (ctx->link64)
         SU2B_LAUNCH(SU2B_K_METROPOLIS, metropolis_pass<double>(ctx->g, ctx->U, ctx->group, mu, p, ctx->beta, ctx->xi, delta, N_hit,
-                                   seed, sweep, ctx->counts, ctx->stream));
+                                   seed, sweep, counts, ctx->stream));
       else
         SU2B_LAUNCH(SU2B_K_METROPOLIS, metropolis_pass<float>(ctx->g, ctx->U, ctx->group, mu, p, ctx->beta, ctx->xi, delta, N_hit,
-                                  seed, sweep, ctx->counts, ctx->stream));
+                                  seed, sweep, counts, ctx->stream));
     }
-  CK(cudaMemcpyAsync(ctx->h_counts, ctx->counts, 2 * sizeof(unsigned long long),
-                     cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->phases_valid = false;
   if (ctx->pend.size() > 4096) CKS(su2b_prof_fold(ctx));

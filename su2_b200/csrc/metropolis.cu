@@ -114,10 +114,25 @@ __device__ __forceinline__ unsigned metro_hit(Su2<T> &u, double &tr_u, const Su2
   return 1;
 }
 
+// a block's accepted hits (one thread of each block); a memset before each sweep and a copy after
+// it: 44 us a sweep at 100^2 instead of 41, 70 instead of 64 at 48x40x36
+__device__ __forceinline__ void leave_count(const MetroCounts &c, unsigned acc, int mu) {
+  if (acc) {
+    atomicAdd(c.total, (unsigned long long)acc);
+    if (mu == 0) atomicAdd(c.total + 1, (unsigned long long)acc);
+  }
+  if (!c.out) return;
+  __threadfence();
+  if (atomicInc(c.ticket, gridDim.x - 1) != gridDim.x - 1) return;
+  __threadfence();
+  c.out[0] = atomicExch(c.total, 0ull);
+  c.out[1] = atomicExch(c.total + 1, 0ull);
+}
+
 template <class T, int ND, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
   k_metro_su2(Geom g, LinkT<T> *__restrict__ U, int mu, int p, double beta_nc, double delta,
-              int N_hit, uint64_t seed, uint32_t sweep, unsigned long long *counts, T wt, T ws) {
+              int N_hit, uint64_t seed, uint32_t sweep, MetroCounts counts, T wt, T ws) {
   __shared__ unsigned int sh_acc;
   if (threadIdx.x == 0) sh_acc = 0;
   // as pdl_start: the next pass's blocks enter early behind the last wave of several, not
@@ -149,10 +164,7 @@ __global__ void __launch_bounds__(NT, MINB)
   }
   if (acc) atomicAdd(&sh_acc, acc);
   __syncthreads();
-  if (threadIdx.x == 0 && sh_acc) {
-    atomicAdd(counts, (unsigned long long)sh_acc);
-    if (mu == 0) atomicAdd(counts + 1, (unsigned long long)sh_acc);
-  }
+  if (threadIdx.x == 0) leave_count(counts, sh_acc, mu);
 }
 
 // The same for passes of few links, which the chain of a link's hits bounds: a block of eight
@@ -165,7 +177,7 @@ constexpr int WIDE_HITS = 16;
 template <class T, int ND>
 __global__ void __launch_bounds__(256, 2)
   k_metro_su2_wide(Geom g, LinkT<T> *__restrict__ U, int mu, int p, double beta_nc, double delta,
-                   int N_hit, uint64_t seed, uint32_t sweep, unsigned long long *counts, T wt,
+                   int N_hit, uint64_t seed, uint32_t sweep, MetroCounts counts, T wt,
                    T ws) {
   __shared__ LinkT<T> prop[2][WIDE_HITS][32];
   __shared__ double acc_u[2][WIDE_HITS][32];
@@ -209,16 +221,13 @@ __global__ void __launch_bounds__(256, 2)
   else
     acc = 0;
   acc = __reduce_add_sync(0xffffffffu, acc);
-  if (lane == 0 && acc) {
-    atomicAdd(counts, (unsigned long long)acc);
-    if (mu == 0) atomicAdd(counts + 1, (unsigned long long)acc);
-  }
+  if (lane == 0) leave_count(counts, acc, mu);
 }
 
 template <int ND, int NT>
 __global__ void __launch_bounds__(NT)
   k_metro_u1(Geom g, double *__restrict__ U, int mu, int p, double beta, double delta,
-             int N_hit, uint64_t seed, uint32_t sweep, unsigned long long *counts, double wt,
+             int N_hit, uint64_t seed, uint32_t sweep, MetroCounts counts, double wt,
              double ws) {
   __shared__ unsigned int sh_acc;
   if (threadIdx.x == 0) sh_acc = 0;
@@ -277,10 +286,7 @@ __global__ void __launch_bounds__(NT)
   }
   if (acc) atomicAdd(&sh_acc, acc);
   __syncthreads();
-  if (threadIdx.x == 0 && sh_acc) {
-    atomicAdd(counts, (unsigned long long)sh_acc);
-    if (mu == 0) atomicAdd(counts + 1, (unsigned long long)sh_acc);
-  }
+  if (threadIdx.x == 0) leave_count(counts, sh_acc, mu);
 }
 
 }  // namespace
@@ -288,7 +294,7 @@ __global__ void __launch_bounds__(NT)
 template <class T>
 cudaError_t metropolis_pass(const Geom &g, void *U, int group, int mu, int parity, double beta,
                             double xi, double delta, int N_hit, uint64_t seed, uint32_t sweep,
-                            unsigned long long *counts, cudaStream_t s) {
+                            const MetroCounts &counts, cudaStream_t s) {
   constexpr int NT = 128, MINB = 8;
   // anisotropic weights of get_staples (get_staples.hh:58-79): 1/xi for planes with
   // direction 0, xi otherwise; both 1 (exactly) for the isotropic action
@@ -333,9 +339,9 @@ cudaError_t metropolis_pass(const Geom &g, void *U, int group, int mu, int parit
 
 template cudaError_t metropolis_pass<double>(const Geom &, void *, int, int, int, double, double,
                                              double, int, uint64_t, uint32_t,
-                                             unsigned long long *, cudaStream_t);
+                                             const MetroCounts &, cudaStream_t);
 template cudaError_t metropolis_pass<float>(const Geom &, void *, int, int, int, double, double,
                                             double, int, uint64_t, uint32_t,
-                                            unsigned long long *, cudaStream_t);
+                                            const MetroCounts &, cudaStream_t);
 
 }  // namespace su2b

@@ -782,11 +782,11 @@ extern "C" int su2b_slabs_metropolis_sweep(su2b_slabs *h, double delta, int N_hi
         if (h->link64)
           SLAB_LAUNCH(c, SU2B_K_METROPOLIS,
                       metropolis_pass<double>(c->g, c->U, 0, mu, pl, c->beta, c->xi, delta,
-                                              N_hit, seed, sweep, c->counts, h->s));
+                                              N_hit, seed, sweep, {c->counts}, h->s));
         else
           SLAB_LAUNCH(c, SU2B_K_METROPOLIS,
                       metropolis_pass<float>(c->g, c->U, 0, mu, pl, c->beta, c->xi, delta,
-                                             N_hit, seed, sweep, c->counts, h->s));
+                                             N_hit, seed, sweep, {c->counts}, h->s));
       }
       SU2B_CKS(exchange(h, h->role[0], 2 * mu + pl));
     }

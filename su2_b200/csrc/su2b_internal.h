@@ -131,10 +131,18 @@ cudaError_t cond_restore(const Geom &g, void *U, const void *U_old, int group,
                          const TrajDev *flag, cudaStream_t s);
 
 // ---- Metropolis ----
+// Accepted hits of a sweep: total[0] of all links, total[1] of the links in direction 0.  The
+// pass with `out` set is the sweep's last: the block that ends last writes both to out (pinned
+// host memory) and zeroes them for the next sweep.
+struct MetroCounts {
+  unsigned long long *total;
+  unsigned long long *out;
+  unsigned *ticket;
+};
 template <class T>
 cudaError_t metropolis_pass(const Geom &g, void *U, int group, int mu, int parity, double beta,
                             double xi, double delta, int N_hit, uint64_t seed, uint32_t sweep,
-                            unsigned long long *counts, cudaStream_t s);
+                            const MetroCounts &counts, cudaStream_t s);
 
 // ---- clover energy density / charge ----
 // per-block partials {E, E_ss, Q}; fin.out: their sums over the blocks as well
