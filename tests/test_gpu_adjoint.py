@@ -126,6 +126,39 @@ def test_flow_adjoint_finite_differences(gpu, orc, every):
                 assert fd == pytest.approx(g[3 * link + k], abs=1e-7 + 1e-6 * np.abs(g).max())
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("dims,nd,n", [((4, 1, 1, 6), 2, 1), ((6, 4, 1, 4), 3, 2), ((4, 6, 4, 8), 4, 5),
+                                       ((4, 4, 4, 4), 4, 30)])
+def test_flow_adjoint_tape(gpu, orc, dims, nd, n, precision):
+    """Every stage kept against checkpoints and recomputed stages: the same objective and
+    gradient to the rounding of the stages' sums (one product and one addition, fused in one
+    and not in the other), grown over 3 n stages; and the same bits from a second call."""
+    U = orc.hotstart(0, dims, nd, 12, 1.0, 4321)
+    tol = 3 * n * (1e-14 if precision == "fp64" else 1e-6)
+    with gpu.gaugeconfig(*dims, nd, 2.4, precision=precision) as c:
+        c.upload(U)
+        O, g = c.flow_objective(0.02, n)
+        O2, g2 = c.flow_objective(0.02, n)
+        assert O == O2 and np.array_equal(g, g2)
+        for every in (1, 3):
+            Oc, gc = c.flow_objective(0.02, n, checkpoint_every=every)
+            assert O == pytest.approx(Oc, rel=tol)
+            assert np.linalg.norm(g - gc) <= tol * np.linalg.norm(gc)
+        assert c.flow_objective(0.02, n, grad=False) == pytest.approx(O, rel=tol)
+
+
+def test_flow_adjoint_tape_limit(gpu, orc):
+    """More steps than the tape may hold (8 GB: about 3,100 steps of an 8^4 FP64 lattice) take
+    the checkpoints that they took without it: the bits of the explicit choice."""
+    dims, n = (8, 8, 8, 8), 3200
+    U = orc.hotstart(0, dims, 4, 13, 1.0, 4321)
+    with gpu.gaugeconfig(*dims, 4, 2.4) as c:
+        c.upload(U)
+        O, g = c.flow_objective(1e-4, n)
+        Oc, gc = c.flow_objective(1e-4, n, checkpoint_every=round(n ** 0.5))
+        assert O == Oc and np.array_equal(g, gc)
+
+
 def test_flow_objective_matches_flow_records(gpu, orc):
     dims, nd = (4, 4, 4, 4), 4
     U = orc.hotstart(0, dims, nd, 11, 1.0, 654321)
