@@ -31,14 +31,13 @@
 #include <utility>
 #include <vector>
 
+#include "site_ops.cuh"
 #include "su2b.h"
 #include "su2b_ctx.h"
 
 using namespace su2b;
 
 namespace {
-
-template <class T> using LinkT = typename LinkOf<T>::type;
 
 // an algebra element i (x s_x + y s_y + z s_z): {Im b, Re b, Im a} of the (a, b) storage
 template <class T> struct V3 {
@@ -100,6 +99,7 @@ template <class T, int ND, int NT>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
   k_force_vjp(Geom g, const LinkT<T> *__restrict__ U, const T *__restrict__ mu,
               Sent<T, ND> sent) {
+  pdl_start<(sizeof(T) == 4 ? 5 : 3)>();
   const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
   const int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
   if (cb >= g.Vh) return;
@@ -228,6 +228,7 @@ template <class T, int ND, int NT, bool EXP>
 __global__ void __launch_bounds__(NT)
   k_force_vjp_gather(Geom g, Sent<T, ND> sent, T *__restrict__ lam, T coef,
                      int acc_lam, const T *__restrict__ Z, T b, T *__restrict__ mu, int acc_mu) {
+  pdl_start<5>();
   const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
   const int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
   if (cb >= g.Vh) return;
@@ -277,12 +278,9 @@ cudaError_t force_vjp_send(const Geom &g, const void *U, const T *mu, void *cons
   const int grid = (g.Vh + NT / 2 - 1) / (NT / 2);
   const LinkT<T> *u = (const LinkT<T> *)U;
 #define SU2B_SEND(ND)                                                                      \
-  k_force_vjp<T, ND, NT><<<grid, NT, 0, s>>>(g, u, mu, sent_in<T, ND>(spare))
-  if (g.nd == 2) SU2B_SEND(2);
-  else if (g.nd == 3) SU2B_SEND(3);
-  else SU2B_SEND(4);
+  launch_force(k_force_vjp<T, ND, NT>, dim3(grid), NT, s, true, 0, g, u, mu, sent_in<T, ND>(spare))
+  return g.nd == 2 ? SU2B_SEND(2) : g.nd == 3 ? SU2B_SEND(3) : SU2B_SEND(4);
 #undef SU2B_SEND
-  return cudaGetLastError();
 }
 template <class T>
 cudaError_t force_vjp_gather(const Geom &g, T *lam, double coef, int acc, void *const (&spare)[3],
@@ -290,13 +288,14 @@ cudaError_t force_vjp_gather(const Geom &g, T *lam, double coef, int acc, void *
   constexpr int NT = 128;
   const int grid = (g.Vh + NT / 2 - 1) / (NT / 2);
 #define SU2B_GATHER(ND, EXP)                                                               \
-  k_force_vjp_gather<T, ND, NT, EXP><<<grid, NT, 0, s>>>(g, sent_in<T, ND>(spare), lam, (T)coef, acc, Z, \
-                                                         (T)b, mu, acc_mu)
-  if (g.nd == 2) Z ? SU2B_GATHER(2, true) : SU2B_GATHER(2, false);
-  else if (g.nd == 3) Z ? SU2B_GATHER(3, true) : SU2B_GATHER(3, false);
-  else Z ? SU2B_GATHER(4, true) : SU2B_GATHER(4, false);
+  launch_force(k_force_vjp_gather<T, ND, NT, EXP>, dim3(grid), NT, s, true, 0, g,           \
+               sent_in<T, ND>(spare), lam, (T)coef, acc, Z, (T)b, mu, acc_mu)
+  switch (g.nd) {
+    case 2: return Z ? SU2B_GATHER(2, true) : SU2B_GATHER(2, false);
+    case 3: return Z ? SU2B_GATHER(3, true) : SU2B_GATHER(3, false);
+    default: return Z ? SU2B_GATHER(4, true) : SU2B_GATHER(4, false);
+  }
 #undef SU2B_GATHER
-  return cudaGetLastError();
 }
 template <class T>
 cudaError_t exp_adjoint(const Geom &g, const T *Z, double b, T *lam, T *mu, cudaStream_t s) {
