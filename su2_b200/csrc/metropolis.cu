@@ -64,9 +64,12 @@ __device__ __forceinline__ Su2<float> proposal(uint32_t lref, int n, uint32_t sw
   uint32_t r[4];
   philox(lref, (uint32_t)n, sweep, TAG_METRO, seed, r);
   float sa, ca, st, ct;
-  sincospif(2.0f * delta * (float)u01_32(r[0]), &sa, &ca);
-  const float uu = fmaf(2.0f, (float)u01_32(r[1]), -1.0f);
-  sincospif(2.0f * (float)u01_32(r[2]), &st, &ct);
+  // x 2^-32 rounded once to FP32 (a power of two: as the FP64 uniform rounded); the conversions
+  // through FP64 run at a quarter of the rate (32^4 mixed 446 us a sweep instead of 434)
+  auto u01 = [](uint32_t x) { return __uint2float_rn(x) * 0x1p-32f; };
+  sincospif(2.0f * delta * u01(r[0]), &sa, &ca);
+  const float uu = fmaf(2.0f, u01(r[1]), -1.0f);
+  sincospif(2.0f * u01(r[2]), &st, &ct);
   const float rr = sqrtf(fmaxf(0.0f, fmaf(-uu, uu, 1.0f)));
   accept = u01_32(r[3]);
   return Su2<float>{ca, sa * uu, sa * rr * st, sa * rr * ct};
