@@ -443,14 +443,13 @@ int flow_adjoint_tape(su2b_ctx *ctx, double eps, int n, Scratch *sc, double *obj
   T *const lam = (T *)sc->get(ab), *const mu = (T *)sc->get(ab);
   const FlowCoef c = flow_coef(ctx, eps);
   SU2B_CK(cudaMemcpyAsync(W[0], ctx->U, lb, cudaMemcpyDeviceToDevice, ctx->stream));
-  const int restore = ctx->link64 ? 0 : FM_RESTORE;
   for (int st = 0; st < n; st++) {
     for (int f = 0; f < 3; f++) {
       const int k = 3 * st + f;
       SU2B_CKS(su2b_q_force(ctx, W[k], Z[k], f ? Z[k - 1] : nullptr, c.a[f], 1.0,
-                            FM_UPDATE | (f ? FM_EXTRA : 0) | (f == 2 ? restore : 0), nullptr,
-                            nullptr, W[k + 1], c.b[f]));
+                            FM_UPDATE | (f ? FM_EXTRA : 0), nullptr, nullptr, W[k + 1], c.b[f]));
     }
+    if (!ctx->link64) SU2B_CKS(su2b_q_restore(ctx, W[3 * st + 3]));
   }
   SU2B_CKS(su2b_q_plaq(ctx, W[3 * n], ctx->h_red + 40));
   const double t = n * eps, VNc = (double)ctx->V * ctx->Nc();
@@ -528,7 +527,8 @@ int flow_adjoint_t(su2b_ctx *ctx, double eps, int n, int every, double *objectiv
     for (int j = 1; j < s1 - s0; j++) {  // seg[j-1] -> seg[j] through W2, seg[j-1] kept
       SU2B_CKS(force(seg[j - 1], Zs[0], c.a[0], 0, seg[j], c.b[0]));
       SU2B_CKS(force(seg[j], Zs[0], c.a[1], FM_HAS_IN, W2, c.b[1]));
-      SU2B_CKS(force(W2, Zs[0], c.a[2], FM_HAS_IN | (ctx->link64 ? 0 : FM_RESTORE), seg[j], c.b[2]));
+      SU2B_CKS(force(W2, Zs[0], c.a[2], FM_HAS_IN, seg[j], c.b[2]));
+      if (!ctx->link64) SU2B_CKS(su2b_q_restore(ctx, seg[j]));
     }
     for (int j = s1 - s0 - 1; j >= 0; j--) {
       const void *W0 = seg[j];

@@ -527,17 +527,14 @@ int su2b_q_flow_step_to(su2b_ctx *ctx, void *src, void *dst, double eps) {
   void *other = in_place ? ctx->U2 : dst;
   const int nfused = !su2 || (in_place && src == ctx->U2) ? 0 : (in_place ? 2 : 3);
   void *W = src;
-  bool restored = false;  // by the last stage's launch
   for (int f = 0; f < 3; f++) {
     const double fac = 2. * Nc * zfac[f] / ctx->beta;
     const double ff = fac * ctx->beta / (double)Nc;
     const int mode = f == 0 ? 0 : FM_HAS_IN;
     if (f < nfused) {
       void *next = W == src ? other : src;
-      restored = f == 2 && !ctx->link64;
-      CKS(su2b_q_force(ctx, W, ctx->Z, nullptr, ff, 1.0,
-                       mode | FM_UPDATE | (restored ? FM_RESTORE : 0), nullptr, nullptr, next,
-                       -eps * expfac[f]));
+      CKS(su2b_q_force(ctx, W, ctx->Z, nullptr, ff, 1.0, mode | FM_UPDATE, nullptr, nullptr,
+                       next, -eps * expfac[f]));
       W = next;
       ctx->phases_valid = false;
     } else {
@@ -548,10 +545,8 @@ int su2b_q_flow_step_to(su2b_ctx *ctx, void *src, void *dst, double eps) {
   // FP32 links: every exp(.)U product rounds |U| by about one ulp in a direction that does not
   // average out over hundreds of steps, and the flowed plaquette (close to 1) amplifies that
   // drift in E = d(d-1)/2 - P/(V Nc).  Reunitarise in FP64 after each step, as the trajectory
-  // does at its end; FP64 links keep the reference's step unchanged.  The last stage's launch
-  // does it on the links that it writes (20 records at 24^4: 3.97 ms, 3.78 ms without the extra
-  // pass over the links).
-  if (!ctx->link64 && su2 && !restored) CKS(su2b_q_restore(ctx, W));
+  // does at its end; FP64 links keep the reference's step unchanged.
+  if (!ctx->link64 && su2) CKS(su2b_q_restore(ctx, W));
   return SU2B_OK;
 }
 int su2b_q_flow_step(su2b_ctx *ctx, void *U, double eps) {

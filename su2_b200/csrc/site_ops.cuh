@@ -95,11 +95,9 @@ __device__ __forceinline__ double finish_link(const Su2<T> &u, const Su2<T> &k, 
   P[l] = p0;
   P[NL + l] = p1;
   P[2 * NL + l] = p2;
-  if (mode & FM_UPDATE) {
-    Su2<T> w = mul(exp_alg(dt_upd * p0, dt_upd * p1, dt_upd * p2), u);
-    if (mode & FM_RESTORE) w = from64<T>(restore_su(to64(w)));
-    st_link(Uout + l, w);
-  } else if (mode & FM_RESTORE)
+  if (mode & FM_UPDATE)
+    st_link(Uout + l, mul(exp_alg(dt_upd * p0, dt_upd * p1, dt_upd * p2), u));
+  else if (mode & FM_RESTORE)
     st_link(Uout + l, from64<T>(restore_su(to64(u))));
   // |P|^2 in FP64 only where the launch sums it (a uniform branch)
   if (!(mode & FM_KINETIC)) return 0.;

@@ -36,8 +36,7 @@ enum ForceMode : int {
   FM_KINETIC = 2,    // also write per-block partials of sum P_out^2
   FM_EXTRA = 4,      // add extra[] (another monomial's derivative) to f*g before scaling
   FM_UPDATE = 8,     // SU(2): also write Uout = exp(dt_upd * P_out) U (the next gauge step)
-  FM_RESTORE = 16    // SU(2): also write Uout = restoreSU(U) (the end of the trajectory); with
-                     // FM_UPDATE, Uout = restoreSU(exp(dt_upd * P_out) U) (the end of a flow step)
+  FM_RESTORE = 16    // SU(2): also write Uout = restoreSU(U) (the end of the trajectory)
 };
 // launch shapes of the SU(2) force kernel (threads per block, minimum resident blocks per
 // SM, which caps registers): one thread per site 0 (256,4) 1 (128,8) 2 (128,4) 3 (128,6)
