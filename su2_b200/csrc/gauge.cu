@@ -553,12 +553,14 @@ __global__ void k_accept(const double *__restrict__ red, const TrajParams *__res
   accept_body(red, tp, out);
 }
 // The end of a fused trajectory in one launch: the plaquettes of the final field (as
-// k_plaq_su2), and in the block that finishes last the closing sums and the accept step.  It
-// adds up the start partials (momenta pass, 4 components, skipped when ns = 0) into red[0..3],
-// the final kinetic partials into red[4] (skipped when nk = 0) and the end plaquettes into
-// red[5..7], each in an order fixed by the grids, and writes red[0..9] and the result to the
-// pinned host copies as well.  A separate reduction launch, two copies and a memset that it
-// replaces took 13 us of the 70 us of a trajectory of ten steps at 8^4.
+// k_plaq_su2), the closing sums and the accept step.  Each block also adds its share of the
+// start partials (momenta pass, 4 components, none when ns = 0) and of the final kinetic
+// partials; the block that finishes last adds the blocks up into red[0..3], red[4] (skipped when
+// nk = 0) and red[5..7], in an order fixed by the grids, and writes red[0..9] and the result to
+// the pinned host copies as well.  A separate reduction launch, two copies and a memset that it
+// replaces took 13 us of the 70 us of a trajectory of ten steps at 8^4; with all the earlier
+// partials left to the last block a mixed trajectory at 32^4 takes 805 to 820 us instead of 785
+// to 790.
 // cached_start: the momenta pass summed no plaquettes (its components 1..3 are zero); the
 // start field is the previous trajectory's result, whose plaquette sums are still in red[]:
 // red[5..7] if that trajectory was accepted (out->accepted), else red[1..3].  They are taken
@@ -567,28 +569,27 @@ template <class T, int ND, int NT>
 __global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
   k_plaq_accept_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part,
                     TrajTail e) {
-  constexpr int NC = 8;
+  constexpr int NC = 8;  // start |P|^2 and three plaquette sums, end |P|^2, three plaquette sums
   __shared__ double shk[NC * (NT / 32)];
   pdl_wait();
-  double v[3] = {0., 0., 0.};
+  double v[3] = {0., 0., 0.}, a[NC];
   plaq_bands<T, ND, NT>(g, U, xi, v);
-  if (!leave_sums<NT, 3>(v, part, e.ticket, shk)) return;
-  double a[NC];
+#pragma unroll
+  for (int k = 0; k < NC; k++) a[k] = k < 5 ? 0. : v[k - 5];
+  // every block also takes its share of the earlier launches' partials (16,384 of the force
+  // launch at 32^4), so the last one adds only the blocks of this launch
+  const int first = blockIdx.x * NT + threadIdx.x, stride = gridDim.x * NT;
+  for (int b = first; b < e.ns; b += stride)
+#pragma unroll
+    for (int k = 0; k < 4; k++) a[k] += e.ps[(size_t)b * 4 + k];
+  for (int b = first; b < e.nk; b += stride) a[4] += e.pk[b];
+  if (!leave_sums<NT, NC>(a, part, e.ticket, shk)) return;
 #pragma unroll
   for (int k = 0; k < NC; k++) a[k] = 0.;
-  const int nmax = max(e.ns, max(e.nk, (int)gridDim.x));
 #pragma unroll 2
-  for (int b = threadIdx.x; b < nmax; b += NT) {
-    if (b < e.ns) {
+  for (int b = threadIdx.x; b < (int)gridDim.x; b += NT)
 #pragma unroll
-      for (int k = 0; k < 4; k++) a[k] += e.ps[(size_t)b * 4 + k];
-    }
-    if (b < e.nk) a[4] += e.pk[b];
-    if (b < (int)gridDim.x) {
-#pragma unroll
-      for (int k = 0; k < 3; k++) a[5 + k] += __ldcg(part + (size_t)b * 3 + k);
-    }
-  }
+    for (int k = 0; k < NC; k++) a[k] += __ldcg(part + (size_t)b * NC + k);
   block_sums<NT, NC>(a, shk);
   if (threadIdx.x == 0) {
     double *red = e.red;
