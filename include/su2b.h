@@ -56,7 +56,8 @@ enum { SU2B_GROUP_SU2 = 0, SU2B_GROUP_U1 = 1 };
  * SU2B_PREC_MIXED: SU(2) links, momenta and forces stored and computed in FP32; every
  *   global reduction (plaquette, action, kinetic energy, Delta H), the accept/reject and
  *   link reunitarisation in FP64.  For U(1) the links stay FP64 and MIXED selects FP32
- *   inner iterations with FP64 reliable updates in the CG. */
+ *   inner iterations with FP64 reliable updates in the CG where the lattice is not solved on
+ *   tiles (three and four dimensions, and two beyond about 150,000 sites). */
 enum { SU2B_PREC_FP64 = 0, SU2B_PREC_MIXED = 1 };
 
 /* integrator ids as the reference enum (integrator.hh:15) */
@@ -194,7 +195,8 @@ typedef struct {
   double tol;     /* residual norm bound */
   int tol_mode;   /* SU2B_TOL_ABS (the reference, CG.hpp:50) or SU2B_TOL_REL (tol*|b|) */
   int max_iter;
-  double delta;   /* mixed CG: reliable-update threshold (0 = default 0.1) */
+  double delta;   /* mixed CG: reliable-update threshold (0 = default 0.1); two-dimensional
+                     lattices up to about 150,000 sites are solved in FP64 throughout */
 } su2b_solve_params;
 typedef struct {
   long iterations;
@@ -372,7 +374,8 @@ SU2B_API int su2b_force_vjp(su2b_ctx *ctx, const double *mu_host, double *out_ho
  * the plaquette energy of gradient_flow (flat-gradient_flow.hh:151); *objective receives O
  * and grad_host (NULL: objective only) its derivative with respect to the starting links,
  * by the adjoint of the RK3 steps with checkpoints every checkpoint_every steps
- * (0 = sqrt(n_steps)).  The links are not modified. */
+ * (0: every stage kept, without recomputation, where 8 GB and a quarter of the free device
+ * memory hold them, else sqrt(n_steps)).  The links are not modified. */
 SU2B_API int su2b_flow_adjoint(su2b_ctx *ctx, double eps, int n_steps, int checkpoint_every,
                                double *objective, double *grad_host);
 
