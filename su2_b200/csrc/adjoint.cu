@@ -52,16 +52,20 @@ template <class T> __device__ __forceinline__ V3<T> operator-(const V3<T> &a, co
 template <class T> __device__ __forceinline__ V3<T> cross(const V3<T> &a, const V3<T> &b) {
   return V3<T>{fm(a.y, b.z, -a.z * b.y), fm(a.z, b.x, -a.x * b.z), fm(a.x, b.y, -a.y * b.x)};
 }
-// The rotation v -> d^+ v d / |d|^2 of an almost unit d = (d0, e): v + d0 w + e x w with
-// w = f x v, f = 2 e / |d|^2; 2 / n = 4 - 2 n up to (1 - n)^2, below rounding for links that are
-// unitary to their storage precision.
+// The rotation v -> d^+ v d / |d|^2 of d = (d0, e): v + d0 w + e x w with w = f x v,
+// f = 2 e / |d|^2.  For links that are unitary to their storage precision 2 / n = 4 - 2 n up to
+// (1 - n)^2, below rounding where the first form is taken; a field uploaded unnormalised takes
+// the quotient (a zero link: none, the plaquettes that it is in are zero).
 template <class T> struct Rot {
   T d0;
   V3<T> e, f;
 };
 template <class T> __device__ __forceinline__ Rot<T> rot_of(const Su2<T> &d) {
+  constexpr bool F64 = sizeof(T) == 8;
   const T n = fm(d.ar, d.ar, fm(d.ai, d.ai, fm(d.br, d.br, d.bi * d.bi)));
-  const T w = fm(T(-2), n, T(4));
+  T w = fm(T(-2), n, T(4));
+  if (!(fabs(n - T(1)) < (F64 ? T(0x1p-27) : T(0x1p-12))))
+    w = n > (F64 ? T(1e-300) : T(1e-37)) ? T(2) / n : T(0);
   return Rot<T>{d.ar, V3<T>{d.bi, d.br, d.ai}, V3<T>{w * d.bi, w * d.br, w * d.ai}};
 }
 // d^+ v d (inverse: d v d^+) over |d|^2

@@ -105,6 +105,45 @@ def test_force_vjp_geometries(gpu, orc, dims, nd):
         assert fd == pytest.approx(float(v["fp64"] @ w.ravel()), abs=1e-6 * scale)
 
 
+@pytest.mark.parametrize("dims,nd", [((6, 1, 1, 4), 2), ((4, 6, 1, 4), 3), ((4, 2, 4, 6), 4)])
+def test_force_vjp_of_links_off_the_unit_sphere(gpu, orc, dims, nd):
+    """An upload neither normalises nor checks: links of norm 0.7 to 1.3, some within 1e-3 and
+    1e-6 of one, and a zero link.  Central differences along seeded directions as for unit links
+    (their terms grow by 1.3^4 at most), FP32 within 1e-5 of FP64."""
+    U = orc.hotstart(0, dims, nd, 10, 1.0, 654321)
+    n = U.size // 4
+    rng = np.random.default_rng(n)
+    r = rng.uniform(0.7, 1.3, n)
+    r[::5] = 1 + 1e-3 * rng.normal(size=r[::5].size)
+    r[1::5] = 1 + 1e-6 * rng.normal(size=r[1::5].size)
+    r[n // 2] = 0.0
+    U = (U.reshape(n, 4) * r[:, None]).ravel()
+    mu = rng.normal(size=3 * n)
+    v = {}
+    for prec in ("fp64", "mixed"):
+        with gpu.gaugeconfig(*dims, nd, 2.0, precision=prec) as c:
+            c.upload(U)
+            v[prec] = c.force_vjp(mu)
+    assert np.isfinite(v["mixed"]).all()
+    assert rel(v["mixed"], v["fp64"]) < 1e-5
+    # a global factor of the field is a factor s^4 of a force whose terms are plaquettes
+    with gpu.gaugeconfig(*dims, nd, 2.0) as c:
+        c.upload(1.25 * U)
+        assert rel(c.force_vjp(mu), 1.25 ** 4 * v["fp64"]) < 1e-13
+
+    from su2_b200.autograd import _exp_links
+
+    def phi(w):
+        return float(mu @ orc.gauge_derivative(0, dims, nd, 2.0, _exp_links(U, w), 1.0, 1.0))
+
+    scale = np.linalg.norm(v["fp64"]) * np.sqrt(3)
+    for _ in range(6):
+        w = rng.normal(size=(n, 3))
+        h = 1e-5
+        fd = (phi(h * w) - phi(-h * w)) / (2 * h)
+        assert fd == pytest.approx(float(v["fp64"] @ w.ravel()), abs=1e-6 * scale)
+
+
 @pytest.mark.parametrize("every", [0, 1, 3])
 def test_flow_adjoint_finite_differences(gpu, orc, every):
     dims, nd = (4, 4, 4, 4), 4
