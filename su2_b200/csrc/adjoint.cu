@@ -331,12 +331,10 @@ int arena(su2b_ctx *ctx, size_t bytes, Scratch *sc) {
       ctx->arena = nullptr;
       ctx->arena_bytes = 0;
     }
-    const cudaError_t e = cudaMalloc(&ctx->arena, bytes);
-    if (e != cudaSuccess) {
-      ctx->arena = nullptr;
+    const cudaError_t e = su2b_malloc(&ctx->arena, ctx->alloc_size(bytes));
+    if (e != cudaSuccess)
       return su2b_fail(ctx, SU2B_ERR_NOMEM, "flow adjoint scratch (%zu bytes): %s", bytes,
                        cudaGetErrorString(e));
-    }
     ctx->arena_bytes = bytes;
   }
   sc->base = (char *)ctx->arena;

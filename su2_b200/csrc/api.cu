@@ -58,14 +58,31 @@ static int enter(su2b_ctx *ctx) {
 
 // ------------------------------------------------------------------------------------
 // context
-template <class P> static int dalloc(su2b_ctx *ctx, P **p, size_t bytes) {
-  if (bytes == 0) bytes = 16;
-  cudaError_t e = cudaMalloc((void **)p, bytes);
+cudaError_t su2b_malloc(void **p, size_t bytes) {
+  const cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
     *p = nullptr;
-    return su2b_fail(ctx, SU2B_ERR_NOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
+    cudaGetLastError();
   }
-  ctx->allocs.push_back((void *)*p);
+  return e;
+}
+int su2b_dalloc(su2b_ctx *ctx, void **p, size_t bytes) {
+  if (bytes == 0) bytes = 16;
+  const cudaError_t e = su2b_malloc(p, ctx->alloc_size(bytes));
+  if (e != cudaSuccess)
+    return su2b_fail(ctx, SU2B_ERR_NOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
+  ctx->allocs.push_back(*p);
+  return SU2B_OK;
+}
+template <class P> static int dalloc(su2b_ctx *ctx, P **p, size_t bytes) {
+  return su2b_dalloc(ctx, (void **)p, bytes);
+}
+extern "C" int su2b_test_set(su2b_ctx *ctx, int what, long value) {
+  if (!ctx) return SU2B_ERR_INVALID;
+  if (what == SU2B_TEST_FAIL_ALLOCS)
+    ctx->fail_allocs = (int)value;
+  else
+    return SU2B_ERR_INVALID;
   return SU2B_OK;
 }
 

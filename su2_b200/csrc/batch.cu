@@ -386,7 +386,7 @@ extern "C" int su2b_batch_create(int n_chains, const su2b_chain_desc *chains, in
     return fin(SU2B_ERR_CUDA);
   const size_t lb = b->link64 ? 32 : 16, ab = b->link64 ? 8 : 4;
   auto dal = [&](void **p, size_t bytes) -> bool {
-    if (cudaMalloc(p, bytes) != cudaSuccess) return false;
+    if (su2b_malloc(p, bytes) != cudaSuccess) return false;
     b->allocs.push_back(*p);
     return true;
   };

@@ -429,7 +429,7 @@ extern "C" int su2b_hmc_trajectory(su2b_ctx *ctx, const su2b_hmc_params *prm,
 
   if (prm->revtest) {  // md_update.hh:62-74
     if (!ctx->U_rev) {
-      SU2B_CK(cudaMalloc(&ctx->U_rev, ctx->link_bytes() * ctx->NL));
+      SU2B_CK(su2b_malloc(&ctx->U_rev, ctx->link_bytes() * ctx->NL));
       ctx->allocs.push_back(ctx->U_rev);
     }
     SU2B_CK(cudaMemcpyAsync(ctx->U_rev, ctx->U, ctx->link_bytes() * ctx->NL,

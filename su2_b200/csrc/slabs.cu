@@ -197,7 +197,7 @@ uint4 *piece_at(su2b_slabs *h, int r, int k, int mu, int p, int ts) {
 
 int upload_table(su2b_slabs *h, const std::vector<Piece> &v, Piece **dev) {
   void *p = nullptr;
-  SLAB_CUDA(cudaMalloc(&p, sizeof(Piece) * v.size()));
+  SLAB_CUDA(su2b_malloc(&p, sizeof(Piece) * v.size()));
   h->allocs.push_back(p);
   SLAB_CUDA(cudaMemcpy(p, v.data(), sizeof(Piece) * v.size(), cudaMemcpyHostToDevice));
   *dev = (Piece *)p;
@@ -225,7 +225,7 @@ int build_local_tables(su2b_slabs *h) {
   std::vector<double *> reds;
   for (su2b_ctx *c : h->sl) reds.push_back(c->red);
   void *p = nullptr;
-  SLAB_CUDA(cudaMalloc(&p, sizeof(double *) * reds.size()));
+  SLAB_CUDA(su2b_malloc(&p, sizeof(double *) * reds.size()));
   h->allocs.push_back(p);
   SLAB_CUDA(cudaMemcpy(p, reds.data(), sizeof(double *) * reds.size(), cudaMemcpyHostToDevice));
   h->reds = (double **)p;
@@ -659,14 +659,14 @@ extern "C" int su2b_slabs_connect(su2b_slabs *h, const void *id, int nranks, int
   h->overlap = true;
   const size_t bytes = (size_t)4 * h->nd * h->piece_n * 16;  // two faces
   void *a = nullptr, *b = nullptr;
-  SLAB_CUDA(cudaMalloc(&a, bytes));
+  SLAB_CUDA(su2b_malloc(&a, bytes));
   h->allocs.push_back(a);
-  SLAB_CUDA(cudaMalloc(&b, bytes));
+  SLAB_CUDA(su2b_malloc(&b, bytes));
   h->allocs.push_back(b);
   h->sendbuf = (uint4 *)a;
   h->recvbuf = (uint4 *)b;
   void *t = nullptr;
-  SLAB_CUDA(cudaMalloc(&t, sizeof(double) * FORCE_VARIANTS));
+  SLAB_CUDA(su2b_malloc(&t, sizeof(double) * FORCE_VARIANTS));
   h->allocs.push_back(t);
   h->tune_dev = (double *)t;
   return build_nccl_tables(h);

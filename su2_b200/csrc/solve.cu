@@ -22,16 +22,6 @@ namespace {
 
 constexpr int CHUNK = 16;
 
-int dalloc2(su2b_ctx *ctx, void **p, size_t bytes) {
-  cudaError_t e = cudaMalloc(p, bytes);
-  if (e != cudaSuccess) {
-    *p = nullptr;
-    return su2b_fail(ctx, SU2B_ERR_NOMEM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
-  }
-  ctx->allocs.push_back(*p);
-  return SU2B_OK;
-}
-
 int put_spinor(su2b_ctx *ctx, const double *host, double2 *dev) {
   SU2B_CK(cudaMemcpyAsync(ctx->stage, host, 2 * ctx->V * sizeof(double), cudaMemcpyHostToDevice,
                           ctx->stream));
@@ -110,7 +100,7 @@ int cg_tile_setup(su2b_ctx *ctx) {
   const CgTilePlan plan = cg_tile_plan(ctx->g);
   if (!plan.K) return SU2B_OK;
   void *work = nullptr;
-  if (cudaMalloc(&work, cg_tile_bytes(ctx->g)) == cudaSuccess &&
+  if (su2b_malloc(&work, ctx->alloc_size(cg_tile_bytes(ctx->g))) == cudaSuccess &&
       cudaMallocHost((void **)&ctx->h_cg, sizeof(CgTileResult)) == cudaSuccess) {
     ctx->allocs.push_back(work);
     SU2B_CK(cudaMemsetAsync(work, 0, cg_tile_bytes(ctx->g), ctx->stream));
@@ -477,17 +467,17 @@ int su2b_fermion_setup(su2b_ctx *ctx, bool need32) {
     return su2b_fail(ctx, SU2B_ERR_UNSUPPORTED,
                      "staggered fermions are not supported for SU(2) (staggered.hpp:343-350)");
   if (!ctx->ph) {
-    SU2B_CKS(dalloc2(ctx, (void **)&ctx->ph, ctx->NL * sizeof(double2)));
-    SU2B_CKS(dalloc2(ctx, (void **)&ctx->fderiv, ctx->NL * sizeof(double)));
-    SU2B_CKS(dalloc2(ctx, (void **)&ctx->st, sizeof(SolverState)));
+    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->ph, ctx->NL * sizeof(double2)));
+    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->fderiv, ctx->NL * sizeof(double)));
+    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->st, sizeof(SolverState)));
     for (int k = 0; k < SV_N; k++)
-      SU2B_CKS(dalloc2(ctx, (void **)&ctx->sv[k], ctx->V * sizeof(double2)));
+      SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->sv[k], ctx->V * sizeof(double2)));
     ctx->phases_valid = false;
   }
   if (need32 && !ctx->ph32) {
-    SU2B_CKS(dalloc2(ctx, (void **)&ctx->ph32, ctx->NL * sizeof(float2)));
+    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->ph32, ctx->NL * sizeof(float2)));
     for (int k = 0; k < SV32_N; k++)
-      SU2B_CKS(dalloc2(ctx, (void **)&ctx->sv32[k], ctx->V * sizeof(float2)));
+      SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->sv32[k], ctx->V * sizeof(float2)));
     ctx->phases32_valid = false;
   }
   return ensure_phases(ctx, need32);

@@ -97,6 +97,14 @@ struct su2b_ctx {
   std::vector<void *> allocs;
   std::string err;
 
+  // su2b_test_set: the next fail_allocs allocations ask for more than any device has
+  int fail_allocs = 0;
+  size_t alloc_size(size_t bytes) {
+    if (fail_allocs == 0) return bytes;
+    fail_allocs--;
+    return (size_t)1 << 62;
+  }
+
   size_t link_bytes() const { return group == 0 ? (link64 ? 32 : 16) : 8; }
   size_t adj_bytes() const { return (group == 0 ? 3 : 1) * (link64 ? 8 : 4); }
   double Nc() const { return group == 0 ? 2.0 : 1.0; }
@@ -118,6 +126,12 @@ std::vector<HmcFusedOp> su2b_fuse(const std::vector<HmcOp> &ops);
 
 // helpers shared by the api*.cu files
 int su2b_fail(su2b_ctx *ctx, int code, const char *fmt, ...);
+// device memory of the context; SU2B_ERR_NOMEM with a message if it is refused
+int su2b_dalloc(su2b_ctx *ctx, void **p, size_t bytes);
+// for the tests, not in su2b.h: failures made on the host
+enum { SU2B_TEST_FAIL_ALLOCS = 0 };
+extern "C" __attribute__((visibility("default"))) int su2b_test_set(su2b_ctx *ctx, int what,
+                                                                    long value);
 int su2b_adj_upload(su2b_ctx *ctx, const double *host, void *dev);
 int su2b_adj_download(su2b_ctx *ctx, const void *dev, double *host);
 // three plaquette / clover sums of U into out, device memory or the pinned h_red

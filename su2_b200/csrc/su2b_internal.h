@@ -5,6 +5,11 @@
 
 #include "su2b_common.cuh"
 
+// Device memory.  A refusal leaves no error behind in the CUDA runtime: the launchers end in
+// cudaGetLastError(), and the next launch of a caller that goes on without the memory would
+// report it.
+cudaError_t su2b_malloc(void **p, size_t bytes);
+
 namespace su2b {
 
 // ---- layout conversion (reference host AoS <-> even/odd SoA) ----

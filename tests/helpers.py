@@ -22,3 +22,11 @@ def rel(a, b):
 
 def group_name(g):
     return "su2" if g == 0 else "u1"
+
+
+def fail_allocations(lattice, n):
+    """The next n device allocations of the lattice's context ask for more than a device has."""
+    import ctypes as C
+    f = lattice.lib.su2b_test_set
+    f.argtypes, f.restype = [C.c_void_p, C.c_int, C.c_long], C.c_int
+    assert f(lattice.ctx, 0, n) == 0

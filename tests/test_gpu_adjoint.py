@@ -9,7 +9,7 @@ gradient within 1e-3 of the FP64 one.
 import numpy as np
 import pytest
 
-from helpers import rel
+from helpers import fail_allocations, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -196,6 +196,27 @@ def test_flow_adjoint_tape_limit(gpu, orc):
         O, g = c.flow_objective(1e-4, n)
         Oc, gc = c.flow_objective(1e-4, n, checkpoint_every=round(n ** 0.5))
         assert O == Oc and np.array_equal(g, gc)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_flow_adjoint_without_memory_for_the_tape(gpu, orc, precision):
+    """A tape whose allocation is refused: the gradient of the checkpoints, bit for bit, in the
+    same call.  Refused both: an error, and the next call is none the worse."""
+    dims, n = (4, 6, 4, 8), 9
+    U = orc.hotstart(0, dims, 4, 14, 1.0, 4321)
+    with gpu.gaugeconfig(*dims, 4, 2.4, precision=precision) as c:
+        c.upload(U)
+        fail_allocations(c, 1)
+        O, g = c.flow_objective(0.02, n)
+        Oc, gc = c.flow_objective(0.02, n, checkpoint_every=3)
+        assert O == Oc and np.array_equal(g, gc)
+    with gpu.gaugeconfig(*dims, 4, 2.4, precision=precision) as c:
+        c.upload(U)
+        fail_allocations(c, 2)
+        with pytest.raises(gpu.Su2bError, match="scratch"):
+            c.flow_objective(0.02, n)
+        assert np.isfinite(c.gauge_energy())
+        assert c.flow_objective(0.02, n)[0] == pytest.approx(Oc, rel=1e-5)
 
 
 def test_flow_objective_matches_flow_records(gpu, orc):
