@@ -375,7 +375,10 @@ SU2B_API int su2b_force_vjp(su2b_ctx *ctx, const double *mu_host, double *out_ho
  * and grad_host (NULL: objective only) its derivative with respect to the starting links,
  * by the adjoint of the RK3 steps with checkpoints every checkpoint_every steps
  * (0: every stage kept, without recomputation, where 8 GB and a quarter of the free device
- * memory hold them, else sqrt(n_steps)).  The links are not modified. */
+ * memory hold them, else sqrt(n_steps)).  The links are not modified.  The scratch memory stays
+ * with the context for the next call, 8 GB at most over all contexts of the process where it
+ * holds stages; a call with checkpoint_every > 0 gives up what it does not need, and an
+ * allocation of this library that finds no memory takes the scratch of idle contexts. */
 SU2B_API int su2b_flow_adjoint(su2b_ctx *ctx, double eps, int n_steps, int checkpoint_every,
                                double *objective, double *grad_host);
 

@@ -309,10 +309,10 @@ cudaError_t exp_adjoint(const Geom &g, const T *Z, double b, T *lam, T *mu, cuda
   return cudaGetLastError();
 }
 
-// device scratch of one adjoint computation, freed on return
-// Scratch carved from the context's arena.  The arena stays allocated between calls (one
-// gradient at 24^4 needs about 1.4 GB; allocating and freeing that per call costs
-// milliseconds, and cudaFree synchronises the device) and only grows.
+// Scratch of one adjoint computation, carved from the context's arena.  The arena stays
+// allocated between calls (allocating and freeing the 2.2 GB of a gradient of 20 steps at 24^4
+// takes 2.4 ms), until the context ends, a call asks for checkpoints and needs less than half of
+// it, or another allocation of the process finds no memory.
 struct Scratch {
   char *base = nullptr;
   size_t off = 0, cap = 0;
@@ -324,24 +324,27 @@ struct Scratch {
     return q;
   }
 };
-int arena(su2b_ctx *ctx, size_t bytes, Scratch *sc) {
-  if (ctx->arena_bytes < bytes) {
-    if (ctx->arena) {
-      cudaFree(ctx->arena);
-      ctx->arena = nullptr;
-      ctx->arena_bytes = 0;
-    }
-    const cudaError_t e = su2b_malloc(&ctx->arena, ctx->alloc_size(bytes));
+int arena(su2b_ctx *ctx, size_t bytes, Scratch *sc, bool shrink, size_t limit) {
+  if (ctx->arena_bytes < bytes || (shrink && ctx->arena_bytes / 2 > bytes)) {
+    const cudaError_t e = su2b_arena_reserve(ctx, bytes, limit);
     if (e != cudaSuccess)
       return su2b_fail(ctx, SU2B_ERR_NOMEM, "flow adjoint scratch (%zu bytes): %s", bytes,
                        cudaGetErrorString(e));
-    ctx->arena_bytes = bytes;
   }
   sc->base = (char *)ctx->arena;
   sc->off = 0;
   sc->cap = ctx->arena_bytes;
   return SU2B_OK;
 }
+// a call's claim on the arena, held until the device is done with it
+struct ArenaUse {
+  su2b_ctx *ctx;
+  explicit ArenaUse(su2b_ctx *c) : ctx(c) { su2b_arena_busy(ctx, true); }
+  ~ArenaUse() {
+    cudaStreamSynchronize(ctx->stream);
+    su2b_arena_busy(ctx, false);
+  }
+};
 
 // Maps the pages of a host buffer that is about to be written, while the device still works on
 // what goes there: the 8,000 pages of a fresh 32 MB array (a gradient at 24^4) otherwise fault
@@ -425,12 +428,18 @@ int get_gradient(su2b_ctx *ctx, const void *lam, double t, double *objective, do
   return SU2B_OK;
 }
 
-// Whether the arena may take that much for a tape: at most 8 GB and a quarter of what is free.
-bool tape_fits(const su2b_ctx *ctx, size_t bytes) {
-  if (bytes <= ctx->arena_bytes) return true;
-  size_t free = 0, total = 0;
-  if (bytes > ((size_t)8 << 30) || cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
-  return bytes - ctx->arena_bytes <= free / 4;
+// The arena for a tape: the arenas of all contexts hold at most 8 GB with it, and it takes at
+// most a quarter of what is free.
+bool tape_arena(su2b_ctx *ctx, size_t bytes, Scratch *sc) {
+  constexpr size_t LIMIT = (size_t)8 << 30;
+  if (bytes > ctx->arena_bytes) {
+    size_t free = 0, total = 0;
+    if (bytes > LIMIT || cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
+    if (bytes - ctx->arena_bytes > free / 4) return false;
+  }
+  if (arena(ctx, bytes, sc, false, LIMIT) == SU2B_OK) return true;
+  ctx->err.clear();
+  return false;
 }
 
 // the gradient with every stage's field W[3 st + f] and accumulator Z[3 st + f] kept
@@ -471,7 +480,6 @@ template <class T>
 int flow_adjoint_t(su2b_ctx *ctx, double eps, int n, int every, double *objective,
                    double *grad_host) {
   cudaStream_t s = ctx->stream;
-  const Geom &g = ctx->g;
   const size_t NL = ctx->NL, lb = ctx->link_bytes() * NL, ab = ctx->adj_bytes() * NL;
   const size_t lb_a = (lb + 255) & ~(size_t)255, ab_a = (ab + 255) & ~(size_t)255;
   Scratch sc;
@@ -479,12 +487,13 @@ int flow_adjoint_t(su2b_ctx *ctx, double eps, int n, int every, double *objectiv
   // caller asked for no checkpoints: the reverse pass then runs no force again.  20 steps at
   // 24^4, mixed precision: 7.35 ms and 2.2 GB against 9.85 ms and 0.3 GB.
   const size_t tape = (size_t)n * 3 * (lb_a + ab_a) + lb_a + 2 * ab_a;
-  if (grad_host && every <= 0 && tape_fits(ctx, tape) && arena(ctx, tape, &sc) == SU2B_OK)
+  const ArenaUse use(ctx);
+  if (grad_host && every <= 0 && tape_arena(ctx, tape, &sc))
     return flow_adjoint_tape<T>(ctx, eps, n, &sc, objective, grad_host);
-  ctx->err.clear();
-  if (every <= 0) every = std::max(1, (int)std::lround(std::sqrt((double)n)));
+  const bool asked = every > 0;
+  if (!asked) every = std::max(1, (int)std::lround(std::sqrt((double)n)));
   const int nseg = (n + every - 1) / every;
-  SU2B_CKS(arena(ctx, (nseg + every + 3) * lb_a + 5 * ab_a, &sc));
+  SU2B_CKS(arena(ctx, (nseg + every + 3) * lb_a + 5 * ab_a, &sc, asked, 0));
   std::vector<void *> ck(nseg), seg(every);
   for (int i = 0; i < nseg; i++) ck[i] = sc.get(lb);
   for (int i = 0; i < every; i++) seg[i] = sc.get(lb);

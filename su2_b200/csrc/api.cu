@@ -4,11 +4,13 @@
 // Host code only orders kernels on the context's stream; every lattice-sized loop runs on
 // the device.  Reductions are two-stage (per-block partials, then one block in a fixed
 // order), so results do not depend on timing.
+#include <algorithm>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <utility>
 #include <cstring>
+#include <mutex>
 #include <random>
 #include <string>
 #include <vector>
@@ -58,13 +60,64 @@ static int enter(su2b_ctx *ctx) {
 
 // ------------------------------------------------------------------------------------
 // context
-cudaError_t su2b_malloc(void **p, size_t bytes) {
+namespace {
+// The contexts that hold an arena, in any thread; guards their arena fields.
+std::mutex arenas_mutex;
+std::vector<su2b_ctx *> arenas;
+
+void drop_arena(su2b_ctx *ctx) {  // under the mutex
+  if (!ctx->arena) return;
+  cudaFree(ctx->arena);
+  ctx->arena = nullptr;
+  ctx->arena_bytes = 0;
+  arenas.erase(std::find(arenas.begin(), arenas.end(), ctx));
+}
+cudaError_t malloc_clean(void **p, size_t bytes) {
   const cudaError_t e = cudaMalloc(p, bytes);
   if (e != cudaSuccess) {
     *p = nullptr;
     cudaGetLastError();
   }
   return e;
+}
+// under the mutex: as malloc_clean, and once more without the idle arenas of the device
+cudaError_t malloc_or_trim(void **p, size_t bytes) {
+  cudaError_t e = malloc_clean(p, bytes);
+  int dev = 0;
+  if (e == cudaSuccess || cudaGetDevice(&dev) != cudaSuccess) return e;
+  bool freed = false;
+  for (su2b_ctx *c : std::vector<su2b_ctx *>(arenas))
+    if (!c->arena_busy && c->device == dev) {
+      drop_arena(c);
+      freed = true;
+    }
+  return freed ? malloc_clean(p, bytes) : e;
+}
+}  // namespace
+
+cudaError_t su2b_malloc(void **p, size_t bytes) {
+  if (malloc_clean(p, bytes) == cudaSuccess) return cudaSuccess;
+  std::lock_guard<std::mutex> lock(arenas_mutex);
+  return malloc_or_trim(p, bytes);
+}
+cudaError_t su2b_arena_reserve(su2b_ctx *ctx, size_t bytes, size_t limit) {
+  std::lock_guard<std::mutex> lock(arenas_mutex);
+  if (limit) {
+    size_t held = bytes;
+    for (su2b_ctx *c : arenas)
+      if (c != ctx && c->device == ctx->device) held += c->arena_bytes;
+    if (held > limit) return cudaErrorMemoryAllocation;
+  }
+  drop_arena(ctx);
+  const cudaError_t e = malloc_or_trim(&ctx->arena, ctx->alloc_size(bytes));
+  if (e != cudaSuccess) return e;
+  ctx->arena_bytes = bytes;
+  arenas.push_back(ctx);
+  return cudaSuccess;
+}
+void su2b_arena_busy(su2b_ctx *ctx, bool busy) {
+  std::lock_guard<std::mutex> lock(arenas_mutex);
+  ctx->arena_busy = busy;
 }
 int su2b_dalloc(su2b_ctx *ctx, void **p, size_t bytes) {
   if (bytes == 0) bytes = 16;
@@ -206,7 +259,10 @@ extern "C" int su2b_ctx_destroy(su2b_ctx *ctx) {
   for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
   for (auto &kv : ctx->graphs) cudaGraphExecDestroy(kv.second.exec);
   for (void *p : ctx->allocs) cudaFree(p);
-  if (ctx->arena) cudaFree(ctx->arena);
+  {
+    std::lock_guard<std::mutex> lock(arenas_mutex);
+    drop_arena(ctx);
+  }
   if (ctx->h_red) cudaFreeHost(ctx->h_red);
   if (ctx->h_traj) cudaFreeHost(ctx->h_traj);
   if (ctx->h_counts) cudaFreeHost(ctx->h_counts);

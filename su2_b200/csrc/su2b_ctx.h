@@ -27,9 +27,11 @@ struct su2b_ctx {
   // trajectory (the start configuration stays untouched in one of them until accept/reject)
   void *U = nullptr, *U_old = nullptr, *U2 = nullptr, *U_aux = nullptr, *U_rev = nullptr;
   void *P = nullptr, *Z = nullptr;
-  // scratch arena of the flow adjoint, kept between calls and grown on demand
+  // scratch arena of the flow adjoint, kept between calls and grown on demand; while no call
+  // uses it (arena_busy) it may be freed for another allocation of the process
   void *arena = nullptr;
   size_t arena_bytes = 0;
+  bool arena_busy = false;
   double *stage = nullptr;  // host-layout staging buffer on the device
   double *part = nullptr;   // NSLOT slots of 3*part_cap partial sums
   size_t part_cap = 0;
@@ -126,6 +128,10 @@ std::vector<HmcFusedOp> su2b_fuse(const std::vector<HmcOp> &ops);
 
 // helpers shared by the api*.cu files
 int su2b_fail(su2b_ctx *ctx, int code, const char *fmt, ...);
+// the context's arena with `bytes`, its contents lost; limit: refused where the arenas of all
+// contexts on the device would exceed it (0: no limit)
+cudaError_t su2b_arena_reserve(su2b_ctx *ctx, size_t bytes, size_t limit);
+void su2b_arena_busy(su2b_ctx *ctx, bool busy);
 // device memory of the context; SU2B_ERR_NOMEM with a message if it is refused
 int su2b_dalloc(su2b_ctx *ctx, void **p, size_t bytes);
 // for the tests, not in su2b.h: failures made on the host

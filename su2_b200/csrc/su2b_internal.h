@@ -5,9 +5,9 @@
 
 #include "su2b_common.cuh"
 
-// Device memory.  A refusal leaves no error behind in the CUDA runtime: the launchers end in
-// cudaGetLastError(), and the next launch of a caller that goes on without the memory would
-// report it.
+// Device memory; where it is short, the flow adjoint's idle arenas are given up for it.  A
+// refusal leaves no error behind in the CUDA runtime: the launchers end in cudaGetLastError(),
+// and the next launch of a caller that goes on without the memory would report it.
 cudaError_t su2b_malloc(void **p, size_t bytes);
 
 namespace su2b {

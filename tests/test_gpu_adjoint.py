@@ -219,6 +219,65 @@ def test_flow_adjoint_without_memory_for_the_tape(gpu, orc, precision):
         assert c.flow_objective(0.02, n)[0] == pytest.approx(Oc, rel=1e-5)
 
 
+def free_bytes():
+    import torch
+    return torch.cuda.mem_get_info(0)[0]
+
+
+def test_tape_memory_is_given_back(gpu, orc):
+    """The stages of 20 steps at 16^4 FP64 are 0.88 GB: they stay for the next gradient, and go
+    when a call asks for checkpoints, when another context finds no memory and when the context
+    ends; the gradients after that are those before.  The device allocates in pieces of 2 MB."""
+    dims, n, piece = (16, 16, 16, 16), 20, 4 << 20
+    tape = 3 * n * 4 * 16 ** 4 * (32 + 24)
+    U = orc.hotstart(0, dims, 4, 15, 1.0, 4321)
+    with gpu.gaugeconfig(*dims, 4, 2.4) as c, gpu.gaugeconfig(4, 1, 1, 4, 2, 2.4) as other:
+        c.upload(U)
+        c.flow_objective(0.01, n, checkpoint_every=5)
+        before = free_bytes()
+        want = c.flow_objective(0.01, n)
+        assert before - free_bytes() > tape // 2
+        held = free_bytes()
+        for k in range(2):
+            got = c.flow_objective(0.01, n)
+            assert got[0] == want[0] and np.array_equal(got[1], want[1])
+        assert free_bytes() == held
+        c.flow_objective(0.01, n, checkpoint_every=5)
+        assert abs(free_bytes() - before) <= piece
+        got = c.flow_objective(0.01, n)
+        assert got[0] == want[0] and np.array_equal(got[1], want[1])
+        fail_allocations(other, 1)
+        with pytest.raises(gpu.Su2bError):
+            other.flow_objective(0.01, 2, checkpoint_every=1)
+        assert free_bytes() >= before - piece
+        got = c.flow_objective(0.01, n)
+        assert got[0] == want[0] and np.array_equal(got[1], want[1])
+        assert before - free_bytes() > tape // 2
+        c.close()
+        assert free_bytes() > before
+
+
+def test_tapes_of_all_contexts_share_one_limit(gpu, orc):
+    """Two contexts whose stages take 5 GB each: the second one's gradient is the checkpoints',
+    bit for bit, until the first context ends."""
+    dims, n = (16, 16, 16, 16), 114
+    U = orc.hotstart(0, dims, 4, 16, 1.0, 4321)
+    with gpu.gaugeconfig(*dims, 4, 2.4) as b:
+        b.upload(U)
+        with gpu.gaugeconfig(*dims, 4, 2.4) as a:
+            a.upload(U)
+            a.flow_objective(1e-3, n)
+            before = free_bytes()
+            O, g = b.flow_objective(1e-3, n)
+            assert before - free_bytes() < 1 << 30
+            Oc, gc = b.flow_objective(1e-3, n, checkpoint_every=round(n ** 0.5))
+            assert O == Oc and np.array_equal(g, gc)
+        before = free_bytes()
+        O, g = b.flow_objective(1e-3, n)
+        assert before - free_bytes() > 4 << 30
+        assert O == pytest.approx(Oc, rel=1e-11)
+
+
 def test_flow_objective_matches_flow_records(gpu, orc):
     dims, nd = (4, 4, 4, 4), 4
     U = orc.hotstart(0, dims, nd, 11, 1.0, 654321)
