@@ -101,11 +101,10 @@ template <class T, int ND> struct Sent {
 // reverse of a link update in the second, against 109 us and 27 us for that update by itself.
 template <class T, int ND, int NT>
 __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
-  k_force_vjp(Geom g, const LinkT<T> *__restrict__ U, const T *__restrict__ mu,
-              Sent<T, ND> sent) {
-  pdl_start<(sizeof(T) == 4 ? 5 : 3)>();
+  k_force_vjp(Geom g, const LinkT<T> *U, const T *mu, Sent<T, ND> sent) {
   const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
-  const int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  pdl_start<T, (sizeof(T) == 4 ? 5 : 3)>(cb);
   if (cb >= g.Vh) return;
   const Site s = site_from_eo(g, p, cb);
   const size_t V = (size_t)g.V, NL = V * ND, self = (size_t)p * g.Vh + cb;
@@ -229,18 +228,18 @@ __global__ void k_exp_adjoint(size_t NL, const T *__restrict__ Z, T b, T *__rest
 // Pass 2 of the VJP, then (EXP) the reverse of the link update before the stage in the same
 // pass over the cotangent: lam is read and written once instead of twice
 template <class T, int ND, int NT, bool EXP>
-__global__ void __launch_bounds__(NT)
+__global__ void __launch_bounds__(NT, 7)
   k_force_vjp_gather(Geom g, Sent<T, ND> sent, T *__restrict__ lam, T coef,
-                     int acc_lam, const T *__restrict__ Z, T b, T *__restrict__ mu, int acc_mu) {
-  pdl_start<5>();
+                     int acc_lam, const T *Z, T b, T *__restrict__ mu, int acc_mu) {
   const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
-  const int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  pdl_start<T, 7>(cb);
   if (cb >= g.Vh) return;
   const Site s = site_from_eo(g, p, cb);
   const size_t V = (size_t)g.V, NL = V * ND, self = (size_t)p * g.Vh + cb;
   T S[3 * ND];
 #pragma unroll
-  for (int k = 0; k < 3 * ND; k++) S[k] = __ldg(sent.at(3 * ND * (ND - 1) + k, V) + self);
+  for (int k = 0; k < 3 * ND; k++) S[k] = sent.at(3 * ND * (ND - 1) + k, V)[self];
 #pragma unroll
   for (int d = 0; d < ND; d++) {
     const size_t z = eo_of(g, s.lex + bwd(g, s, d), q);
@@ -249,7 +248,7 @@ __global__ void __launch_bounds__(NT)
       if (m == d) continue;
       const int k = 3 * ((ND - 1) * d + (m < d ? m : m - 1));
 #pragma unroll
-      for (int i = 0; i < 3; i++) S[3 * m + i] += __ldg(sent.at(k + i, V) + z);
+      for (int i = 0; i < 3; i++) S[3 * m + i] += sent.at(k + i, V)[z];
     }
   }
   const T c2 = T(2) * coef;

@@ -66,13 +66,13 @@ __global__ void __launch_bounds__(NT, MINB)
   // the tables do not change in a trajectory: read while the previous launch ends
   const int c = __ldg(&of[tile]);
   load_chain<NT>(d, ch + c);
-  const int cb = (tile - d.tile0) * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  int cb = (tile - d.tile0) * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
   const int S = cur[c];
   const LinkT<T> *U = bufs.at((S + rel_in) % 3) + d.off_link;
   LinkT<T> *Uo = rel_out >= 0 ? bufs.at((S + rel_out) % 3) + d.off_link : nullptr;
   T *P = Pall + d.off_adj;
   const T f = (T)(d.beta / 2.0);
-  pdl_start<MINB>();
+  pdl_start<T, MINB>(cb);
   double k2 = 0.;
   if (cb < d.g.Vh) {
     if (d.g.nd == 4)
@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(NT)
   const int w = threadIdx.x >> 5, p = w & 1, tile = blockIdx.x;
   const int c = __ldg(&of[tile]);
   load_chain<NT>(d, ch + c);
-  pdl_wait();
-  const int cb = (tile - d.tile0) * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  int cb = (tile - d.tile0) * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  pdl_wait<T>(cb);
   const LinkT<T> *U = bufs.at((cur[c] + rel) % 3) + d.off_link;
   double full = 0., spat = 0., wsum = 0.;
   if (cb < d.g.Vh) {
@@ -231,8 +231,7 @@ __device__ __forceinline__ void accept_chain(const ChainDev &d, const double *r,
   if (t.accepted) *cur_c = (*cur_c + rel_final) % 3;
 }
 __global__ void __launch_bounds__(256)
-  k_batch_reduce_accept(const ChainDev *__restrict__ ch, const double *__restrict__ ps,
-                        const double *__restrict__ pk, const double *__restrict__ pe,
+  k_batch_reduce_accept(const ChainDev *__restrict__ ch, const double *ps, const double *pk, const double *pe,
                         double *red, const uint32_t *__restrict__ traj, int rel_final, int *cur,
                         TrajDev *out, int cached, int *h_cur, TrajDev *h_out, double *h_red) {
   __shared__ double shk[7 * 8];

@@ -121,8 +121,8 @@ template <class T, int NT> constexpr int plaq_min_blocks() {
 
 template <class T, int ND, int NT>
 __device__ __forceinline__ void plaq_bands(const Geom &g, const LinkT<T> *__restrict__ U,
-                                           double xi, double (&v)[3]) {
-  for (int c = blockIdx.x * (NT / 32) + (threadIdx.x >> 5); 32 * (c >> 1) < g.ncb;
+                                           double xi, int first, double (&v)[3]) {
+  for (int c = first; 32 * (c >> 1) < g.ncb;
        c += gridDim.x * (NT / 32)) {  // band c/2 of 32 sites, parity c%2
     const int b = 32 * (c >> 1) + (threadIdx.x & 31);
     if (b < g.ncb) plaq_site<T, ND>(g, U, c & 1, g.cb0 + b, xi, v[0], v[1], v[2]);
@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
   k_plaq_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part, Finish fin) {
   __shared__ double shk[3 * (NT / 32)];
   double v[3] = {0., 0., 0.};
-  plaq_bands<T, ND, NT>(g, U, xi, v);
+  plaq_bands<T, ND, NT>(g, U, xi, blockIdx.x * (NT / 32) + (threadIdx.x >> 5), v);
   finish_sums<NT, 3>(v, part, fin, shk);
 }
 
@@ -241,16 +241,16 @@ __global__ void __launch_bounds__(NT)
 // fused staple/force/momentum(/link update) kernel: one thread per site, force_site body
 template <class T, int ND, int NT, int MINB, bool ANISO>
 __global__ void __launch_bounds__(NT, MINB)
-  k_force_su2(Geom g, const LinkT<T> *__restrict__ U, T *__restrict__ P,
-              const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
+  k_force_su2(Geom g, const LinkT<T> *U, T *__restrict__ P,
+              const T *extra, T f, T scale_, int mode, T wt, T ws,
               double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   __shared__ double sh[NT / 32];
-  pdl_start<MINB>();
   // warps alternate between the parities of one band of NT/2 sites per parity, so the
   // +-z / +-y neighbours of a site are mostly the own links of another warp of the block
   const int w = threadIdx.x >> 5;
   const int p = w & 1;
-  const int cb = g.cb0 + blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  int cb = g.cb0 + blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  pdl_start<T, MINB>(cb);
   double k2 = 0.;
   if (cb < g.cb0 + g.ncb)
     k2 = force_site_impl<T, ND, ANISO>(g, U, P, extra, f, scale_, mode, wt, ws, Uout, dt_upd, p,
@@ -267,14 +267,14 @@ __global__ void __launch_bounds__(NT, MINB)
 // sites; for lattices too small to fill the GPU one thread per site
 template <class T, int ND, int MINB>
 __global__ void __launch_bounds__(32 * ND, MINB)
-  k_force_su2_link(Geom g, const LinkT<T> *__restrict__ U, T *__restrict__ P,
-                   const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
+  k_force_su2_link(Geom g, const LinkT<T> *U, T *__restrict__ P,
+                   const T *extra, T f, T scale_, int mode, T wt, T ws,
                    double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   constexpr int NT = 32 * ND;
   __shared__ double sh[NT / 32];
-  pdl_start<MINB>();
   const int mu = threadIdx.x >> 5, p = blockIdx.x & 1;
-  const int cb = g.cb0 + (blockIdx.x >> 1) * 32 + (threadIdx.x & 31);
+  int cb = g.cb0 + (blockIdx.x >> 1) * 32 + (threadIdx.x & 31);
+  pdl_start<T, MINB>(cb);
   double k2 = 0.;
   // the direction is a compile-time constant in each warp's body (static site indexing)
 #define SU2B_LINK_BODY(M)                                                                     \
@@ -303,8 +303,8 @@ __global__ void __launch_bounds__(32 * ND, MINB)
 // (one thread per link 55.3), FP32 44.4 us (48.4); 12^4, where the SMs are full: 99 us (75).
 template <class T>
 __global__ void __launch_bounds__(384, 1)
-  k_force_su2_planes(Geom g, const LinkT<T> *__restrict__ U, T *__restrict__ P,
-                     const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
+  k_force_su2_planes(Geom g, const LinkT<T> *U, T *__restrict__ P,
+                     const T *extra, T f, T scale_, int mode, T wt, T ws,
                      double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   __shared__ double sh[12];
   __shared__ LinkT<T> xs[2][4][32];
@@ -312,9 +312,9 @@ __global__ void __launch_bounds__(384, 1)
   const int p = blockIdx.x & 1, cb = g.cb0 + (blockIdx.x >> 1) * 32 + lane;
   const bool on = cb < g.cb0 + g.ncb;  // lanes past the end compute the last site, write nothing
   const int c = on ? cb : g.cb0 + g.ncb - 1;
-  const Site s = site_from_eo(g, p, c);
-  const size_t V = (size_t)g.V, l = mu * V + (size_t)p * g.Vh + c;
-  pdl_start<1>();
+  Site s = site_from_eo(g, p, c);
+  pdl_start<T, 1>(s.lex);
+  const size_t V = (size_t)g.V, l = mu * V + eo_of(g, s.lex, p);
   if (j == 0 && (mode & FM_HAS_IN)) prefetch_momenta(P, l, 4 * V);
   Su2<T> K;
   switch (w) {  // direction and plane are compile-time constants in each warp's body
@@ -567,13 +567,14 @@ __global__ void k_accept(const double *__restrict__ red, const TrajParams *__res
 // before the end plaquettes overwrite red[5..7].
 template <class T, int ND, int NT>
 __global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
-  k_plaq_accept_su2(Geom g, const LinkT<T> *__restrict__ U, double xi, double *part,
+  k_plaq_accept_su2(Geom g, const LinkT<T> *U, double xi, double *part,
                     TrajTail e) {
   constexpr int NC = 8;  // start |P|^2 and three plaquette sums, end |P|^2, three plaquette sums
   __shared__ double shk[NC * (NT / 32)];
-  pdl_wait();
+  int band = blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
+  pdl_wait<T>(band);
   double v[3] = {0., 0., 0.}, a[NC];
-  plaq_bands<T, ND, NT>(g, U, xi, v);
+  plaq_bands<T, ND, NT>(g, U, xi, band, v);
 #pragma unroll
   for (int k = 0; k < NC; k++) a[k] = k < 5 ? 0. : v[k - 5];
   // every block also takes its share of the earlier launches' partials (16,384 of the force
@@ -711,14 +712,14 @@ cudaError_t reduce_final(const double *part, int nblocks, int ncomp, double *out
 // sites of one parity, warps (4k+2, 4k+3) of the 32 sites of the other parity beside them
 template <class T, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
-  k_force_su2_split(Geom g, const LinkT<T> *__restrict__ U, T *__restrict__ P,
-                    const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
+  k_force_su2_split(Geom g, const LinkT<T> *U, T *__restrict__ P,
+                    const T *extra, T f, T scale_, int mode, T wt, T ws,
                     double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   __shared__ double sh[NT / 32];
-  pdl_start<MINB>();
   const int w = threadIdx.x >> 5;
   const int half = w & 1, p = (w >> 1) & 1;
-  const int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
+  int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
+  pdl_start<T, MINB>(cb);
   double k2 = 0.;
   if (cb < g.cb0 + g.ncb)
     k2 = half == 0 ? force_half_impl<T, 0, false>(g, U, P, extra, f, scale_, mode, wt, ws, Uout,
@@ -736,16 +737,16 @@ __global__ void __launch_bounds__(NT, MINB)
 // Every thread reaches its pair barrier: threads past the lattice end run on a clamped site.
 template <class T, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB)
-  k_force_su2_xsplit(Geom g, const LinkT<T> *__restrict__ U, T *__restrict__ P,
-                     const T *__restrict__ extra, T f, T scale_, int mode, T wt, T ws,
+  k_force_su2_xsplit(Geom g, const LinkT<T> *U, T *__restrict__ P,
+                     const T *extra, T f, T scale_, int mode, T wt, T ws,
                      double *kin_part, LinkT<T> *__restrict__ Uout, T dt_upd) {
   static_assert(NT == 128, "two warp pairs per block, hardware barriers 1 and 2");
   __shared__ double sh[NT / 32];
   __shared__ LinkT<T> xs[2][NT];
-  pdl_start<MINB>();
   const int w = threadIdx.x >> 5;
   const int half = w & 1, p = (w >> 1) & 1;
-  const int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
+  int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
+  pdl_start<T, MINB>(cb);
   const bool valid = cb < g.cb0 + g.ncb;
   const int cbc = valid ? cb : g.cb0 + g.ncb - 1;
   const int bar_id = 1 + (w >> 1);

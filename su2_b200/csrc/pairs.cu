@@ -23,7 +23,7 @@
 // Within a trajectory only: the start field is copied into the paired layout once
 // (to_pairs), the force launches read and write paired buffers, and the last launch writes
 // the reunitarised final field in the standard layout.
-#include "su2b_internal.h"
+#include "site_ops.cuh"
 
 namespace su2b {
 namespace {
@@ -58,7 +58,7 @@ __device__ __forceinline__ Q2 qdag(const Q2 &u) { return Q2{u.ar, neg(u.ai), neg
 
 template <bool SWAPPED>
 __device__ __forceinline__ Q2 ld_pair(const float4 *__restrict__ Upl, size_t at) {
-  const float4 a = __ldg(Upl + 2 * at), b = __ldg(Upl + 2 * at + 1);
+  const float4 a = Upl[2 * at], b = Upl[2 * at + 1];
   if (SWAPPED)
     return Q2{make_float2(a.y, a.x), make_float2(a.w, a.z), make_float2(b.y, b.x),
               make_float2(b.w, b.z)};
@@ -108,9 +108,6 @@ __global__ void __launch_bounds__(256) k_to_pairs(Geom g, const float4 *__restri
     Upl[2 * i + 1] = make_float4(a.z, b.z, a.w, b.w);
   }
 }
-
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // the fused force step on site pairs: warp mu of block b takes link mu of the 32 pairs
 // (b >> 1) * 32 .. of parity b & 1.  TB: the pair's lower site sits next to the half-lattice
@@ -206,14 +203,13 @@ __device__ __forceinline__ double pair_link(const Geom &g, const Site &s,
 
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB)
-  k_force_su2_pair(Geom g, const float4 *__restrict__ Upl, float *__restrict__ P, float f,
+  k_force_su2_pair(Geom g, const float4 *Upl, float *__restrict__ P, float f,
                    float scale_, int mode, double *kin_part, void *__restrict__ Uout,
                    float dt_upd) {
   __shared__ double sh[4];
-  pdl_trigger();
-  pdl_wait();
   const int w = threadIdx.x >> 5, p = blockIdx.x & 1;
-  const int q = (blockIdx.x >> 1) * 32 + (threadIdx.x & 31);
+  int q = (blockIdx.x >> 1) * 32 + (threadIdx.x & 31);
+  pdl_start<float, MINB>(q);
   double k2 = 0.;
   if (q < g.Vh / 2) {
     const Site s = site_from_eo(g, p, q);
@@ -260,18 +256,8 @@ cudaError_t force_pair(const Geom &g, const void *Upl, float *P, double f, doubl
                        bool pdl) {
   const dim3 grid(2 * ((g.Vh / 2 + 31) / 32));
   if (nblocks) *nblocks = grid.x;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(128);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, k_force_su2_pair<PAIR_MINB>, g, (const float4 *)Upl, P,
-                            (float)f, (float)scale, mode, kin_part, Uout, (float)dt_upd);
+  return launch_force(k_force_su2_pair<PAIR_MINB>, grid, 128, s, pdl, 0, g, (const float4 *)Upl, P,
+                      (float)f, (float)scale, mode, kin_part, Uout, (float)dt_upd);
 }
 
 }  // namespace su2b

@@ -8,12 +8,26 @@ namespace su2b {
 
 template <class T> using LinkT = typename LinkOf<T>::type;
 
-// Programmatic dependent launch between the chained force launches of a trajectory: each
-// block lets the next launch start as soon as it is itself resident, and waits for the
-// previous launch to complete (and its writes to be visible) before it touches global
-// memory.  Both are no-ops for a launch without a programmatic dependency.
+// Programmatic dependent launch between the launches of a chain.  pdl_trigger lets the next
+// launch start once every block of this one has called it or ended; pdl_wait waits for the
+// previous launch to complete and its writes to be visible.  Both are no-ops for a launch
+// without a programmatic dependency.
+// A chained kernel is resident while the launch before still writes what it will read, so it
+//   - reads no field, nor anything else that launch writes, before the wait;
+//   - takes such pointers without const __restrict__, from which the compiler would conclude
+//     that the read-only path may be used, and reads them with ordinary loads;
+//   - with FP64 links passes the index that its addresses come from through the wait (`at`):
+//     their ld_link is an asm statement that a memory clobber does not order, and nothing but
+//     the operand keeps it below.  The FP32 load is the compiler's own and heeds the clobber;
+//     there the operand would cost the 64-register force shapes 20 bytes of spills.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class T> __device__ __forceinline__ void pdl_wait(int &at) {
+  if constexpr (sizeof(T) == 8)
+    asm volatile("griddepcontrol.wait;" : "+r"(at)::"memory");
+  else
+    pdl_wait();
+}
 
 // The start of a chained launch with MINB resident blocks per SM.  A launch of several waves
 // lets the next one start at once: its first blocks take the places that the last wave leaves
@@ -22,9 +36,9 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // down (each of them releases its own successor while it waits); there the next launch starts
 // as blocks exit: ten steps at 12^4 FP64 take 75 us instead of 83 us, at 16^4 124 instead of
 // 131, at 48x40x36 148 instead of 155.
-template <int MINB> __device__ __forceinline__ void pdl_start() {
+template <class T, int MINB> __device__ __forceinline__ void pdl_start(int &at) {
   if (gridDim.x > 148u * MINB) pdl_trigger();
-  pdl_wait();
+  pdl_wait<T>(at);
 }
 
 // launch with the programmatic-stream-serialization attribute when pdl is set

@@ -144,11 +144,14 @@ template <class T> struct Su2 {
   T ar, ai, br, bi;
 };
 
-// The loads carry no side effect, so they are not volatile: the compiler may hoist and
-// overlap them.
+// Loads of links that the kernel itself does not write.  They carry no side effect, so they are
+// not volatile: the compiler may hoist and overlap them, but never above the definition of their
+// address, which in a chained launch is the wait for the launch before (pdl_wait).  Ordinary
+// loads, not the read-only path (.nc): that one asks for memory that nothing writes while the
+// kernel lives, and a chained kernel lives before its links are written.
 __device__ __forceinline__ Su2<double> ld_link(const Link64 *p) {
   Su2<double> r;
-  asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];"
+  asm("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
                : "=d"(r.ar), "=d"(r.ai), "=d"(r.br), "=d"(r.bi)
                : "l"(p));
   return r;
@@ -167,10 +170,10 @@ __device__ __forceinline__ void st_link(Link64 *p, const Su2<double> &u) {
                "d"(u.br), "d"(u.bi)
                : "memory");
 }
-// The FP32 load is left to the compiler (__ldg) rather than written as inline PTX: a link it
-// can no longer keep in a register it may then load again (an L1 hit) instead of spilling.
+// The FP32 load is left to the compiler rather than written as inline PTX: a link it can no
+// longer keep in a register it may then load again (an L1 hit) instead of spilling.
 __device__ __forceinline__ Su2<float> ld_link(const Link32 *p) {
-  const float4 v = __ldg(p);
+  const float4 v = *p;
   return Su2<float>{v.x, v.y, v.z, v.w};
 }
 __device__ __forceinline__ Su2<float> ld_link_rw(const Link32 *p) {
