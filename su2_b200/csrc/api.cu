@@ -134,6 +134,8 @@ extern "C" int su2b_test_set(su2b_ctx *ctx, int what, long value) {
   if (!ctx) return SU2B_ERR_INVALID;
   if (what == SU2B_TEST_FAIL_ALLOCS)
     ctx->fail_allocs = (int)value;
+  else if (what == SU2B_TEST_WAIT_LIMIT)
+    ctx->wait_limit = value;
   else
     return SU2B_ERR_INVALID;
   return SU2B_OK;

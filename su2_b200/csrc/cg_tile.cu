@@ -23,7 +23,8 @@
 // 1e-12: 2.8 ms for 717 iterations at 64^2 where k_bicgstab_persistent takes 9.4 ms for 723,
 // 7.3 ms at 256^2 against 11.9 ms.
 // Every block adds the partials in the same order, so all take the same decisions.  Every wait
-// is bounded: one that gives up tells the host and all blocks return.
+// is bounded: one that gives up tells the host, and all blocks return, those that the missing
+// data were meant for when their own waits run out, a second later at most.
 #include <algorithm>
 #include <cmath>
 #include <type_traits>
@@ -37,7 +38,11 @@ namespace {
 constexpr int MAX_THREADS = 512;
 constexpr int MAX_BLOCKS = 160;  // partials a warp polls: 5 per lane
 constexpr int BI_SUMS = 5;  // sums of one phase at most: the BiCGStab's (the CG: 1)
-constexpr long SPIN_LIMIT = 1L << 21;  // polls of an L2 round trip each: gives up after a second
+// When a wait gives up, after about a second: k_cg_tile counts its polls, an L2 round trip each;
+// k_cg_cluster's try_wait suspends the thread for a time of the hardware's choosing (TRY_NS is a
+// hint), so there the clock is read.
+constexpr long POLL_LIMIT = 1L << 21, CYCLE_LIMIT = 2000000000L;
+constexpr unsigned TRY_NS = 1000000;
 
 __device__ __forceinline__ void put_packet(ulonglong2 *p, double v, unsigned long long epoch) {
   asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}"
@@ -68,6 +73,7 @@ struct CgTileArgs {
   int *err;
   double tol;
   long max_iter;
+  long limit;  // POLL_LIMIT or CYCLE_LIMIT; a test sets 0, and every wait of a cluster runs out
 };
 
 // m v + sgn hop(v) at a site of slice t: the arithmetic of hop_site64 (staggered.cu) in d = 2.
@@ -328,7 +334,8 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_tile(CgTileArgs a) {
 #pragma unroll
       for (int j = 0; j < N; j++)
         if ((want >> j & 1) && e[j] == ep) v[j] = __longlong_as_double((long long)d[j]), want &= ~(1u << j);
-      if ((++spins & 255) == 0 && (spins > SPIN_LIMIT || *(volatile int *)a.err)) {
+      spins++;
+      if (spins > a.limit || ((spins & 255) == 0 && *(volatile int *)a.err)) {
         atomicExch(a.err, 1);
         *(volatile int *)&a.out->failed = 1;
         sh_bad = 1;
@@ -469,7 +476,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
   using Buf = ClusterBuf<K, BI>;
   Buf *const B = (Buf *)smem;
   constexpr uint32_t STEP = sizeof(Buf);
-  __shared__ unsigned sh_bad;  // the first phase in which a wait gave up
+  __shared__ unsigned sh_bad;  // the phase in which a wait gave up
   const CgTilePlan tp = a.tp;
   const int Lt = a.g.L[0], Lx = a.g.L[1], V = a.g.V, Vh = a.g.Vh;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
@@ -578,7 +585,7 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
       push(dst2[k], dbar2[k]);
     }
     __syncthreads();
-    if (*(volatile unsigned *)&sh_bad < n) return false;  // in an earlier phase: the same for all
+    if (*(volatile unsigned *)&sh_bad < n) return false;  // in the last phase: the same for all
     for (int i = warp; i < NS; i += nw) {  // a warp for each sum
       double q[MAX_THREADS / 32];
 #pragma unroll
@@ -594,20 +601,24 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
                      "d"(q[0]), "r"(peer_bar + off)
                      : "memory");
     }
-    {
+    // A warp waits as one.  One that gives up joins the barrier at which the block's other warps
+    // next meet, in their next phase or after their last one, and so tells them all.
+    for (long long since = 0;;) {
       uint32_t ok = 0;
-      for (long spins = 0; !ok; spins++) {
-        asm volatile("{\n\t.reg .pred q;\n\t"
-                     "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2;\n\t"
-                     "selp.u32 %0, 1, 0, q;\n\t}"
-                     : "=r"(ok)
-                     : "r"(my_bar + off), "r"(parity)
-                     : "memory");
-        if (spins > SPIN_LIMIT) {
-          *(volatile int *)&a.out->failed = 1;
-          atomicMin(&sh_bad, n);
-          break;
-        }
+      asm volatile("{\n\t.reg .pred q;\n\t"
+                   "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 q, [%1], %2, %3;\n\t"
+                   "selp.u32 %0, 1, 0, q;\n\t}"
+                   : "=r"(ok)
+                   : "r"(my_bar + off), "r"(parity), "r"(TRY_NS)
+                   : "memory");
+      if (__all_sync(0xffffffffu, ok) && a.limit > 0) break;
+      const long long now = clock64();
+      if (since == 0) since = now;
+      if (__any_sync(0xffffffffu, now - since >= a.limit)) {
+        *(volatile int *)&a.out->failed = 1;
+        *(volatile unsigned *)&sh_bad = n;
+        __syncthreads();
+        return false;
       }
     }
     double2 w[K][4];
@@ -635,13 +646,21 @@ __global__ void __launch_bounds__(MAX_THREADS, 1) k_cg_cluster(CgTileArgs a) {
     return true;
   };
   CgEnd end;
-  const bool good = BI ? bi_run<K>(on, x, b, a.tol, a.max_iter, phase, end)
-                       : cg_run<K>(on, x, b, a.tol, a.max_iter, phase, end);
+  bool good = BI ? bi_run<K>(on, x, b, a.tol, a.max_iter, phase, end)
+                 : cg_run<K>(on, x, b, a.tol, a.max_iter, phase, end);
+  if (good) {
+    __syncthreads();
+    good = *(volatile unsigned *)&sh_bad > n;
+  }
   if (good) {
 #pragma unroll
     for (int k = 0; k < K; k++)
       if (on[k]) a.x[eo(t0 + r0 + k * tp.rp, xc)] = x[k];
     if (blockIdx.x == 0 && tid == 0) write_result(a.out, end, a.epoch);
+  } else {
+    // what was sent to a block that no longer waits for it is still to arrive: a millisecond
+    for (const long long since = clock64(); clock64() - since < 2000000;) {
+    }
   }
   cluster_sync();  // no block leaves while another may send to it
 }
@@ -754,13 +773,14 @@ size_t cg_tile_bytes(const Geom &g) {
 
 cudaError_t cg_tile(const Geom &g, const CgTilePlan &tp, bool bicgstab, const double2 *ph,
                     double m, const double2 *b, double2 *x, double tol, long max_iter, void *work,
-                    unsigned long long epoch, CgTileResult *out, cudaStream_t s) {
+                    unsigned long long epoch, CgTileResult *out, cudaStream_t s, long limit) {
   CgTileArgs a{};
   a.g = g, a.tp = tp, a.ph = ph, a.m = m, a.b = b, a.x = x, a.tol = tol, a.max_iter = max_iter;
   a.halo = (ulonglong2 *)work;
   a.sums = a.halo + (size_t)4 * g.V;
   a.err = (int *)(a.sums + 2 * BI_SUMS * MAX_BLOCKS);
   a.epoch = epoch, a.out = out;
+  a.limit = limit >= 0 ? limit : tp.cluster ? CYCLE_LIMIT : POLL_LIMIT;
   const int nt = (tp.rp * tp.hx + 31) / 32 * 32;
   if (tp.cluster) {
     const auto kern = bicgstab ? (tp.K == 1 ? k_cg_cluster<1, true> : k_cg_cluster<2, true>)

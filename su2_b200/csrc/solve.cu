@@ -130,7 +130,7 @@ int cg_tiled(su2b_ctx *ctx, bool bicgstab, double m, double tol, int max_iter,
   h.failed = 0;
   const cudaError_t e = cg_tile(ctx->g, ctx->cg_plan, bicgstab, ctx->ph, m, ctx->sv[SV_B],
                                 ctx->sv[SV_X], tol, max_iter, ctx->cg_work, ctx->cg_epoch,
-                                ctx->h_cg, s);
+                                ctx->h_cg, s, ctx->wait_limit);
   if (e == cudaErrorNotSupported) return SU2B_OK;
   SU2B_CK(e);
   ctx->launches++;

@@ -89,7 +89,8 @@ cudaError_t bicgstab_persistent(const Geom &g, const double2 *ph, double m, doub
 // plan: cg_tile_plan, K = 0 where the lattice does not take it (d != 2, too large, or no
 // cooperative launch).  work: cg_tile_bytes of memory zeroed once, kept between solves; epoch:
 // the result's epoch of the last solve with this work (0 at first).  out: pinned host memory.
-// cudaErrorNotSupported: the blocks do not fit beside each other now.
+// cudaErrorNotSupported: the blocks do not fit beside each other now.  limit: polls or cycles
+// after which a wait gives up (-1: about a second)
 struct CgTilePlan {
   int K;       // sites per thread
   int ht, hx;  // tile rows (t) and columns (x)
@@ -109,7 +110,7 @@ size_t cg_tile_bytes(const Geom &g);
 bool cg_tile_bicgstab(const CgTilePlan &p);
 cudaError_t cg_tile(const Geom &g, const CgTilePlan &tp, bool bicgstab, const double2 *ph,
                     double m, const double2 *b, double2 *x, double tol, long max_iter, void *work,
-                    unsigned long long epoch, CgTileResult *out, cudaStream_t s);
+                    unsigned long long epoch, CgTileResult *out, cudaStream_t s, long limit = -1);
 int cg_barrier_failed(const void *bar_mem, cudaStream_t s, int *failed);
 size_t cg_barrier_bytes();
 

@@ -99,7 +99,8 @@ struct su2b_ctx {
   std::vector<void *> allocs;
   std::string err;
 
-  // su2b_test_set: the next fail_allocs allocations ask for more than any device has
+  // su2b_test_set: the tiled solve's wait limit (-1: its own); the next fail_allocs allocations ask for more than any device has
+  long wait_limit = -1;
   int fail_allocs = 0;
   size_t alloc_size(size_t bytes) {
     if (fail_allocs == 0) return bytes;
@@ -135,7 +136,7 @@ void su2b_arena_busy(su2b_ctx *ctx, bool busy);
 // device memory of the context; SU2B_ERR_NOMEM with a message if it is refused
 int su2b_dalloc(su2b_ctx *ctx, void **p, size_t bytes);
 // for the tests, not in su2b.h: failures made on the host
-enum { SU2B_TEST_FAIL_ALLOCS = 0 };
+enum { SU2B_TEST_FAIL_ALLOCS = 0, SU2B_TEST_WAIT_LIMIT = 1 };
 extern "C" __attribute__((visibility("default"))) int su2b_test_set(su2b_ctx *ctx, int what,
                                                                     long value);
 int su2b_adj_upload(su2b_ctx *ctx, const double *host, void *dev);

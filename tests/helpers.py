@@ -24,9 +24,19 @@ def group_name(g):
     return "su2" if g == 0 else "u1"
 
 
-def fail_allocations(lattice, n):
-    """The next n device allocations of the lattice's context ask for more than a device has."""
+def context_setting(lattice, what, value):
+    """A setting of the lattice's context that only tests use (su2b_ctx.h)."""
     import ctypes as C
     f = lattice.lib.su2b_test_set
     f.argtypes, f.restype = [C.c_void_p, C.c_int, C.c_long], C.c_int
-    assert f(lattice.ctx, 0, n) == 0
+    assert f(lattice.ctx, what, value) == 0
+
+
+def fail_allocations(lattice, n):
+    """The next n device allocations of the lattice's context ask for more than a device has."""
+    context_setting(lattice, 0, n)
+
+
+def wait_limit(lattice, n):
+    """The polls or cycles after which a wait of the tiled solves gives up (-1: their own)."""
+    context_setting(lattice, 1, n)

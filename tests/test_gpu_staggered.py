@@ -7,7 +7,7 @@ residual, 1e-12, so they differ by rounding only); fermion force 1e-8 relative.
 import numpy as np
 import pytest
 
-from helpers import rel
+from helpers import rel, wait_limit
 
 pytestmark = pytest.mark.gpu
 
@@ -275,3 +275,29 @@ def test_cg_tilings(gpu, Lx, Lt):
         assert again.converged and again.iterations == 0 and np.array_equal(again.x, r.x)
         few = c.solve(b, m, tol=1e-14, tol_mode="rel", max_iter=2)
         assert few.iterations <= 2
+
+
+# one cluster of one and of two sites per thread; the whole GPU with one and with two
+@pytest.mark.parametrize("solver", ["CG", "BiCGStab"])
+@pytest.mark.parametrize("Lx,Lt", [(64, 64), (128, 128), (256, 250), (300, 340)])
+def test_a_wait_of_the_tiled_solve_gives_up(gpu, Lx, Lt, solver):
+    """With no patience every wait of the cluster gives up, and over the whole GPU every wait that
+    does not find its data at the first look: the solve ends with the timeout's status, and the
+    next one in the same context, whose packets the failed one has used, is that of a fresh
+    context, bit for bit."""
+    from su2_b200 import _abi
+    rng = np.random.default_rng(Lx)
+    U, b = rng.normal(size=2 * Lx * Lt), rng.normal(size=2 * Lx * Lt)
+    with u1(gpu, (Lx, 1, 1, Lt), 2) as c, u1(gpu, (Lx, 1, 1, Lt), 2) as fresh:
+        c.upload(U)
+        fresh.upload(U)
+        for _ in range(2):
+            wait_limit(c, 0)
+            with pytest.raises(gpu.Su2bError) as e:
+                c.solve(b, 0.3, tol=1e-10, tol_mode="rel", solver=solver)
+            assert e.value.code == _abi.ERR_TIMEOUT
+            wait_limit(c, -1)
+            r = c.solve(b, 0.3, tol=1e-10, tol_mode="rel", solver=solver)
+            want = fresh.solve(b, 0.3, tol=1e-10, tol_mode="rel", solver=solver)
+            assert r.converged and r.iterations == want.iterations
+            np.testing.assert_array_equal(r.x, want.x)
