@@ -837,7 +837,7 @@ def profile_run(args):
     n1 = launches()
     print(json.dumps({"profile_run": f"SU(2) d=4 {L}^4, beta={BETA}", "op": args.profile_op,
                       "precision": args.precision,
-                      "force_variant": su2_b200._abi.FORCE_SHAPES[args.force_variant],
+                      "force_variant": su2_b200._abi.force_shape(args.force_variant, [L] * 4, 4),
                       "setup_launches": n0, "launches_per_step": (n1 - n0) / max(1, args.steps),
                       "steps": args.steps, "warmup": args.warmup}), flush=True)
     c.close()
@@ -914,8 +914,9 @@ def config1(args):
               dtype="fp64", acceptance=sum(r.accepted for r in res) / K,
               plaquette_mean=float(np.mean(plaq)), plaquette_last=plaq[-1],
               gpu_launches=c.kernel_launches() - n0, cpu_baseline=cpu,
-              autotune_force_us={str(su2_b200._abi.FORCE_SHAPES[k]): v for k, v in tune.items()},
-              force_shape=su2_b200._abi.FORCE_SHAPES[c.force_variant])
+              autotune_force_us={str(su2_b200._abi.force_shape(k, (8, 8, 8, 8), 4)): v
+                                 for k, v in tune.items()},
+              force_shape=su2_b200._abi.force_shape(c.force_variant, (8, 8, 8, 8), 4))
     c.close()
 
 

@@ -146,11 +146,21 @@ BATCH_VARIANTS = 4
 BATCH_SHAPES = [(64, 8), (128, 4), (128, 6), (256, 3)]
 # (threads per block, min resident blocks per SM) of the force kernel's launch shapes; the
 # "split" shapes run two threads per site (d = 4; other d use (128, 8)), "xsplit" with the
-# cross-plane products formed once per site and swapped in shared memory; (256, 3) runs three
-# threads per link on d = 4 lattices of at most 1024 sites per time slice; the anisotropic
-# action always runs (128, 6)
+# cross-plane products formed once per site and swapped in shared memory; force_shape names what
+# a variant runs on a given lattice; the anisotropic action always runs (128, 6)
 FORCE_SHAPES = [(256, 4), (128, 8), (128, 4), (128, 6), (256, 2), (256, 3), ("split", 128, 8),
                 (64, 16), ("xsplit", 128, 8), ("link", 128, 6), ("split", 128, 5), ("pair", 128, 8)]
+# sites of a time slice up to which variant 5 of a d = 4 lattice runs three threads per link
+PLANES_SLICE = 1024
+
+
+def force_shape(variant, dims, ndims):
+    """The launch shape that a force variant runs on a lattice of extents (Lx, Ly, Lz, Lt)."""
+    Lx, Ly, Lz, _ = dims
+    if variant == 5 and ndims == 4 and Lx * Ly * Lz <= PLANES_SLICE:
+        return ("planes", 384, 1)
+    return FORCE_SHAPES[variant]
+
 
 K_FORCE, K_UPDATE, K_PLAQUETTE, K_MOMENTA, K_RESTORE, K_METROPOLIS, K_CLOVER, K_STAGGERED, \
     K_OTHER = range(9)

@@ -28,8 +28,10 @@ std::string tune_key(su2b_ctx *ctx) {
   for (char &c : gpu)
     if (c == ' ') c = '_';
   char buf[256];
-  snprintf(buf, sizeof buf, "%s/force/%s/%dx%dx%dx%d/d%d", gpu.c_str(),
-           ctx->link64 ? "fp64" : "fp32", ctx->Lx, ctx->Ly, ctx->Lz, ctx->Lt, ctx->g.nd);
+  // where shape 5 is three threads per link the key says so: an earlier file's 5 was (256, 3)
+  snprintf(buf, sizeof buf, "%s/force/%s/%dx%dx%dx%d/d%d%s", gpu.c_str(),
+           ctx->link64 ? "fp64" : "fp32", ctx->Lx, ctx->Ly, ctx->Lz, ctx->Lt, ctx->g.nd,
+           force_planes_apply(ctx->g) ? "/planes" : "");
   return buf;
 }
 

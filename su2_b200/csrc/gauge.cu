@@ -767,7 +767,7 @@ __global__ void __launch_bounds__(NT, MINB)
 // larger lattices ties with (128, 6).  The line is drawn in the sites of a time slice, not in
 // all sites, so that a slab takes the shape that the whole lattice takes, bit for bit; long
 // lattices that it admits are left to the tuner, which times the other shapes as well.
-static bool force_planes_apply(const Geom &g) {
+bool force_planes_apply(const Geom &g) {
   return g.nd == 4 && (long)g.L[1] * g.L[2] * g.L[3] <= 1024;
 }
 

@@ -52,6 +52,7 @@ enum ForceMode : int {
 // paired copy of the field; every other caller, and FP64 links, run the one-thread-per-link
 // kernel, whose arithmetic force_pair reproduces lane for lane)
 constexpr int FORCE_VARIANTS = 12;
+bool force_planes_apply(const Geom &g);
 constexpr int FORCE_PAIR = 11;
 constexpr int PAIR_MINB = 8;  // resident blocks of 128 threads per SM of force_pair
 // site pairs (pairs.cu): whether a geometry takes them (d = 4, T % 4 == 0, the whole

@@ -97,6 +97,22 @@ def test_launch_shape_tables_agree_with_the_header():
     assert int(re.search(r"constexpr int FORCE_VARIANTS = (\d+);", src).group(1)) == nf
 
 
+def test_force_shape_names_what_a_variant_runs():
+    """Variant 5 is three threads per link up to the number of sites of a time slice that the
+    library's rule has, and (256, 3) beyond it and below four dimensions."""
+    from su2_b200 import _abi
+    src = open(os.path.join(ROOT, "su2_b200", "csrc", "gauge.cu")).read()
+    rule = re.search(r"bool force_planes_apply\(const Geom &g\) \{\s*return g\.nd == 4 && "
+                     r"\(long\)g\.L\[1\] \* g\.L\[2\] \* g\.L\[3\] <= (\d+);", src)
+    assert int(rule.group(1)) == _abi.PLANES_SLICE
+    for dims, nd, want in (((8, 8, 8, 8), 4, "planes"), ((8, 8, 16, 4), 4, "planes"),
+                           ((8, 8, 18, 4), 4, 256), ((32, 32, 32, 32), 4, 256),
+                           ((8, 8, 1, 8), 3, 256)):
+        assert _abi.force_shape(5, dims, nd)[0] == want
+        for v in set(range(_abi.FORCE_VARIANTS)) - {5}:
+            assert _abi.force_shape(v, dims, nd) == _abi.FORCE_SHAPES[v]
+
+
 def test_noalloc_rejects_bad_sizes_before_touching_a_device():
     """su2b_gauge_energy_noalloc validates its geometry on the host: lattices beyond its
     fixed scratch array, extents whose product would wrap, bad ids and NULL buffers are

@@ -564,6 +564,22 @@ def test_autotune_cache(gpu, orc, tmp_path):
         assert all(v < 0 for v in t2.values()) and c.force_variant == best
 
 
+def test_autotune_cache_of_an_earlier_shape_5(gpu, tmp_path):
+    """On a lattice where shape 5 became three threads per link, a cache line that chose the
+    earlier shape 5 is timed afresh; on a larger one it still holds."""
+    import torch
+    name = torch.cuda.get_device_name(0).replace(" ", "_")
+    path = tmp_path / "tune.txt"
+    path.write_text(f"{name}/force/fp64/8x8x8x8/d4 5 1.0\n"
+                    f"{name}/force/fp64/12x12x12x12/d4 5 1.0\n")
+    with make(gpu, 0, (8, 8, 8, 8), 4) as a, make(gpu, 0, (12, 12, 12, 12), 4) as b:
+        assert all(v > 0 for v in a.autotune(str(path)).values())
+        chosen = a.force_variant
+        a.force_variant = (chosen + 1) % gpu._abi.FORCE_VARIANTS
+        assert all(v < 0 for v in a.autotune(str(path)).values()) and a.force_variant == chosen
+        assert all(v < 0 for v in b.autotune(str(path)).values()) and b.force_variant == 5
+
+
 @pytest.mark.parametrize("dims", [(8, 8, 8, 8), (4, 6, 8, 12), (6, 6, 6, 4), (4, 4, 6, 6)],
                          ids=["8^4", "4x6x8x12", "6^3x4", "4x4x6x6-no-pairs"])
 def test_site_pairs_equal_the_link_kernel(gpu, orc, dims):
