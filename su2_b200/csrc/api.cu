@@ -136,6 +136,8 @@ extern "C" int su2b_test_set(su2b_ctx *ctx, int what, long value) {
     ctx->fail_allocs = (int)value;
   else if (what == SU2B_TEST_WAIT_LIMIT)
     ctx->wait_limit = value;
+  else if (what == SU2B_TEST_LEAVE_ERROR)
+    cudaSetDevice(-1);  // refused: the error stays for the next launch's check
   else
     return SU2B_ERR_INVALID;
   return SU2B_OK;
@@ -559,6 +561,12 @@ extern "C" int su2b_metropolis_sweep(su2b_ctx *ctx, double delta, int N_hit, uin
   CKS(enter(ctx));
   NEED(rates, "rates is NULL");
   NEED(N_hit >= 0, "N_hit < 0");
+  if (ctx->sweep_open) {  // a sweep ended early: it left its counts
+    CK(cudaMemsetAsync(ctx->counts, 0, 2 * sizeof(unsigned long long), ctx->stream));
+    CK(cudaMemsetAsync(ctx->ticket, 0, sizeof(unsigned), ctx->stream));
+  }
+  ctx->sweep_open = true;
+  ctx->phases_valid = false;
   for (int mu = 0; mu < ctx->g.nd; mu++)
     for (int p = 0; p < 2; p++) {
       const bool last = mu == ctx->g.nd - 1 && p == 1;
@@ -571,7 +579,7 @@ extern "C" int su2b_metropolis_sweep(su2b_ctx *ctx, double delta, int N_hit, uin
                                   seed, sweep, counts, ctx->stream));
     }
   CK(cudaStreamSynchronize(ctx->stream));
-  ctx->phases_valid = false;
+  ctx->sweep_open = false;
   if (ctx->pend.size() > 4096) CKS(su2b_prof_fold(ctx));
   const double nh = (double)(N_hit > 0 ? N_hit : 1);
   rates[0] = (double)ctx->h_counts[0] / nh / (double)ctx->NL;

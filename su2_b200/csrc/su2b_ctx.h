@@ -38,7 +38,8 @@ struct su2b_ctx {
   double *red = nullptr;    // 64 reduced scalars
   su2b::TrajDev *traj = nullptr;
   su2b::TrajParams *tparams = nullptr, *h_tparams = nullptr;
-  unsigned long long *counts = nullptr;
+  unsigned long long *counts = nullptr;  // of a Metropolis sweep, zero between sweeps
+  bool sweep_open = false;               // unless one ended with an error
   unsigned *ticket = nullptr;  // of finish_sums, zero between launches
 
   // pinned host mirrors
@@ -136,7 +137,7 @@ void su2b_arena_busy(su2b_ctx *ctx, bool busy);
 // device memory of the context; SU2B_ERR_NOMEM with a message if it is refused
 int su2b_dalloc(su2b_ctx *ctx, void **p, size_t bytes);
 // for the tests, not in su2b.h: failures made on the host
-enum { SU2B_TEST_FAIL_ALLOCS = 0, SU2B_TEST_WAIT_LIMIT = 1 };
+enum { SU2B_TEST_FAIL_ALLOCS = 0, SU2B_TEST_WAIT_LIMIT = 1, SU2B_TEST_LEAVE_ERROR = 2 };
 extern "C" __attribute__((visibility("default"))) int su2b_test_set(su2b_ctx *ctx, int what,
                                                                     long value);
 int su2b_adj_upload(su2b_ctx *ctx, const double *host, void *dev);

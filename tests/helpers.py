@@ -37,6 +37,11 @@ def fail_allocations(lattice, n):
     context_setting(lattice, 0, n)
 
 
+def leave_error(lattice):
+    """An error of this thread's CUDA runtime that nobody has looked at."""
+    context_setting(lattice, 2, 0)
+
+
 def wait_limit(lattice, n):
     """The polls or cycles after which a wait of the tiled solves gives up (-1: their own)."""
     context_setting(lattice, 1, n)

@@ -6,7 +6,7 @@ Tolerances: FP64 results within 1e-12 relative (norm-wise for fields), FP64 sums
 import numpy as np
 import pytest
 
-from helpers import GEOM_IDS, GEOMS, group_name, rel
+from helpers import GEOM_IDS, GEOMS, group_name, leave_error, rel
 
 pytestmark = pytest.mark.gpu
 
@@ -271,6 +271,23 @@ def test_metropolis_pass_forms(gpu, orc, dims, nd, hits):
             assert rel(c.download(), U) < 1e-11
             if hits:
                 np.testing.assert_array_equal(rates, want)
+
+
+def test_metropolis_rates_after_a_sweep_that_failed(gpu, orc):
+    """A sweep that ends at its first launch has moved links and counted hits; the next one
+    counts its own only.  (The U(1) passes report an error that was there before them.)"""
+    dims, nd = (8, 1, 1, 6), 2
+    U = hot(orc, 1, dims, nd)
+    with make(gpu, 1, dims, nd) as c:
+        c.upload(U)
+        want = c.sweep(0.3, 5, 99, 0)
+        c.upload(U)
+        leave_error(c)
+        with pytest.raises(gpu.Su2bError):
+            c.sweep(0.3, 5, 99, 0)
+        for _ in range(2):
+            c.upload(U)
+            np.testing.assert_array_equal(c.sweep(0.3, 5, 99, 0), want)
 
 
 @pytest.mark.parametrize("group,dims,nd", [g for g in GEOMS if g[0] == 0],
