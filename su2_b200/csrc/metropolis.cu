@@ -15,6 +15,8 @@
 // one Philox4x32-10 draw per hit, counter {reference link index, hit, sweep, TAG_METRO}:
 // 32-bit uniforms for alpha, u, theta and the accept test, the same stream in both
 // precisions.
+#include <climits>
+
 #include "site_ops.cuh"
 
 namespace su2b {
@@ -177,6 +179,18 @@ __global__ void __launch_bounds__(NT, MINB)
 // one thread per link (65 us before the chain of a hit lost its square root and division and the
 // passes their launch gaps).
 constexpr int WIDE_HITS = 16;
+// chunks of N hits and the hits of chunk c < chunks, in the range of int for every N
+__host__ __device__ constexpr int wide_chunks(int N) {
+  return N / WIDE_HITS + (N % WIDE_HITS != 0);
+}
+__host__ __device__ constexpr int wide_hits(int c, int N) {
+  return N - c * WIDE_HITS < WIDE_HITS ? N - c * WIDE_HITS : WIDE_HITS;
+}
+static_assert(wide_chunks(0) == 0 && wide_chunks(16) == 1 && wide_chunks(17) == 2 &&
+              wide_hits(0, 16) == 16 && wide_hits(1, 17) == 1, "chunks of sixteen hits");
+static_assert(wide_chunks(INT_MAX) == INT_MAX / WIDE_HITS + 1 &&
+              wide_hits(wide_chunks(INT_MAX) - 1, INT_MAX) == INT_MAX % WIDE_HITS,
+              "the last chunk of the most hits, whose successor's first hit is no int");
 template <class T, int ND>
 __global__ void __launch_bounds__(256, 2)
   k_metro_su2_wide(Geom g, LinkT<T> *__restrict__ U, int mu, int p, double beta_nc, double delta,
@@ -190,8 +204,11 @@ __global__ void __launch_bounds__(256, 2)
   const bool on = cb < g.cb0 + g.ncb;
   const Site s = site_from_eo(g, p, on ? cb : g.cb0);
   const uint32_t lref = (uint32_t)(s.lex + g.lex0) * (uint32_t)g.nd + (uint32_t)mu;
+  const int chunks = wide_chunks(N_hit);
   auto draw = [&](int chunk, int first, int step) {
-    for (int i = first; i < WIDE_HITS && chunk * WIDE_HITS + i < N_hit; i += step)
+    if (chunk >= chunks) return;
+    const int n = wide_hits(chunk, N_hit);
+    for (int i = first; i < n; i += step)
       prop[chunk & 1][i][lane] = as_link(proposal(lref, chunk * WIDE_HITS + i, sweep, seed, (T)delta,
                                                   acc_u[chunk & 1][i][lane]));
   };
@@ -207,10 +224,10 @@ __global__ void __launch_bounds__(256, 2)
     tr_u = retr_mul(to64(u), K64);
   }
   unsigned acc = 0;
-  for (int c = 0; c * WIDE_HITS < N_hit; c++) {
+  for (int c = 0; c < chunks; c++) {
     __syncthreads();
     if (w == 0) {
-      const int n = min(WIDE_HITS, N_hit - c * WIDE_HITS);
+      const int n = wide_hits(c, N_hit);
       for (int i = 0; i < n; i++)
         acc += metro_hit(u, tr_u, K64, from_link(prop[c & 1][i][lane]), acc_u[c & 1][i][lane],
                          beta_nc);
