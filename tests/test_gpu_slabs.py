@@ -106,6 +106,21 @@ def test_slab_metropolis_sweeps(gpu, orc, precision, dims, nd, nslabs):
         assert s.gauge_energy() == pytest.approx(c.gauge_energy(), rel=1e-13)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("dims,nd,xi", [((12, 12, 12, 12), 4, 1.0), ((12, 10, 14, 12), 4, 0.8),
+                                        ((24, 20, 1, 44), 3, 1.0), ((100, 1, 1, 200), 2, 1.0)])
+def test_slabs_whose_passes_take_another_form(gpu, orc, precision, dims, nd, xi):
+    """More than 9,472 links in a pass of the lattice, fewer in a pass of each of its two slabs:
+    one thread per link here, eight warps per 32 links there, and the same links and rates."""
+    U = hot(orc, dims, nd)
+    with single(gpu, dims, nd, precision, xi=xi) as c, slabs(dims, nd, 2, precision, xi=xi) as s:
+        c.upload(U)
+        s.upload(U)
+        for k in range(3):
+            assert np.array_equal(c.sweep(0.25, 6, 21, k), s.sweep(0.25, 6, 21, k)), k
+            assert np.array_equal(c.download(), s.download()), k
+
+
 def test_slabs_alternate_sweeps_and_trajectories(gpu, orc):
     """The workload's alternation (Metropolis sweeps between HMC trajectories) over 4 slabs
     in mixed precision: after each step the single lattice's field."""
