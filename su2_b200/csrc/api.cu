@@ -240,9 +240,12 @@ extern "C" int su2b_ctx_create(int group, int Lx, int Ly, int Lz, int Lt, int nd
   if (cudaMallocHost((void **)&ctx->h_red, sizeof(double) * 64) != cudaSuccess ||
       cudaMallocHost((void **)&ctx->h_traj, sizeof(TrajDev)) != cudaSuccess ||
       cudaMallocHost((void **)&ctx->h_counts, sizeof(unsigned long long) * 4) != cudaSuccess ||
-      cudaMallocHost((void **)&ctx->h_st, sizeof(SolverState)) != cudaSuccess ||
+      cudaMallocHost((void **)&ctx->h_st, sizeof(SolverState) + sizeof(CgTileResult)) !=
+        cudaSuccess ||
       cudaMallocHost((void **)&ctx->h_tparams, sizeof(TrajParams)) != cudaSuccess)
     return fin(SU2B_ERR_NOMEM);
+  static_assert(sizeof(SolverState) % alignof(CgTileResult) == 0, "the result follows the state");
+  ctx->h_cg = (CgTileResult *)(ctx->h_st + 1);
   if (cudaMemsetAsync(ctx->U, 0, lb * NL, ctx->stream) != cudaSuccess ||
       cudaMemsetAsync(ctx->counts, 0, 4 * sizeof(unsigned long long), ctx->stream) !=
         cudaSuccess ||
@@ -271,7 +274,6 @@ extern "C" int su2b_ctx_destroy(su2b_ctx *ctx) {
   if (ctx->h_traj) cudaFreeHost(ctx->h_traj);
   if (ctx->h_counts) cudaFreeHost(ctx->h_counts);
   if (ctx->h_st) cudaFreeHost(ctx->h_st);
-  if (ctx->h_cg) cudaFreeHost(ctx->h_cg);
   if (ctx->h_tparams) cudaFreeHost(ctx->h_tparams);
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;

@@ -100,15 +100,11 @@ int cg_tile_setup(su2b_ctx *ctx) {
   const CgTilePlan plan = cg_tile_plan(ctx->g);
   if (!plan.K) return SU2B_OK;
   void *work = nullptr;
-  if (su2b_malloc(&work, ctx->alloc_size(cg_tile_bytes(ctx->g))) == cudaSuccess &&
-      cudaMallocHost((void **)&ctx->h_cg, sizeof(CgTileResult)) == cudaSuccess) {
+  if (su2b_malloc(&work, ctx->alloc_size(cg_tile_bytes(ctx->g))) == cudaSuccess) {
     ctx->allocs.push_back(work);
     SU2B_CK(cudaMemsetAsync(work, 0, cg_tile_bytes(ctx->g), ctx->stream));
     ctx->cg_work = work;
     ctx->cg_plan = plan;
-  } else {
-    cudaFree(work);
-    cudaGetLastError();
   }
   return SU2B_OK;
 }
@@ -462,22 +458,30 @@ int solve_phi(su2b_ctx *ctx, double mass, double tol, int max_iter, long *iters)
 }  // namespace
 
 // ===================================================================================
+// The fields of the fermions in one allocation: all of them or none, and a new context's first
+// solve at 256^2 takes 1.4 ms, 3.9 ms with an allocation for each of 17.
+static size_t aligned(size_t bytes) { return (bytes + 255) & ~(size_t)255; }
 int su2b_fermion_setup(su2b_ctx *ctx, bool need32) {
   if (ctx->group != SU2B_GROUP_U1)
     return su2b_fail(ctx, SU2B_ERR_UNSUPPORTED,
                      "staggered fermions are not supported for SU(2) (staggered.hpp:343-350)");
   if (!ctx->ph) {
-    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->ph, ctx->NL * sizeof(double2)));
-    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->fderiv, ctx->NL * sizeof(double)));
-    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->st, sizeof(SolverState)));
-    for (int k = 0; k < SV_N; k++)
-      SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->sv[k], ctx->V * sizeof(double2)));
+    char *at = nullptr;
+    const size_t ph = aligned(ctx->NL * sizeof(double2)), fd = aligned(ctx->NL * sizeof(double)),
+                 st = aligned(sizeof(SolverState)), v = aligned(ctx->V * sizeof(double2));
+    SU2B_CKS(su2b_dalloc(ctx, (void **)&at, ph + fd + st + SV_N * v));
+    ctx->ph = (double2 *)at;
+    ctx->fderiv = (double *)(at + ph);
+    ctx->st = (SolverState *)(at + ph + fd);
+    for (int k = 0; k < SV_N; k++) ctx->sv[k] = (double2 *)(at + ph + fd + st + k * v);
     ctx->phases_valid = false;
   }
   if (need32 && !ctx->ph32) {
-    SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->ph32, ctx->NL * sizeof(float2)));
-    for (int k = 0; k < SV32_N; k++)
-      SU2B_CKS(su2b_dalloc(ctx, (void **)&ctx->sv32[k], ctx->V * sizeof(float2)));
+    char *at = nullptr;
+    const size_t ph = aligned(ctx->NL * sizeof(float2)), v = aligned(ctx->V * sizeof(float2));
+    SU2B_CKS(su2b_dalloc(ctx, (void **)&at, ph + SV32_N * v));
+    ctx->ph32 = (float2 *)at;
+    for (int k = 0; k < SV32_N; k++) ctx->sv32[k] = (float2 *)(at + ph + k * v);
     ctx->phases32_valid = false;
   }
   return ensure_phases(ctx, need32);

@@ -62,7 +62,7 @@ struct su2b_ctx {
   int bi_tiled = -1;  // whether the BiCGStab runs on the plan (-1: not asked yet)
   void *cg_work = nullptr;
   unsigned long long cg_epoch = 0;
-  su2b::CgTileResult *h_cg = nullptr;
+  su2b::CgTileResult *h_cg = nullptr;  // pinned, behind h_st
   long x0_seed = -1;  // seed of the reference CG start held in sv[SV_X0]
 
   // set at the end of a fused trajectory: red[] then holds the plaquette sums of both the

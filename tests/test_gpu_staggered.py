@@ -7,7 +7,7 @@ residual, 1e-12, so they differ by rounding only); fermion force 1e-8 relative.
 import numpy as np
 import pytest
 
-from helpers import rel, wait_limit
+from helpers import fail_allocations, rel, wait_limit
 
 pytestmark = pytest.mark.gpu
 
@@ -301,3 +301,30 @@ def test_a_wait_of_the_tiled_solve_gives_up(gpu, Lx, Lt, solver):
             want = fresh.solve(b, 0.3, tol=1e-10, tol_mode="rel", solver=solver)
             assert r.converged and r.iterations == want.iterations
             np.testing.assert_array_equal(r.x, want.x)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("refused", [1, 2, 3])
+def test_a_solve_without_memory(gpu, orc, precision, refused):
+    """A solve whose fields find no memory is an error, and the next call has all of them.  (In
+    d = 3 the mixed solver takes a second set; the tiled solve's packets are the second in d = 2,
+    where the other form runs without them.)"""
+    for dims, nd in (((8, 1, 1, 6), 2), ((6, 4, 1, 4), 3)):
+        U, b, _ = setup(orc, dims, nd)
+        solver = "CG_mixed" if precision == "mixed" else "CG"
+        with u1(gpu, dims, nd, precision=precision) as c, u1(gpu, dims, nd) as d:
+            c.upload(U)
+            d.upload(U)
+            want = d.solve(b, 0.2, tol=1e-10, solver="CG").x
+            fail_allocations(c, refused)
+            failed = 0
+            for _ in range(refused + 1):
+                try:
+                    r = c.solve(b, 0.2, tol=1e-10, solver=solver)
+                    break
+                except gpu.Su2bError as e:
+                    assert e.code == gpu._abi.ERR_NOMEM
+                    failed += 1
+            assert failed >= 1 and rel(r.x, want) < 1e-7
+            fail_allocations(c, 0)
+            assert rel(c.solve(b, 0.2, tol=1e-10, solver=solver).x, want) < 1e-7
