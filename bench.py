@@ -762,7 +762,9 @@ def profile_run(args):
     (all) each of these plus every other kernel of the path once: plaquette, clover, Polyakov
     and Wilson loops, APE smearing, gauge-file save/load, download, CG / BiCGStab (and the
     mixed CG, or in FP64 a pseudofermion trajectory) on the U(1) 256^2 staggered workload,
-    and a leapfrog trajectory of eight chains of the batched ensemble.
+    a leapfrog trajectory of eight chains of the batched ensemble, a two-step flow gradient at
+    24^4, and the forms of small lattices: a trajectory at 8^4 with three threads per link, a
+    sweep at 100^2, a CG and a BiCGStab at 64^2.
     Prints one JSON line with the number of kernel launches made before the K steps (the ncu
     ``-s`` to skip to them) and per step.
     """
@@ -774,7 +776,7 @@ def profile_run(args):
     c.upload(haar_links(V * 4, 20240))
     c.force_variant = args.force_variant
 
-    u1 = batch = None
+    others = []
     if args.profile_op == "all":
         # the staggered solvers run on the U(1) 256^2 workload (vectors of 65,536 sites)
         u1 = su2_b200.gaugeconfig(256, 1, 1, 256, 2, 4.0, group="u1", precision=args.precision)
@@ -787,6 +789,17 @@ def profile_run(args):
         batch = chain_batch(chains, precision="mixed")
         for i, ch in enumerate(chains):
             batch.upload(i, haar_links(replicas.chain_sites(ch) * ch["ndims"], ch["seed"]))
+        grad = su2_b200.gaugeconfig(24, 24, 24, 24, 4, BETA, precision=args.precision)
+        grad.upload(haar_links(24 ** 4 * 4, 20241))
+        small = su2_b200.gaugeconfig(8, 8, 8, 8, 4, 2.3, precision=args.precision)
+        small.upload(haar_links(8 ** 4 * 4, 20242))
+        small.force_variant = 5
+        plane = su2_b200.gaugeconfig(100, 1, 1, 100, 2, 2.0, precision=args.precision)
+        plane.upload(haar_links(100 ** 2 * 2, 20243))
+        u64 = su2_b200.gaugeconfig(64, 1, 1, 64, 2, 4.0, group="u1")
+        u64.upload(np.random.default_rng(4244).uniform(-np.pi, np.pi, size=64 * 64 * 2))
+        b64 = np.random.default_rng(4245).normal(size=2 * 64 * 64)
+        others = [u1, batch, grad, small, plane, u64]
     td = tempfile.mkdtemp()
 
     def step(k):
@@ -813,19 +826,18 @@ def profile_run(args):
             else:  # pseudofermion trajectory (det D D^+ monomial, FP64 U(1) only)
                 u1.md_update("omf2", 2, 0.2, seed=7, traj=k, fermion_mass=0.05, cg_tol=1e-10)
             batch.md_update("leapfrog", 10, 1.0, traj=k)
+            grad.flow_objective(0.01, 2)
+            small.md_update("leapfrog", 10, 1.0, seed=20242, traj=k)
+            plane.sweep(0.15, 10, 20243, k)
+            u64.solve(b64, 0.05, tol=1e-10, solver="CG", tol_mode="rel")
+            u64.solve(b64, 0.05, tol=1e-10, solver="BiCGStab", tol_mode="rel")
 
     def launches():  # over every context of the loop
-        n = c.kernel_launches()
-        if u1 is not None:
-            n += u1.kernel_launches() + batch.kernel_launches()
-        return n
+        return sum(x.kernel_launches() for x in [c, *others])
 
     for k in range(args.warmup):
         step(k)
-    c.synchronize()
-    if u1 is not None:
-        u1.synchronize()
-        torch.cuda.synchronize()
+    torch.cuda.synchronize()
     n0 = launches()
     for k in range(args.steps):
         # an NVTX range per timed step, so that a profiler can select exactly these launches
@@ -840,10 +852,8 @@ def profile_run(args):
                       "force_variant": su2_b200._abi.force_shape(args.force_variant, [L] * 4, 4),
                       "setup_launches": n0, "launches_per_step": (n1 - n0) / max(1, args.steps),
                       "steps": args.steps, "warmup": args.warmup}), flush=True)
-    c.close()
-    if u1 is not None:
-        u1.close()
-        batch.close()
+    for x in [c, *others]:
+        x.close()
     torch.cuda.synchronize()
 
 
