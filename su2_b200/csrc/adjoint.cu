@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
   k_force_vjp(Geom g, const LinkT<T> *U, const T *mu, Sent<T, ND> sent) {
   const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
   int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
-  pdl_start<T, (sizeof(T) == 4 ? 5 : 3)>(cb);
+  pdl_start<(sizeof(T) == 4 ? 5 : 3)>(cb);
   if (cb >= g.Vh) return;
   const Site s = site_from_eo(g, p, cb);
   const size_t V = (size_t)g.V, NL = V * ND, self = (size_t)p * g.Vh + cb;
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(NT, 7)
                      int acc_lam, const T *Z, T b, T *__restrict__ mu, int acc_mu) {
   const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
   int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
-  pdl_start<T, 7>(cb);
+  pdl_start<7>(cb);
   if (cb >= g.Vh) return;
   const Site s = site_from_eo(g, p, cb);
   const size_t V = (size_t)g.V, NL = V * ND, self = (size_t)p * g.Vh + cb;

@@ -72,7 +72,7 @@ __global__ void __launch_bounds__(NT, MINB)
   LinkT<T> *Uo = rel_out >= 0 ? bufs.at((S + rel_out) % 3) + d.off_link : nullptr;
   T *P = Pall + d.off_adj;
   const T f = (T)(d.beta / 2.0);
-  pdl_start<T, MINB>(cb);
+  pdl_start<MINB>(cb);
   double k2 = 0.;
   if (cb < d.g.Vh) {
     if (d.g.nd == 4)
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(NT)
   const int c = __ldg(&of[tile]);
   load_chain<NT>(d, ch + c);
   int cb = (tile - d.tile0) * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
-  pdl_wait<T>(cb);
+  pdl_wait(cb);
   const LinkT<T> *U = bufs.at((cur[c] + rel) % 3) + d.off_link;
   double full = 0., spat = 0., wsum = 0.;
   if (cb < d.g.Vh) {

@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(NT, MINB)
   const int w = threadIdx.x >> 5;
   const int p = w & 1;
   int cb = g.cb0 + blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
-  pdl_start<T, MINB>(cb);
+  pdl_start<MINB>(cb);
   double k2 = 0.;
   if (cb < g.cb0 + g.ncb)
     k2 = force_site_impl<T, ND, ANISO>(g, U, P, extra, f, scale_, mode, wt, ws, Uout, dt_upd, p,
@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(32 * ND, MINB)
   __shared__ double sh[NT / 32];
   const int mu = threadIdx.x >> 5, p = blockIdx.x & 1;
   int cb = g.cb0 + (blockIdx.x >> 1) * 32 + (threadIdx.x & 31);
-  pdl_start<T, MINB>(cb);
+  pdl_start<MINB>(cb);
   double k2 = 0.;
   // the direction is a compile-time constant in each warp's body (static site indexing)
 #define SU2B_LINK_BODY(M)                                                                     \
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(384, 1)
   const bool on = cb < g.cb0 + g.ncb;  // lanes past the end compute the last site, write nothing
   const int c = on ? cb : g.cb0 + g.ncb - 1;
   Site s = site_from_eo(g, p, c);
-  pdl_start<T, 1>(s.lex);
+  pdl_start<1>(s.lex);
   const size_t V = (size_t)g.V, l = mu * V + eo_of(g, s.lex, p);
   if (j == 0 && (mode & FM_HAS_IN)) prefetch_momenta(P, l, 4 * V);
   Su2<T> K;
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(NT, plaq_min_blocks<T, NT>())
   constexpr int NC = 8;  // start |P|^2 and three plaquette sums, end |P|^2, three plaquette sums
   __shared__ double shk[NC * (NT / 32)];
   int band = blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
-  pdl_wait<T>(band);
+  pdl_wait(band);
   double v[3] = {0., 0., 0.}, a[NC];
   plaq_bands<T, ND, NT>(g, U, xi, band, v);
 #pragma unroll
@@ -719,7 +719,7 @@ __global__ void __launch_bounds__(NT, MINB)
   const int w = threadIdx.x >> 5;
   const int half = w & 1, p = (w >> 1) & 1;
   int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
-  pdl_start<T, MINB>(cb);
+  pdl_start<MINB>(cb);
   double k2 = 0.;
   if (cb < g.cb0 + g.ncb)
     k2 = half == 0 ? force_half_impl<T, 0, false>(g, U, P, extra, f, scale_, mode, wt, ws, Uout,
@@ -746,7 +746,7 @@ __global__ void __launch_bounds__(NT, MINB)
   const int w = threadIdx.x >> 5;
   const int half = w & 1, p = (w >> 1) & 1;
   int cb = g.cb0 + blockIdx.x * (NT / 4) + (w >> 2) * 32 + (threadIdx.x & 31);
-  pdl_start<T, MINB>(cb);
+  pdl_start<MINB>(cb);
   const bool valid = cb < g.cb0 + g.ncb;
   const int cbc = valid ? cb : g.cb0 + g.ncb - 1;
   const int bar_id = 1 + (w >> 1);

@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(128, MINB)
   __shared__ double sh[4];
   const int w = threadIdx.x >> 5, p = blockIdx.x & 1;
   int q = (blockIdx.x >> 1) * 32 + (threadIdx.x & 31);
-  pdl_start<float, MINB>(q);
+  pdl_start<MINB>(q);
   double k2 = 0.;
   if (q < g.Vh / 2) {
     const Site s = site_from_eo(g, p, q);

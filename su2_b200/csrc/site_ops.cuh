@@ -16,17 +16,14 @@ template <class T> using LinkT = typename LinkOf<T>::type;
 //   - reads no field, nor anything else that launch writes, before the wait;
 //   - takes such pointers without const __restrict__, from which the compiler would conclude
 //     that the read-only path may be used, and reads them with ordinary loads;
-//   - with FP64 links passes the index that its addresses come from through the wait (`at`):
-//     their ld_link is an asm statement that a memory clobber does not order, and nothing but
-//     the operand keeps it below.  The FP32 load is the compiler's own and heeds the clobber;
-//     there the operand would cost the 64-register force shapes 20 bytes of spills.
+//   - passes the index that its addresses come from through the wait (`at`): ld_link is an asm
+//     statement that a memory clobber does not order, and nothing but the operand keeps it
+//     below.  (FP32 links read by the compiler's own loads instead, which heed the clobber:
+//     32^4 mixed, 33 launches, 2.31 to 2.36 ms a trajectory against 2.25.)
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-template <class T> __device__ __forceinline__ void pdl_wait(int &at) {
-  if constexpr (sizeof(T) == 8)
-    asm volatile("griddepcontrol.wait;" : "+r"(at)::"memory");
-  else
-    pdl_wait();
+__device__ __forceinline__ void pdl_wait(int &at) {
+  asm volatile("griddepcontrol.wait;" : "+r"(at)::"memory");
 }
 
 // The start of a chained launch with MINB resident blocks per SM.  A launch of several waves
@@ -36,9 +33,9 @@ template <class T> __device__ __forceinline__ void pdl_wait(int &at) {
 // down (each of them releases its own successor while it waits); there the next launch starts
 // as blocks exit: ten steps at 12^4 FP64 take 75 us instead of 83 us, at 16^4 124 instead of
 // 131, at 48x40x36 148 instead of 155.
-template <class T, int MINB> __device__ __forceinline__ void pdl_start(int &at) {
+template <int MINB> __device__ __forceinline__ void pdl_start(int &at) {
   if (gridDim.x > 148u * MINB) pdl_trigger();
-  pdl_wait<T>(at);
+  pdl_wait(at);
 }
 
 // launch with the programmatic-stream-serialization attribute when pdl is set

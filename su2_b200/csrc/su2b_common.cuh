@@ -170,11 +170,12 @@ __device__ __forceinline__ void st_link(Link64 *p, const Su2<double> &u) {
                "d"(u.br), "d"(u.bi)
                : "memory");
 }
-// The FP32 load is left to the compiler rather than written as inline PTX: a link it can no
-// longer keep in a register it may then load again (an L1 hit) instead of spilling.
 __device__ __forceinline__ Su2<float> ld_link(const Link32 *p) {
-  const float4 v = *p;
-  return Su2<float>{v.x, v.y, v.z, v.w};
+  Su2<float> r;
+  asm("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];"
+      : "=f"(r.ar), "=f"(r.ai), "=f"(r.br), "=f"(r.bi)
+      : "l"(p));
+  return r;
 }
 __device__ __forceinline__ Su2<float> ld_link_rw(const Link32 *p) {
   const float4 v = *p;
