@@ -226,7 +226,7 @@ SU2B_API int su2b_pion_correlator(su2b_ctx *ctx, double mass, double tol, int ma
 
 /* ---- batched ensembles of independent SU(2) chains ------------------------------------------ */
 /* Chains of different geometry (d = 3 or 4, even extents), coupling and seed advanced together:
- * every stage of a trajectory is one persistent launch over all chains, a trajectory is one
+ * every stage of a trajectory is one launch over all chains, a trajectory is one
  * CUDA graph, and each chain keeps its own accept/reject (md_update.hh:18-81).  A chain's
  * trajectory equals the one of a single-lattice context with the same seed and traj. */
 typedef struct {

@@ -234,9 +234,9 @@ extern "C" int su2b_ctx_create(int group, int Lx, int Ly, int Lz, int Lt, int nd
       (st = dalloc(ctx, &ctx->part, sizeof(double) * 3 * ctx->part_cap * NSLOT)) ||
       (st = dalloc(ctx, &ctx->red, sizeof(double) * 64)) ||
       (st = dalloc(ctx, &ctx->traj, sizeof(TrajDev))) ||
-      (st = dalloc(ctx, &ctx->counts, sizeof(unsigned long long) * 4)) ||
-      (st = dalloc(ctx, &ctx->ticket, sizeof(unsigned))))
+      (st = dalloc(ctx, &ctx->counts, sizeof(unsigned long long) * 4)))
     return fin(st);
+  ctx->ticket = (unsigned *)(ctx->counts + 2);
   if (cudaMallocHost((void **)&ctx->h_red, sizeof(double) * 64) != cudaSuccess ||
       cudaMallocHost((void **)&ctx->h_traj, sizeof(TrajDev)) != cudaSuccess ||
       cudaMallocHost((void **)&ctx->h_counts, sizeof(unsigned long long) * 4) != cudaSuccess ||
@@ -248,8 +248,7 @@ extern "C" int su2b_ctx_create(int group, int Lx, int Ly, int Lz, int Lt, int nd
   ctx->h_cg = (CgTileResult *)(ctx->h_st + 1);
   if (cudaMemsetAsync(ctx->U, 0, lb * NL, ctx->stream) != cudaSuccess ||
       cudaMemsetAsync(ctx->counts, 0, 4 * sizeof(unsigned long long), ctx->stream) !=
-        cudaSuccess ||
-      cudaMemsetAsync(ctx->ticket, 0, sizeof(unsigned), ctx->stream) != cudaSuccess)
+        cudaSuccess)
     return fin(SU2B_ERR_CUDA);
   if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fin(SU2B_ERR_CUDA);
   return fin(SU2B_OK);
@@ -563,10 +562,8 @@ extern "C" int su2b_metropolis_sweep(su2b_ctx *ctx, double delta, int N_hit, uin
   CKS(enter(ctx));
   NEED(rates, "rates is NULL");
   NEED(N_hit >= 0, "N_hit < 0");
-  if (ctx->sweep_open) {  // a sweep ended early: it left its counts
-    CK(cudaMemsetAsync(ctx->counts, 0, 2 * sizeof(unsigned long long), ctx->stream));
-    CK(cudaMemsetAsync(ctx->ticket, 0, sizeof(unsigned), ctx->stream));
-  }
+  if (ctx->sweep_open)  // a sweep ended early: it left its counts
+    CK(cudaMemsetAsync(ctx->counts, 0, 4 * sizeof(unsigned long long), ctx->stream));
   ctx->sweep_open = true;
   ctx->phases_valid = false;
   for (int mu = 0; mu < ctx->g.nd; mu++)

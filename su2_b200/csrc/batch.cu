@@ -608,10 +608,10 @@ int enqueue_batch(su2b_batch *b, const std::vector<BOp> &ops, int *rel_final, bo
   }
 }
 
-// Times the batched force step (momentum step + link update of every chain, one persistent
-// launch) of one launch shape: fresh momenta from the Philox stream, then `reps` launches
-// that read each chain's current field and write the update into a buffer the chain does
-// not use, so the chains' states are untouched.  Returns microseconds per launch.
+// Times the batched force step (momentum step + link update of every chain, one launch) of
+// one launch shape: fresh momenta from the Philox stream, then `reps` launches that read each
+// chain's current field and write the update into a buffer the chain does not use, so the
+// chains' states are untouched.  Returns microseconds per launch.
 template <class T, int NT, int MINB> int time_force_v(su2b_batch *b, int v, double *us) {
   cudaStream_t s = b->stream;
   const ChainDev *ch = b->ch[v];

@@ -40,7 +40,7 @@ struct su2b_ctx {
   su2b::TrajParams *tparams = nullptr, *h_tparams = nullptr;
   unsigned long long *counts = nullptr;  // of a Metropolis sweep, zero between sweeps
   bool sweep_open = false;               // unless one ended with an error
-  unsigned *ticket = nullptr;  // of finish_sums, zero between launches
+  unsigned *ticket = nullptr;  // of finish_sums, zero between launches; behind the counts
 
   // pinned host mirrors
   double *h_red = nullptr;
