@@ -53,20 +53,30 @@ template <class T> __device__ __forceinline__ V3<T> cross(const V3<T> &a, const 
   return V3<T>{fm(a.y, b.z, -a.z * b.y), fm(a.z, b.x, -a.x * b.z), fm(a.x, b.y, -a.y * b.x)};
 }
 // The rotation v -> d^+ v d / |d|^2 of d = (d0, e): v + d0 w + e x w with w = f x v,
-// f = 2 e / |d|^2.  For links that are unitary to their storage precision 2 / n = 4 - 2 n up to
-// (1 - n)^2, below rounding where the first form is taken; a field uploaded unnormalised takes
-// the quotient (a zero link: none, the plaquettes that it is in are zero).
+// f = 2 e / |d|^2 (any w for a zero link, the plaquettes that it is in are zero).  FP32: the fast
+// quotient (2 ulp) and a Newton step.  FP64, where a division is a branch: 2 / n = 4 - 2 n up to
+// (1 - n)^2, below rounding for links that are unitary to 2^-27; a field uploaded unnormalised has
+// others, for which `far` asks for the site once more with EXACT.
 template <class T> struct Rot {
   T d0;
   V3<T> e, f;
 };
-template <class T> __device__ __forceinline__ Rot<T> rot_of(const Su2<T> &d) {
-  constexpr bool F64 = sizeof(T) == 8;
-  const T n = fm(d.ar, d.ar, fm(d.ai, d.ai, fm(d.br, d.br, d.bi * d.bi)));
-  T w = fm(T(-2), n, T(4));
-  if (!(fabs(n - T(1)) < (F64 ? T(0x1p-27) : T(0x1p-12))))
-    w = n > (F64 ? T(1e-300) : T(1e-37)) ? T(2) / n : T(0);
+template <class T> __device__ __forceinline__ Rot<T> rot_by(const Su2<T> &d, T w) {
   return Rot<T>{d.ar, V3<T>{d.bi, d.br, d.ai}, V3<T>{w * d.bi, w * d.br, w * d.ai}};
+}
+template <bool EXACT>
+__device__ __forceinline__ Rot<double> rot_of(const Su2<double> &d, bool &far) {
+  const double n = fm(d.ar, d.ar, fm(d.ai, d.ai, fm(d.br, d.br, d.bi * d.bi)));
+  if constexpr (EXACT) return rot_by(d, n > 1e-300 ? 2.0 / n : 0.0);
+  far |= !(fabs(n - 1.0) < 0x1p-27);
+  return rot_by(d, fm(-2.0, n, 4.0));
+}
+template <bool EXACT>
+__device__ __forceinline__ Rot<float> rot_of(const Su2<float> &d, bool &) {
+  const float n = fm(d.ar, d.ar, fm(d.ai, d.ai, fm(d.br, d.br, d.bi * d.bi)));
+  const float m = fmaxf(n, 1e-37f), r = __fdividef(1.0f, m);
+  const float y = fm(r, fm(-m, r, 1.0f), r);
+  return rot_by(d, y + y);
 }
 // d^+ v d (inverse: d v d^+) over |d|^2
 template <class T>
@@ -99,16 +109,20 @@ template <class T, int ND> struct Sent {
 // thread per link forming all staples with a cotangent in each of their four places took 5,000
 // FMAs and 76 links.  Memory bounds both passes: at 24^4 FP32, cold, 27 us and 35 us with the
 // reverse of a link update in the second, against 109 us and 27 us for that update by itself.
-template <class T, int ND, int NT>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
-  k_force_vjp(Geom g, const LinkT<T> *U, const T *mu, Sent<T, ND> sent) {
-  const int w = threadIdx.x >> 5, p = w & 1, q = 1 - p;
-  int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
-  pdl_start<(sizeof(T) == 4 ? 5 : 3)>(cb);
-  if (cb >= g.Vh) return;
+// An FP64 site whose own links are far from unit norm is done again with exact rotations, after
+// the loads and stores of the first time.  With the division's branch in each rotation, between
+// the loads, 20 steps at 24^4 took 10.8 ms instead of 10.45 (10.25 without any other than unit
+// links), mixed 7.3 instead of 7.0 (6.9).
+template <bool EXACT, class T, int ND>
+__device__ __forceinline__ bool vjp_site(const Geom &g, const LinkT<T> *U, const T *mu,
+                                         const Sent<T, ND> &sent, int p, int cb) {
+  const int q = 1 - p;
   const Site s = site_from_eo(g, p, cb);
   const size_t V = (size_t)g.V, NL = V * ND, self = (size_t)p * g.Vh + cb;
-  auto M = [&](size_t l) { return V3<T>{mu[l], mu[NL + l], mu[2 * NL + l]}; };
+  auto M = [&](size_t l) {
+    return V3<T>{ld_real(mu + l), ld_real(mu + NL + l), ld_real(mu + 2 * NL + l)};
+  };
+  bool far = false;
   Su2<T> u[ND];
   V3<T> S[ND];
 #pragma unroll
@@ -121,7 +135,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
       const size_t lc = d * V + eo_of(g, s.lex + fwd(g, s, e), q);
       const Su2<T> P = mul(mul(u[d], ld_link(U + lb)), dag(mul(u[e], ld_link(U + lc))));
       const V3<T> pv{P.bi, P.br, P.ai};
-      const Rot<T> ra = rot_of(u[d]), rd = rot_of(u[e]);
+      const Rot<T> ra = rot_of<EXACT>(u[d], far), rd = rot_of<EXACT>(u[e], far);
       const V3<T> nb = rotate(ra, M(lb), true), nc = rotate(rd, M(lc), true);
       const V3<T> N = (M(d * V + self) + nb) - (nc + M(e * V + self));
       const V3<T> v{P.ar * N.x, P.ar * N.y, P.ar * N.z}, x = cross(pv, N);
@@ -145,6 +159,20 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
     sent.at(k, V)[self] = S[d].x;
     sent.at(k + 1, V)[self] = S[d].y;
     sent.at(k + 2, V)[self] = S[d].z;
+  }
+  return far;
+}
+template <class T, int ND, int NT>
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 5 : 3)
+  k_force_vjp(Geom g, const LinkT<T> *U, const T *mu, Sent<T, ND> sent) {
+  const int w = threadIdx.x >> 5, p = w & 1;
+  int cb = blockIdx.x * (NT / 2) + (w >> 1) * 32 + (threadIdx.x & 31);
+  pdl_start<(sizeof(T) == 4 ? 5 : 3)>(cb);
+  if (cb >= g.Vh) return;
+  const bool far = vjp_site<false>(g, U, mu, sent, p, cb);
+  if (sizeof(T) == 8 && far) {
+    asm volatile("" : "+r"(cb));  // loads of its own, so that none is kept for it
+    vjp_site<sizeof(T) == 8>(g, U, mu, sent, p, cb);
   }
 }
 

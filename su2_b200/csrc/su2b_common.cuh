@@ -177,6 +177,18 @@ __device__ __forceinline__ Su2<float> ld_link(const Link32 *p) {
       : "l"(p));
   return r;
 }
+// the same of one real (of a field that the kernel's own stores might alias for all that the
+// compiler knows, whose loads it would otherwise keep behind them)
+__device__ __forceinline__ double ld_real(const double *p) {
+  double v;
+  asm("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float ld_real(const float *p) {
+  float v;
+  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ Su2<float> ld_link_rw(const Link32 *p) {
   const float4 v = *p;
   return Su2<float>{v.x, v.y, v.z, v.w};
