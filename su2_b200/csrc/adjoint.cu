@@ -107,7 +107,7 @@ template <class T, int ND> struct Sent {
 // four results into `sent`; pass 2 adds a link's own sum and what the backward neighbours sent.
 // 930 FMAs and 16 links per site in d = 4 and 384 B (FP32) of intermediate values, where one
 // thread per link forming all staples with a cotangent in each of their four places took 5,000
-// FMAs and 76 links.  Memory bounds both passes: at 24^4 FP32, cold, 27 us and 35 us with the
+// FMAs and 76 links.  Memory bounds both passes: at 24^4 FP32, cold, 33 us and 38 us with the
 // reverse of a link update in the second, against 109 us and 27 us for that update by itself.
 // An FP64 site whose own links are far from unit norm is done again with exact rotations, after
 // the loads and stores of the first time.  With the division's branch in each rotation, between
@@ -512,7 +512,7 @@ int flow_adjoint_t(su2b_ctx *ctx, double eps, int n, int every, double *objectiv
   Scratch sc;
   // Every stage's field and Z kept from the forward pass where there is room for them and the
   // caller asked for no checkpoints: the reverse pass then runs no force again.  20 steps at
-  // 24^4, mixed precision: 7.35 ms and 2.2 GB against 9.85 ms and 0.3 GB.
+  // 24^4, mixed precision: 7.0 ms and 2.2 GB against 9.85 ms and 0.3 GB.
   const size_t tape = (size_t)n * 3 * (lb_a + ab_a) + lb_a + 2 * ab_a;
   const ArenaUse use(ctx);
   if (grad_host && every <= 0 && tape_arena(ctx, tape, &sc))
