@@ -74,7 +74,8 @@ def test_chained_kernel_reads_its_input_coherently(src, name, params, body):
     # FP64 links are read below the wait only if their addresses come out of it
     waits = re.findall(r"pdl_(?:start|wait)(?:<.*?>)?\(([^()]*)\);", body)
     own_loads = "ld_link" in body or re.search(r"\b(force_\w+_impl|force_half_x|staple_pair|"
-                                               r"plaq_site|plaq_bands|pair_link)\b", body)
+                                               r"plaq_site|plaq_bands|pair_link|vjp_site)\b",
+                                               body)
     assert waits
     if own_loads and "ld_link_rw" not in body:
         assert all(waits), f"{src}: {name} waits without the index of its loads"
